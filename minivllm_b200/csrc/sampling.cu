@@ -13,11 +13,14 @@
 // row instead of a gather of the logits) and decoded to token ids.
 // HBM-bound: one read of the logits, rows * cols * 2 bytes.
 #include <climits>
+#include <cooperative_groups.h>
 #include "common.cuh"
 
 namespace mv {
 
+namespace cg = cooperative_groups;
 constexpr int kArgmaxThreads = 256;
+constexpr int kMaxRowCtas = 8;         // the portable cluster size
 
 // float -> int32 whose signed order is the float order; NaN sorts above +inf (torch.argmax treats NaN as the
 // maximum) and -0.0 maps to the key of +0.0 (they compare equal, so the lower index must win between them).
@@ -37,88 +40,125 @@ __device__ __forceinline__ long long token_of_key(long long key) {
 
 // One CTA per row.  A thread walks its columns in increasing order and keeps the first maximum it meets
 // (strict >), so equal logits resolve to the lowest index within a thread; across threads the keys do it.
-template <typename T>
-__global__ void __launch_bounds__(kArgmaxThreads)
-argmax_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t cols, uint32_t index_offset, bool aligned,
-                   long long* __restrict__ keys, long long* __restrict__ tokens) {
-  using T2 = typename Elem<T>::T2;
-  const T* row = logits + static_cast<int64_t>(blockIdx.x) * row_stride;
-  float best = -INFINITY;
-  bool best_nan = false, have = false;
-  uint32_t best_idx = 0;
-  auto offer = [&](float v, uint32_t idx) {
-    if (best_nan) return;                       // a NaN already won: it is the maximum and came first
-    const bool is_nan = v != v;
-    if (is_nan || v > best || !have) {
-      best = v;
-      best_idx = idx;
-      best_nan = is_nan;
+// The best logit or score that a thread has met: the first maximum in visiting order, and a NaN is the maximum.
+struct Best {
+  float v = -INFINITY;
+  bool nan = false, have = false;
+  uint32_t idx = 0;
+  __device__ __forceinline__ void offer(float x, uint32_t i) {
+    if (nan) return;                            // a NaN already won: it is the maximum and came first
+    const bool is_nan = x != x;
+    if (is_nan || x > v || !have) {
+      v = x;
+      idx = i;
+      nan = is_nan;
       have = true;
     }
-  };
-  const int64_t chunks = sizeof(T) == 2 && aligned ? cols / 8 : 0;  // 16-byte chunks when every row starts on a 16-byte boundary
-  // Per chunk of eight logits only its maximum is computed (packed 16-bit maxima, exact, NaN-propagating) and
-  // compared with the running one; the chunk that raised it is kept and searched for the position at the end.
-  // Chunks are visited in increasing order and only a strictly larger maximum replaces the kept chunk, so the
-  // first of equal maxima survives.
-  constexpr int kUnroll = 4;
-  uint4 best_raw = make_uint4(0, 0, 0, 0);
-  int64_t best_chunk = -1;
-  float cbest = -INFINITY;
-  bool cbest_nan = false;
-  if constexpr (sizeof(T) == 2) {
-  for (int64_t c0 = threadIdx.x; c0 < chunks; c0 += static_cast<int64_t>(kArgmaxThreads) * kUnroll) {
-    uint4 raw[kUnroll];
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const int64_t c = c0 + static_cast<int64_t>(u) * kArgmaxThreads;
-      if (c < chunks) raw[u] = ld_stream16(row + c * 8);
-    }
-#pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
-      const int64_t c = c0 + static_cast<int64_t>(u) * kArgmaxThreads;
-      if (c < chunks && !cbest_nan) {
-        const T2* p2 = reinterpret_cast<const T2*>(&raw[u]);
-        const float m = Elem<T>::hmax_nan_f(Elem<T>::max2_nan(Elem<T>::max2_nan(p2[0], p2[1]),
-                                                              Elem<T>::max2_nan(p2[2], p2[3])));
-        const bool is_nan = m != m;
-        if (is_nan || m > cbest || best_chunk < 0) {
-          cbest = m;
-          cbest_nan = is_nan;
-          best_chunk = c;
-          best_raw = raw[u];
-        }
-      }
-    }
   }
-  if (best_chunk >= 0) {   // position of the first maximum (or first NaN) inside the kept chunk
-    const T2* p2 = reinterpret_cast<const T2*>(&best_raw);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = Elem<T>::to_f2(p2[j]);
-      offer(f.x, static_cast<uint32_t>(best_chunk * 8 + 2 * j));
-      offer(f.y, static_cast<uint32_t>(best_chunk * 8 + 2 * j + 1));
-    }
-  }
-  }
-  for (int64_t i = chunks * 8 + threadIdx.x; i < cols; i += kArgmaxThreads)   // ragged tail
-    offer(Elem<T>::to_f(row[i]), static_cast<uint32_t>(i));
+};
 
-  long long key = have ? make_key(best, index_offset + best_idx) : LLONG_MIN;
+// A row belongs to the CTAs of a cluster; thread `at` of `threads` takes every threads-th piece.
+struct RowShare {
+  uint32_t at, threads, rank, ctas;
+  __device__ __forceinline__ RowShare() {
+    ctas = cg::this_cluster().num_blocks();
+    rank = cg::this_cluster().block_rank();
+    at = rank * kArgmaxThreads + threadIdx.x;
+    threads = ctas * kArgmaxThreads;
+  }
+};
+
+// The row's largest key from all threads of its cluster, written by its first CTA.
+__device__ __forceinline__ void finish_row(const Best& best, uint32_t index_offset, const RowShare& my, int64_t row, long long* keys,
+                                           long long* tokens) {
+  long long key = best.have ? make_key(best.v, index_offset + best.idx) : LLONG_MIN;
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) {
     const long long other = __shfl_xor_sync(0xffffffffu, key, off);
     key = other > key ? other : key;
   }
-  __shared__ long long s_keys[kArgmaxThreads / 32];
+  __shared__ long long s_keys[kArgmaxThreads / 32], s_ctas[kMaxRowCtas];
   if ((threadIdx.x & 31) == 0) s_keys[threadIdx.x >> 5] = key;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0)
 #pragma unroll
     for (int w = 1; w < kArgmaxThreads / 32; ++w) key = s_keys[w] > key ? s_keys[w] : key;
-    if (keys) keys[blockIdx.x] = key;
-    if (tokens) tokens[blockIdx.x] = token_of_key(key);
+  if (my.ctas > 1) {
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();                             // the first CTA has begun: its shared memory may be written
+    if (threadIdx.x == 0) cluster.map_shared_rank(s_ctas, 0)[my.rank] = key;
+    cluster.sync();
+    if (my.rank == 0 && threadIdx.x == 0)
+      for (uint32_t c = 1; c < my.ctas; ++c) key = s_ctas[c] > key ? s_ctas[c] : key;
   }
+  if (my.rank == 0 && threadIdx.x == 0) {
+    if (keys) keys[row] = key;
+    if (tokens) tokens[row] = token_of_key(key);
+  }
+}
+
+// The plain maximum over this thread's share of a row.  Per chunk of eight logits only its maximum is computed (packed 16-bit
+// maxima, exact, NaN-propagating) and compared with the running one; the chunk that raised it is kept and searched for the
+// position at the end.  Chunks are visited in increasing order and only a strictly larger maximum replaces the kept chunk,
+// so the first of equal maxima survives.
+template <typename T>
+__device__ __forceinline__ void argmax_share(const T* row, int64_t cols, bool aligned, const RowShare& my, Best& best) {
+  // 16-byte chunks when every row starts on a 16-byte boundary
+  const int64_t chunks = sizeof(T) == 2 && aligned ? cols / 8 : 0;
+  if constexpr (sizeof(T) == 2) {
+    using T2 = typename Elem<T>::T2;
+    constexpr int kUnroll = 4;
+    uint4 best_raw = make_uint4(0, 0, 0, 0);
+    int64_t best_chunk = -1;
+    float cbest = -INFINITY;
+    bool cbest_nan = false;
+    for (int64_t c0 = my.at; c0 < chunks; c0 += static_cast<int64_t>(my.threads) * kUnroll) {
+      uint4 raw[kUnroll];
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const int64_t c = c0 + static_cast<int64_t>(u) * my.threads;
+        if (c < chunks) raw[u] = ld_stream16(row + c * 8);
+      }
+#pragma unroll
+      for (int u = 0; u < kUnroll; ++u) {
+        const int64_t c = c0 + static_cast<int64_t>(u) * my.threads;
+        if (c < chunks && !cbest_nan) {
+          const T2* p2 = reinterpret_cast<const T2*>(&raw[u]);
+          const float m = Elem<T>::hmax_nan_f(Elem<T>::max2_nan(Elem<T>::max2_nan(p2[0], p2[1]),
+                                                                Elem<T>::max2_nan(p2[2], p2[3])));
+          const bool is_nan = m != m;
+          if (is_nan || m > cbest || best_chunk < 0) {
+            cbest = m;
+            cbest_nan = is_nan;
+            best_chunk = c;
+            best_raw = raw[u];
+          }
+        }
+      }
+    }
+    if (best_chunk >= 0) {   // position of the first maximum (or first NaN) inside the kept chunk
+      const T2* p2 = reinterpret_cast<const T2*>(&best_raw);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 f = Elem<T>::to_f2(p2[j]);
+        best.offer(f.x, static_cast<uint32_t>(best_chunk * 8 + 2 * j));
+        best.offer(f.y, static_cast<uint32_t>(best_chunk * 8 + 2 * j + 1));
+      }
+    }
+  }
+  for (int64_t i = chunks * 8 + my.at; i < cols; i += my.threads)   // ragged tail, or rows that start anywhere
+    best.offer(Elem<T>::to_f(row[i]), static_cast<uint32_t>(i));
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kArgmaxThreads)
+argmax_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t cols, uint32_t index_offset, bool aligned,
+                   long long* __restrict__ keys, long long* __restrict__ tokens) {
+  const RowShare my;
+  const int64_t r = blockIdx.x / my.ctas;
+  Best best;
+  argmax_share(logits + r * row_stride, cols, aligned, my, best);
+  finish_row(best, index_offset, my, r, keys, tokens);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -157,84 +197,99 @@ __device__ __forceinline__ float race_noise(uint32_t bits) {
   return -__logf(-logf(u));
 }
 
-template <typename T>
+// One thread takes the columns of kPiece / 4 Philox groups at a time: 16-byte loads of eight 16-bit or four 32-bit logits where
+// rows and the shard start on such boundaries, else four single loads per group, so that a group's four words are drawn once
+// in either case.
+//
+// Bound: instruction issue (a column's share of Philox is 15 slots).  A score is only formed where it can win.  With E = -log u
+// >= 1 - u a score is at most v / T - log(1 - u), so a column whose 1 - u exceeds e^(v / T - best) is passed over for one
+// ex2.approx instead of two logarithms; `best` is the warp's, which moves about ten times in a row.  The test errs on the side
+// of forming the score: `slack` covers the roundings of the exponent (a few 2^-23 of best, and those of the noise itself),
+// kEdge those of u, and a NaN or an infinity fails the comparison.  Every score that is formed is the same as before, so are the
+// tokens.  512 x 151,936 bf16: 236 us when every score was formed, 132 us now.
+template <typename T, bool kVec>
 __global__ void __launch_bounds__(kArgmaxThreads)
 sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t cols, uint32_t index_offset, bool aligned,
                    const float* __restrict__ temperatures, unsigned long long seed, const long long* __restrict__ step_ptr,
                    long long* __restrict__ keys, long long* __restrict__ tokens) {
-  using T2 = typename Elem<T>::T2;
-  const uint32_t rowi = blockIdx.x;
+  const RowShare my;
+  const uint32_t rowi = blockIdx.x / my.ctas;
   const T* row = logits + static_cast<int64_t>(rowi) * row_stride;
   const float temp = temperatures[rowi];
-  const bool greedy = !(temp > 0.f);
-  const float inv_t = greedy ? 1.0f : 1.0f / temp;
+  Best best;
+  if (!(temp > 0.f)) {                           // a greedy row
+    argmax_share(row, cols, aligned, my, best);
+    finish_row(best, index_offset, my, rowi, keys, tokens);
+    return;
+  }
+  const float inv_t = 1.0f / temp;
   const unsigned long long step = static_cast<unsigned long long>(*step_ptr);
   const uint32_t k0 = static_cast<uint32_t>(seed), k1 = static_cast<uint32_t>(seed >> 32);
   const uint32_t s0 = static_cast<uint32_t>(step), s1 = static_cast<uint32_t>(step >> 32);
-  float best = -INFINITY;
-  bool best_nan = false, have = false;
-  uint32_t best_idx = 0;
-  auto offer = [&](float v, uint32_t idx) {       // first maximum in visiting order; a NaN is the maximum
-    if (best_nan) return;
-    const bool is_nan = v != v;
-    if (is_nan || v > best || !have) {
-      best = v;
-      best_idx = idx;
-      best_nan = is_nan;
-      have = true;
+  constexpr int kPiece = kVec && sizeof(T) == 2 ? 8 : 4;
+  constexpr float kLog2 = 1.4426950408889634f, kEdge = 2.f - 0x1p-21f;
+  const float slope = inv_t * kLog2;
+  float shift = INFINITY;                        // (slack - best) in base 2: everything may win at first
+  // Global columns base .. base + kPiece - 1 of piece p; the first piece may begin before the shard.
+  const uint32_t base0 = index_offset & ~3u;
+  const int64_t lead = static_cast<int64_t>(index_offset) - base0, pieces = (cols + lead + kPiece - 1) / kPiece;
+  const int64_t rounds = (pieces + my.threads - 1) / my.threads;
+  for (int64_t it = 0; it < rounds; ++it) {      // the same number for all lanes: they vote
+    const int64_t p = it * my.threads + my.at, i0 = p * kPiece - lead;
+    float v[kPiece];
+    bool live = false;                           // some column of the piece exists
+    if constexpr (kVec) {
+      live = p < pieces;
+      if (live) {
+        if (i0 + kPiece <= cols) {
+          const uint4 raw = ld_stream16(row + i0);
+          if constexpr (sizeof(T) == 2) {
+            const typename Elem<T>::T2* p2 = reinterpret_cast<const typename Elem<T>::T2*>(&raw);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 f = Elem<T>::to_f2(p2[j]);
+              v[2 * j] = f.x;
+              v[2 * j + 1] = f.y;
+            }
+          } else {
+            const float4 f = *reinterpret_cast<const float4*>(&raw);
+            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < kPiece; ++j) v[j] = i0 + j < cols ? Elem<T>::to_f(row[i0 + j]) : -INFINITY;
+        }
+      }
+    } else {
+      live = p < pieces;
+#pragma unroll
+      for (int j = 0; j < kPiece; ++j) v[j] = live && i0 + j >= 0 && i0 + j < cols ? Elem<T>::to_f(row[i0 + j]) : -INFINITY;
     }
-  };
-  auto noise_of = [&](uint32_t gcol) {           // one column on its own (ragged edges)
-    const Philox r = philox4x32_10(Philox{gcol >> 2, rowi, s0, s1}, k0, k1);
-    const uint32_t lane = gcol & 3u;
-    return race_noise(lane == 0 ? r.x : lane == 1 ? r.y : lane == 2 ? r.z : r.w);
-  };
-  // 16-byte chunks of eight logits = two Philox groups, when rows and the shard start on such boundaries
-  const bool fast = sizeof(T) == 2 && aligned && (index_offset & 7u) == 0;
-  const int64_t chunks = fast ? cols / 8 : 0;
-  if constexpr (sizeof(T) == 2) {
-  for (int64_t c = threadIdx.x; c < chunks; c += kArgmaxThreads) {
-    const uint4 raw = ld_stream16(row + c * 8);
-    const T2* p2 = reinterpret_cast<const T2*>(&raw);
-    float v[8];
+    uint32_t bits[kPiece], may = 0;
+    if (live) {
+      const uint32_t group = (base0 >> 2) + static_cast<uint32_t>(p * (kPiece / 4));
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = Elem<T>::to_f2(p2[j]);
-      v[2 * j] = f.x;
-      v[2 * j + 1] = f.y;
+      for (int q = 0; q < kPiece / 4; ++q) {
+        const Philox a = philox4x32_10(Philox{group + q, rowi, s0, s1}, k0, k1);
+        bits[4 * q] = a.x; bits[4 * q + 1] = a.y; bits[4 * q + 2] = a.z; bits[4 * q + 3] = a.w;
+      }
+#pragma unroll
+      for (int j = 0; j < kPiece; ++j) {
+        const float e = fast_exp2(fmaf(v[j], slope, shift)), u1 = __uint_as_float((bits[j] >> 9) | 0x3f800000u);     // 1 + u
+        may |= u1 + e < kEdge ? 0u : 1u << j;
+      }
     }
-    const uint32_t g0 = index_offset + static_cast<uint32_t>(c * 8);
-    if (!greedy) {
-      const Philox a = philox4x32_10(Philox{g0 >> 2, rowi, s0, s1}, k0, k1);
-      const Philox b = philox4x32_10(Philox{(g0 >> 2) + 1, rowi, s0, s1}, k0, k1);
-      const uint32_t bits[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    if (!__any_sync(0xffffffffu, may != 0)) continue;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = v[j] * inv_t + race_noise(bits[j]);
-    }
+    for (int j = 0; j < kPiece; ++j)
+      if ((may >> j & 1) && i0 + j >= 0 && i0 + j < cols) best.offer(v[j] * inv_t + race_noise(bits[j]), static_cast<uint32_t>(i0 + j));
+    float top = best.v;                          // a NaN leaves the others' maximum
 #pragma unroll
-    for (int j = 0; j < 8; ++j) offer(v[j], static_cast<uint32_t>(c * 8 + j));
+    for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+    const float slack = 0.02f + 4e-6f * fabsf(top);
+    shift = (slack - top) * kLog2;
   }
-  }
-  for (int64_t i = chunks * 8 + threadIdx.x; i < cols; i += kArgmaxThreads) {
-    float v = Elem<T>::to_f(row[i]);
-    if (!greedy) v = v * inv_t + noise_of(index_offset + static_cast<uint32_t>(i));
-    offer(v, static_cast<uint32_t>(i));
-  }
-  long long key = have ? make_key(best, index_offset + best_idx) : LLONG_MIN;
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const long long other = __shfl_xor_sync(0xffffffffu, key, off);
-    key = other > key ? other : key;
-  }
-  __shared__ long long s_keys[kArgmaxThreads / 32];
-  if ((threadIdx.x & 31) == 0) s_keys[threadIdx.x >> 5] = key;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-#pragma unroll
-    for (int w = 1; w < kArgmaxThreads / 32; ++w) key = s_keys[w] > key ? s_keys[w] : key;
-    if (keys) keys[blockIdx.x] = key;
-    if (tokens) tokens[blockIdx.x] = token_of_key(key);
-  }
+  finish_row(best, index_offset, my, rowi, keys, tokens);
 }
 
 // keys (shards, rows) -> tokens (rows): the largest key of each row, decoded.
@@ -250,6 +305,32 @@ __global__ void argmax_decode_kernel(const long long* __restrict__ keys, int sha
   tokens[r] = token_of_key(key);
 }
 
+// A row's CTAs, one cluster: more of them while the rows alone would leave SMs with fewer than four, as long as each thread has
+// two 16-byte pieces.
+static unsigned row_ctas(int64_t rows, int64_t cols) {
+  unsigned n = 1;
+  while (n < kMaxRowCtas && rows * n < 4 * kNumSMs && cols >= static_cast<int64_t>(n) * 2 * kArgmaxThreads * 16) n *= 2;
+  return n;
+}
+
+template <typename... P, typename... A>
+static int launch_rows(const char* what, void (*kernel)(P...), int64_t rows, int64_t cols, cudaStream_t st, A... args) {
+  const unsigned ctas = row_ctas(rows, cols);
+  if (rows * ctas > 0x7fffffffLL) return fail(MV_ERR_LIMIT, "%s: too many rows", what);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(rows) * ctas);
+  cfg.blockDim = dim3(kArgmaxThreads);
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = ctas;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = ctas > 1 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  return check_launch(what);
+}
+
 }  // namespace mv
 
 extern "C" int mv_argmax_rows(const void* logits, int64_t row_stride, int64_t rows, int64_t cols,
@@ -263,21 +344,13 @@ extern "C" int mv_argmax_rows(const void* logits, int64_t row_stride, int64_t ro
   const bool aligned = row_stride % 8 == 0 && aligned16(logits);   // otherwise element-wise loads
   if (index_offset + cols > 0xffffffffLL || rows > 0x7fffffffLL)
     return fail(MV_ERR_LIMIT, "argmax_rows: column index beyond 32 bits or too many rows");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const unsigned grid = static_cast<unsigned>(rows);
-  if (dtype == MV_F16)
-    argmax_rows_kernel<__half><<<grid, kArgmaxThreads, 0, st>>>(
-        static_cast<const __half*>(logits), row_stride, cols, static_cast<uint32_t>(index_offset), aligned,
-        reinterpret_cast<long long*>(keys), reinterpret_cast<long long*>(tokens));
-  else if (dtype == MV_F32)
-    argmax_rows_kernel<float><<<grid, kArgmaxThreads, 0, st>>>(
-        static_cast<const float*>(logits), row_stride, cols, static_cast<uint32_t>(index_offset), aligned,
-        reinterpret_cast<long long*>(keys), reinterpret_cast<long long*>(tokens));
-  else
-    argmax_rows_kernel<__nv_bfloat16><<<grid, kArgmaxThreads, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(logits), row_stride, cols, static_cast<uint32_t>(index_offset), aligned,
-        reinterpret_cast<long long*>(keys), reinterpret_cast<long long*>(tokens));
-  return check_launch("argmax_rows_kernel");
+  auto run = [&](auto zero) {
+    using T = decltype(zero);
+    return launch_rows("argmax_rows_kernel", argmax_rows_kernel<T>, rows, cols, static_cast<cudaStream_t>(stream),
+                       static_cast<const T*>(logits), row_stride, cols, static_cast<uint32_t>(index_offset), aligned,
+                       reinterpret_cast<long long*>(keys), reinterpret_cast<long long*>(tokens));
+  };
+  return dtype == MV_F16 ? run(__half{}) : dtype == MV_F32 ? run(float{}) : run(__nv_bfloat16{});
 }
 
 extern "C" int mv_argmax_decode(const int64_t* keys, int shards, int64_t rows, int64_t* tokens, void* stream) {
@@ -304,25 +377,18 @@ extern "C" int mv_sample_rows(const void* logits, int64_t row_stride, int64_t ro
   if (row_stride < cols) return fail(MV_ERR_SHAPE, "sample_rows: row stride smaller than a row");
   if (index_offset + cols > 0xffffffffLL || rows > 0x7fffffffLL)
     return fail(MV_ERR_LIMIT, "sample_rows: column index beyond 32 bits or too many rows");
-  const bool aligned = row_stride % 8 == 0 && aligned16(logits);
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const unsigned grid = static_cast<unsigned>(rows);
-  if (dtype == MV_F16)
-    sample_rows_kernel<__half><<<grid, kArgmaxThreads, 0, st>>>(
-        static_cast<const __half*>(logits), row_stride, cols, static_cast<uint32_t>(index_offset), aligned, temperatures,
-        seed, reinterpret_cast<const long long*>(step), reinterpret_cast<long long*>(keys),
-        reinterpret_cast<long long*>(tokens));
-  else if (dtype == MV_F32)
-    sample_rows_kernel<float><<<grid, kArgmaxThreads, 0, st>>>(
-        static_cast<const float*>(logits), row_stride, cols, static_cast<uint32_t>(index_offset), aligned, temperatures,
-        seed, reinterpret_cast<const long long*>(step), reinterpret_cast<long long*>(keys),
-        reinterpret_cast<long long*>(tokens));
-  else
-    sample_rows_kernel<__nv_bfloat16><<<grid, kArgmaxThreads, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(logits), row_stride, cols, static_cast<uint32_t>(index_offset), aligned,
-        temperatures, seed, reinterpret_cast<const long long*>(step), reinterpret_cast<long long*>(keys),
-        reinterpret_cast<long long*>(tokens));
-  return check_launch("sample_rows_kernel");
+  auto run = [&](auto zero) {
+    using T = decltype(zero);
+    constexpr int kPiece = 16 / sizeof(T);
+    const bool aligned = row_stride % 8 == 0 && aligned16(logits);
+    const bool vec = row_stride % kPiece == 0 && aligned16(logits) && index_offset % kPiece == 0;
+    return launch_rows("sample_rows_kernel", vec ? sample_rows_kernel<T, true> : sample_rows_kernel<T, false>, rows, cols,
+                       static_cast<cudaStream_t>(stream), static_cast<const T*>(logits), row_stride, cols,
+                       static_cast<uint32_t>(index_offset), aligned, temperatures, static_cast<unsigned long long>(seed),
+                       reinterpret_cast<const long long*>(step), reinterpret_cast<long long*>(keys),
+                       reinterpret_cast<long long*>(tokens));
+  };
+  return dtype == MV_F16 ? run(__half{}) : dtype == MV_F32 ? run(float{}) : run(__nv_bfloat16{});
 }
 
 // The generator of mv_sample_rows on the host: the four 32-bit words for (seed, step, row, column group).

@@ -245,3 +245,22 @@ def test_sampled_token_frequencies_follow_the_softmax():
     p = np.exp(z) / np.exp(z).sum()
     freq = np.bincount(toks, minlength=8) / rows
     assert np.abs(freq - p).max() < 0.01, (freq, p)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols,offset,dtype", [(1, 70001, 0, torch.bfloat16), (3, 16384, 8, torch.float16), (2, 16391, 5, torch.float32),
+                                                    (5, 8200, 4, torch.float32), (2, 7, 3, torch.bfloat16), (700, 33, 1, torch.float16)])
+def test_sampled_scores_at_any_start_and_length(rows, cols, offset, dtype):
+    """Rows over one to eight CTAs, pieces of eight, four and single columns, a shard that begins inside a group of four: the
+    winner's score is the oracle's largest to 32-bit rounding (2^-21.4 from the outer
+    logarithm, a few 2^-24 of the score from the rest)."""
+    from minivllm_b200.layers import sampler as S
+    x = _logits(11, rows, cols, dtype)
+    temps = torch.linspace(0.3, 2.0, rows)
+    step = torch.tensor([5], dtype=torch.int64, device="cuda")
+    keys, tokens = S.sample_rows(x.cuda(), temps.cuda(), 77, step, index_offset=offset, want_tokens=True)
+    got = tokens.cpu().numpy() - offset
+    scores = oracle.race_scores(x[:3].float().numpy(), temps[:3].tolist(), 77, 5, offset)
+    for r, sc in enumerate(scores):
+        assert 0 <= got[r] < cols and sc[got[r]] >= sc.max() - 4e-6 * max(1.0, abs(float(sc.max()))), r
+    assert np.array_equal(S.decode_keys(keys).cpu().numpy(), tokens.cpu().numpy())
