@@ -657,13 +657,14 @@ int mv_delta_scan(void* out, int64_t out_stride, const void* qkv, int64_t stride
 /*
  * The same recurrences for packed portions in chunks of 64 tokens on tensor cores, bf16: dim a multiple of 8 up to 128,
  * vdim a multiple of 8, rows on 16-byte boundaries.  tokens = cu[num_seqs]; workspace_bytes is -1 when the sizes are not
- * taken.
+ * taken.  error_word: an int on the device that a bounded wait sets when it runs out, as in mv_prefill_varlen (version 6).
  */
 int64_t mv_gla_chunk_workspace_bytes(int64_t tokens, int num_seqs, int heads, int dim, int vdim);
 int mv_gla_chunk_scan(void* out, int64_t out_stride, const void* q, const void* k, const void* v,
     int64_t stride, const void* z, int64_t z_stride, float tau, const int32_t* cu, int num_seqs,
     int64_t tokens, const int32_t* slots, const int32_t* start, float* state, int num_slots, int
-    heads, int dim, int vdim, float q_scale, void* workspace, int64_t workspace_bytes, void* stream);
+    heads, int dim, int vdim, float q_scale, void* workspace, int64_t workspace_bytes, int* error_word,
+    void* stream);
 int64_t mv_delta_chunk_workspace_bytes(int64_t tokens, int num_seqs, int heads, int dim, int vdim);
 int mv_delta_chunk_scan(void* out, int64_t out_stride, const void* qkv, int64_t stride, const void*
     beta, const void* a, int64_t ba_stride, const void* A_log, const void* dt_bias, const int32_t* cu,
@@ -698,7 +699,8 @@ int64_t mv_mlstm_chunk_workspace_bytes(int64_t tokens, int num_seqs, int heads, 
 int mv_mlstm_chunk_scan(void* out, int64_t out_stride, float* den, const void* q, const void* k, const void*
     v, int64_t stride, const float* chain, const int32_t* cu, int num_seqs, int64_t tokens, const int32_t*
     slots, const int32_t* start, float* S, float* n, int num_slots, int heads, int dim, int vdim, float
-    q_scale, void* workspace, int64_t workspace_bytes, void* stream);
+    q_scale, void* workspace, int64_t workspace_bytes, int* error_word,
+    void* stream);
 int mv_mlstm_step(void* out, int64_t out_stride, const void* q, const void* k, const void* v, int64_t stride,
     const void* x, int64_t x_stride, const void* gates_w, int width, const void* i_b, const void* f_b, float
     cap, int num_seqs, const int32_t* slots, const int32_t* start, float* S, float* n, float* m, int num_slots, int heads, int
@@ -793,7 +795,8 @@ int mv_time_scan(void* out, int64_t out_stride, const void* r, const void* k, co
 int mv_time_chunk_scan(void* out, int64_t out_stride, const void* r, const void* k, const void* v, int64_t stride, const
     float* z, int64_t z_stride, const void* w0, const void* bonus, const int32_t* cu, int num_seqs, int64_t tokens, const
     int32_t* slots, const int32_t* start, float* state, int num_slots, int heads, int dim, int vdim, void* workspace,
-    int64_t workspace_bytes, void* stream);
+    int64_t workspace_bytes, int* error_word,
+    void* stream);
 
 /*
  * Between two sublayers of a decoder with one fp32 residual stream and an element-wise norm: out = tanh(alpha x') w + b, where

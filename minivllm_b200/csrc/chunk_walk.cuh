@@ -1,0 +1,573 @@
+// The walk over a sequence's chunks (state_chunk.cuh) on tcgen05, the state in tensor memory.
+//
+// Everything is transposed: tensor memory's 128 lanes are 128 value columns.  Per chunk of 64 tokens
+//   O^T = S_0^T Q^T (+) V^T A^T        S_0 as a TMEM operand in two bf16 terms, V^T straight from rows of tokens (MN-major)
+//   S^T = decay S_0^T + V^T K          accumulated onto the decayed state where it lies
+// gla and time mixing (kMem false): Q, K and A come decayed and in two terms each from the preparing kernel, as one block of
+// scratch that lies there as the swizzled tiles want it, so a chunk is one bulk copy and its V.  mLSTM (kMem): Q and K are the
+// projection's rows; alpha is applied to O^T's first product, and w V is split into two terms here.
+//
+// 17 warps: 0-7 own the state (a thread has a value column and half of the channels: scales, splits and writes it back),
+// 8-11 read O and store rows, 12-15 load (and form w V, n and the denominators), 16 issues the products.  The chain of a chunk
+// is state -> update -> state; O's products run beside the next chunk's scaling and splitting.
+//
+// Bound: that chain (about 1,500 cycles a chunk, 512 of them the update's products), so a sequence's chunks take their time one
+// after the other.  Where sequences, heads and column blocks are too few for the SMs, sequences are cut into segments: a pass
+// over each segment from a zero state (kState: no O), a join that turns the segments' own states into the states in front of
+// them, and the full pass over all segments at once.
+#pragma once
+#include "state_chunk.cuh"
+#include "tcgen05.cuh"
+
+namespace mv {
+
+constexpr int kWalkThreads = 17 * 32, kWalkCols = 128;
+constexpr int kSlab = kChunk * 128;                       // bytes of 64 rows of 64 bf16 values
+constexpr int kWalkV = 2 * kSlab;
+
+// Byte offset of element (row, col) in a tile of 64 rows, slabs of 64 columns, 128-byte swizzle.
+__host__ __device__ constexpr int tile_at(int row, int col) {
+  return (col >> 6) * kSlab + row * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4) + (col & 7) * 2;
+}
+
+// Scratch of a chunk and head.  kMem: [A hi, A lo, vectors]; else [Q hi, Q lo, K hi, K lo, A hi, A lo, decays].
+template <int K, bool kMem> struct WalkBlob {
+  static constexpr int kT = K / 64 * kSlab;               // bytes of a tile of 64 tokens x K
+  static constexpr int kQ = 0, kK = 2 * kT, kA = kMem ? 0 : 4 * kT, kVec = kA + 2 * kSlab;
+  static constexpr int kFloats = kMem ? 4 * kChunk + K + 4 : K;
+  // vectors of kMem, in floats
+  static constexpr int kAlpha = 0, kWrite = kChunk, kRow = 2 * kChunk, kFloor = 3 * kChunk, kSum = 4 * kChunk, kDecay = kSum + K;
+  static constexpr int64_t kBytes = kVec + kFloats * 4;
+};
+// One stage of shared memory: the blob, then for kMem Q and K, then V, then for kMem w V in two terms.
+template <int K, bool kMem> struct WalkStage {
+  using B = WalkBlob<K, kMem>;
+  static constexpr int kQ = (static_cast<int>(B::kBytes) + 1023) / 1024 * 1024, kK = kQ + (kMem ? B::kT : 0);
+  static constexpr int kV = kK + (kMem ? B::kT : 0), kW = kV + kWalkV, kBytes = kW + (kMem ? 2 * kWalkV : 0);
+  static constexpr int kSmem = 2 * kBytes + kChunk * kWalkCols * 2 + 1024;      // stages, rows of O, alignment
+};
+
+struct WalkParams {
+  __nv_bfloat16* out; int64_t out_stride;
+  float* den;                                             // kMem
+  const __nv_bfloat16 *q, *k, *v; int64_t stride;         // q and k: kMem
+  const int32_t *cu, *slots, *start;
+  int num_seqs;
+  float *state, *n_state; int num_slots, heads, K, V;
+  const unsigned char* scratch;
+  int seg_chunks;                                         // chunks of a segment, 0: sequences are whole
+  float *seg_state, *seg_n, *seg_decay;                   // per segment and head: K x V, K (kMem), K
+  int* error_word;
+};
+
+// Segment x of the batch: its sequence and its place in it.  Whole warp; false past the last.
+__device__ __forceinline__ bool find_segment(const int32_t* cu, int num_seqs, int seg_chunks, int x, int& seq, int& seg) {
+  const int lane = threadIdx.x & 31, tokens = seg_chunks * kChunk;
+  int base = 0;
+  for (int b = 0; b < num_seqs; b += 32) {
+    const int s = b + lane, n = s < num_seqs ? (max(cu[s + 1] - cu[s], 0) + tokens - 1) / tokens : 0;
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    const uint32_t past = __ballot_sync(0xffffffffu, base + incl > x);
+    if (past) {
+      const int at = __ffs(past) - 1;
+      seq = b + at;
+      seg = x - base - __shfl_sync(0xffffffffu, incl - n, at);
+      return true;
+    }
+    base += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  return false;
+}
+__device__ __forceinline__ int segments_before(const int32_t* cu, int s, int seg_chunks) {
+  int n = 0;
+  for (int i = threadIdx.x & 31; i < s; i += 32) n += (max(cu[i + 1] - cu[i], 0) + seg_chunks * kChunk - 1) / (seg_chunks * kChunk);
+  return __reduce_add_sync(0xffffffffu, n);
+}
+
+namespace tc {
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// Four K = 16 steps, A and B in shared memory, by the elected lane of a converged warp; descriptors move by kA and kB units.
+template <int kA, int kB>
+__device__ __forceinline__ void mma_ss_4(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, bool accum) {
+  const uint32_t acc = accum ? 1u : 0u;
+  asm volatile(
+      "{\n\t.reg .pred pe, pt, pf;\n\t.reg .b64 da, db;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
+      "setp.eq.u32 pt, %3, %3;\n\t"
+      "setp.ne.u32 pf, %4, 0;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, pf;\n\t"
+      "add.s64 da, %1, %5;\n\tadd.s64 db, %2, %6;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, pt;\n\t"
+      "add.s64 da, %1, %7;\n\tadd.s64 db, %2, %8;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, pt;\n\t"
+      "add.s64 da, %1, %9;\n\tadd.s64 db, %2, %10;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, pt;\n\t}"
+      ::"r"(d_tmem), "l"(a), "l"(b), "r"(idesc), "r"(acc), "n"(kA), "n"(kB), "n"(2 * kA), "n"(2 * kB), "n"(3 * kA), "n"(3 * kB)
+      : "memory");
+}
+// The same with A in tensor memory, eight columns a step.
+template <int kB>
+__device__ __forceinline__ void mma_ts_4(uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc, bool accum) {
+  const uint32_t acc = accum ? 1u : 0u;
+  asm volatile(
+      "{\n\t.reg .pred pe, pt, pf;\n\t.reg .b64 db;\n\t.reg .b32 ta;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
+      "setp.eq.u32 pt, %3, %3;\n\t"
+      "setp.ne.u32 pf, %4, 0;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, pf;\n\t"
+      "add.u32 ta, %1, 8;\n\tadd.s64 db, %2, %5;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %3, pt;\n\t"
+      "add.u32 ta, %1, 16;\n\tadd.s64 db, %2, %6;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %3, pt;\n\t"
+      "add.u32 ta, %1, 24;\n\tadd.s64 db, %2, %7;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [ta], db, %3, pt;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b), "r"(idesc), "r"(acc), "n"(kB), "n"(2 * kB), "n"(3 * kB) : "memory");
+}
+}  // namespace tc
+
+enum WalkBar { WB_BLOB = 0, WB_FULL = 2, WB_EMPTY = 4, WB_SREADY = 6, WB_SDONE, WB_ODONE, WB_OFREE, WB_COUNT };
+
+template <int K, bool kMem, bool kState>
+__global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const WalkParams p) {
+  using B = WalkBlob<K, kMem>;
+  using St = WalkStage<K, kMem>;
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ uint64_t s_bar[WB_COUNT];
+  __shared__ uint32_t s_tmem;
+  __shared__ volatile int s_abort;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y;
+  const int p0 = blockIdx.z * kWalkCols, pw = min(kWalkCols, p.V - p0);
+  // what this CTA walks
+  int s, seg = 0, unit = blockIdx.x;
+  if (p.seg_chunks) {
+    if (!find_segment(p.cu, p.num_seqs, p.seg_chunks, unit, s, seg)) return;      // uniform: the grid is an upper bound
+  } else {
+    s = unit;
+  }
+  const int n_all = p.cu[s + 1] - p.cu[s];
+  if (n_all <= 0) return;
+  const int seq_chunks = (n_all + kChunk - 1) / kChunk, c0 = seg * p.seg_chunks;
+  const int chunks = p.seg_chunks ? min(p.seg_chunks, seq_chunks - c0) : seq_chunks;
+  const bool last_seg = c0 + chunks == seq_chunks;
+  if (kState && last_seg) return;                          // nobody starts behind it
+  const int first = p.cu[s] + c0 * kChunk, n_tok = n_all - c0 * kChunk;
+  const int chunk0 = chunks_before(p.cu, s) + c0;
+  const int slot = p.slots[s], st0 = p.start[s];
+  const bool live = slot >= 0 && slot < p.num_slots && st0 >= 0;
+  const int64_t pair = (static_cast<int64_t>(live ? slot : 0) * p.heads + h), seg_pair = static_cast<int64_t>(unit) * p.heads + h;
+
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  unsigned char* smem = smem_raw + (base - smem_u32(smem_raw));
+  auto bar = [&](int i) { return smem_u32(&s_bar[i]); };
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(bar(WB_BLOB + i), 1);
+      tc::mbar_init(bar(WB_FULL + i), 128);
+      tc::mbar_init(bar(WB_EMPTY + i), kMem && !kState ? 1 + 128 : 1);
+    }
+    tc::mbar_init(bar(WB_SREADY), 256);
+    tc::mbar_init(bar(WB_SDONE), 1);
+    tc::mbar_init(bar(WB_ODONE), 1);
+    tc::mbar_init(bar(WB_OFREE), 128);
+    tc::mbar_fence_init();
+    s_abort = 0;
+  }
+  if (warp == 16) {
+    tc::tmem_alloc(smem_u32(&s_tmem), 512);
+    tc::tmem_relinquish();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = s_tmem;
+  // columns: S, two buffers of [hi | lo], then O (kMem: its two products)
+  const uint32_t tS = tmem, tHL = tmem + 128, tO = tmem + 384;
+  auto wait = [&](int b, int parity, int where) { tc::mbar_wait(bar(b), parity, &s_abort, p.error_word, where); };
+  auto stage_at = [&](int i) { return (i & 1) * St::kBytes; };
+
+  if (warp < 8) {
+    // ---------------------------------------------------------------- the state
+    const int row = (warp & 3) * 32 + lane, ch0 = (warp >> 2) * (K / 2);
+    const bool on = row < pw;
+    const uint32_t lanes = static_cast<uint32_t>(warp & 3) << 21;
+    float S[K / 2];
+    {
+      const float* src = p.seg_chunks ? p.seg_state + seg_pair * p.K * p.V : p.state + pair * p.K * p.V;
+      const bool has = !kState && on && (p.seg_chunks || (live && st0 > 0));
+#pragma unroll
+      for (int c = 0; c < K / 2; ++c)
+        S[c] = has && ch0 + c < p.K ? src[static_cast<int64_t>(ch0 + c) * p.V + p0 + row] : 0.f;
+    }
+    auto read_state = [&] {
+#pragma unroll
+      for (int c = 0; c < K / 2; c += 32) tc::tmem_ld32(tS + lanes + ch0 + c, *reinterpret_cast<uint32_t(*)[32]>(S + c));
+      tc::wait_ld();
+    };
+    for (int i = 0; i < chunks; ++i) {
+      const unsigned char* st = smem + stage_at(i);
+      if (i > 0) {
+        wait(WB_SDONE, (i - 1) & 1, 1);
+        tc::fence_after_sync();
+        read_state();
+      }
+      wait(WB_BLOB + (i & 1), (i >> 1) & 1, 2);
+      const float* vec = reinterpret_cast<const float*>(st + B::kVec);
+      const uint32_t hl = tHL + (i & 1) * 128 + lanes + ch0 / 2;
+#pragma unroll
+      for (int c = 0; c < K / 2; c += 16) {
+        if (!kState) {
+          uint32_t hi[8], lo[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) split2(S[c + 2 * e], S[c + 2 * e + 1], hi[e], lo[e]);
+          tc::tmem_st8(hl + c / 2, hi);
+          tc::tmem_st8(hl + 64 + c / 2, lo);
+        }
+        if constexpr (kMem) {
+          const float d = vec[B::kDecay];
+#pragma unroll
+          for (int e = 0; e < 16; ++e) S[c + e] *= d;
+        } else {
+#pragma unroll
+          for (int e = 0; e < 16; e += 4) {
+            const float4 d = *reinterpret_cast<const float4*>(vec + ch0 + c + e);
+            S[c + e] *= d.x; S[c + e + 1] *= d.y; S[c + e + 2] *= d.z; S[c + e + 3] *= d.w;
+          }
+        }
+        tc::tmem_st16(tS + lanes + ch0 + c, *reinterpret_cast<const uint32_t(*)[16]>(S + c));
+      }
+      tc::wait_st();
+      tc::fence_before_sync();
+      tc::mbar_arrive(bar(WB_SREADY));
+    }
+    wait(WB_SDONE, (chunks - 1) & 1, 3);
+    tc::fence_after_sync();
+    read_state();
+    if (on && (kState || (last_seg && live))) {
+      float* dst = kState ? p.seg_state + seg_pair * p.K * p.V : p.state + pair * p.K * p.V;
+#pragma unroll
+      for (int c = 0; c < K / 2; ++c)
+        if (ch0 + c < p.K) dst[static_cast<int64_t>(ch0 + c) * p.V + p0 + row] = S[c];
+    }
+  } else if (warp < 12) {
+    // ---------------------------------------------------------------- results
+    if constexpr (!kState) {
+      const int t4 = tid - 256, row = (warp & 3) * 32 + lane;
+      const uint32_t lanes = static_cast<uint32_t>(warp & 3) << 21;
+      __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(smem + 2 * St::kBytes);
+      for (int i = 0; i < chunks; ++i) {
+        wait(WB_ODONE, i & 1, 4);
+        tc::fence_after_sync();
+        const float* vec = reinterpret_cast<const float*>(smem + stage_at(i) + B::kVec);
+        uint32_t o[64];
+#pragma unroll
+        for (int c = 0; c < 64; c += 32) tc::tmem_ld32(tO + lanes + c, *reinterpret_cast<uint32_t(*)[32]>(o + c));
+        tc::wait_ld();
+        if constexpr (kMem) {
+#pragma unroll
+          for (int c = 0; c < 64; c += 16) {
+            uint32_t a[16];
+            tc::tmem_ld16(tO + 64 + lanes + c, a);
+            tc::wait_ld();
+#pragma unroll
+            for (int e = 0; e < 16; e += 4) {
+              const float4 al = *reinterpret_cast<const float4*>(vec + B::kAlpha + c + e);
+              o[c + e] = __float_as_uint(fmaf(__uint_as_float(o[c + e]), al.x, __uint_as_float(a[e])));
+              o[c + e + 1] = __float_as_uint(fmaf(__uint_as_float(o[c + e + 1]), al.y, __uint_as_float(a[e + 1])));
+              o[c + e + 2] = __float_as_uint(fmaf(__uint_as_float(o[c + e + 2]), al.z, __uint_as_float(a[e + 2])));
+              o[c + e + 3] = __float_as_uint(fmaf(__uint_as_float(o[c + e + 3]), al.w, __uint_as_float(a[e + 3])));
+            }
+          }
+          tc::mbar_arrive(bar(WB_EMPTY + (i & 1)));        // the stage's alpha is read
+        }
+        tc::fence_before_sync();
+        tc::mbar_arrive(bar(WB_OFREE));
+        asm volatile("bar.sync 1, 128;" ::: "memory");     // the rows of the chunk before are stored
+#pragma unroll
+        for (int t = 0; t < kChunk; ++t) rows[t * kWalkCols + row] = __float2bfloat16_rn(__uint_as_float(o[t]));
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        const int nt = min(kChunk, n_tok - i * kChunk);
+        __nv_bfloat16* dst = p.out + (static_cast<int64_t>(first) + i * kChunk) * p.out_stride + static_cast<int64_t>(h) * p.V + p0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int r = j * 8 + (t4 >> 4), c = (t4 & 15) * 8;
+          if (r < nt && c < pw)
+            *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(r) * p.out_stride + c) = *reinterpret_cast<const uint4*>(rows + r * kWalkCols + c);
+        }
+      }
+    }
+  } else if (warp < 16) {
+    // ---------------------------------------------------------------- loads
+    const int t = tid - 384, lw = warp - 12;
+    const bool first_block = blockIdx.z == 0, keeps_n = kMem && first_block;
+    const __nv_bfloat16* v = p.v + static_cast<int64_t>(h) * p.V + p0;
+    float n[K / 32], prod = 1.f;                           // channels lane * (K / 32) ..; the segment's decay of channel t
+    if constexpr (kMem) {
+      const float* src = p.seg_chunks ? p.seg_n + seg_pair * p.K : p.n_state + pair * p.K;
+#pragma unroll
+      for (int e = 0; e < K / 32; ++e) {
+        const int ch = lane * (K / 32) + e;
+        n[e] = !kState && keeps_n && ch < p.K && (p.seg_chunks || (live && st0 > 0)) ? src[ch] : 0.f;
+      }
+    }
+    auto issue = [&](int i) {
+      const int s2 = i & 1, nt = min(kChunk, n_tok - i * kChunk);
+      const uint32_t st = base + stage_at(i);
+      if (i >= 2) wait(WB_EMPTY + s2, ((i >> 1) - 1) & 1, 5);
+      if ((kMem || kState) && i >= 2) asm volatile("bar.sync 2, 128;" ::: "memory");       // no loader reads the stage any more
+      if (t == 0) {
+        const unsigned char* src = p.scratch + (static_cast<int64_t>(chunk0 + i) * p.heads + h) * B::kBytes;
+        const uint32_t b = bar(WB_BLOB + s2);
+        if (kState && !kMem) {
+          tc::mbar_expect_tx(b, 2 * B::kT + B::kFloats * 4);
+          tc::bulk_load(st + B::kK, src + B::kK, 2 * B::kT, b);
+          tc::bulk_load(st + B::kVec, src + B::kVec, B::kFloats * 4, b);
+        } else if (kState) {
+          tc::mbar_expect_tx(b, B::kFloats * 4);
+          tc::bulk_load(st + B::kVec, src + B::kVec, B::kFloats * 4, b);
+        } else {
+          tc::mbar_expect_tx(b, static_cast<uint32_t>(B::kBytes));
+          tc::bulk_load(st, src, static_cast<uint32_t>(B::kBytes), b);
+        }
+      }
+      const int64_t row0 = static_cast<int64_t>(first) + i * kChunk;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int r = j * 8 + (t >> 4), c = (t & 15) * 8;
+        const bool ok = r < nt && c < pw;
+        cp_async16(st + St::kV + tile_at(r, c), ok ? v + (row0 + r) * p.stride + c : p.v, ok ? 16 : 0);
+      }
+      if constexpr (kMem) {
+#pragma unroll 4
+        for (int j = t; j < kChunk * (K / 8); j += 128) {
+          const int r = j / (K / 8), c = (j % (K / 8)) * 8;
+          const bool ok = r < nt && c < p.K;
+          const int64_t off = ok ? (row0 + r) * p.stride + h * p.K + c : 0;
+          if (!kState) cp_async16(st + St::kQ + tile_at(r, c), p.q + off, ok ? 16 : 0);
+          cp_async16(st + St::kK + tile_at(r, c), p.k + off, ok ? 16 : 0);
+        }
+      }
+    };
+    issue(0);
+    cp_async_commit();
+    for (int i = 0; i < chunks; ++i) {
+      if (i + 1 < chunks) issue(i + 1);
+      cp_async_commit();
+      cp_async_wait<1>();
+      unsigned char* st = smem + stage_at(i);
+      const float* vec = reinterpret_cast<const float*>(st + B::kVec);
+      if constexpr (kMem) {
+        wait(WB_BLOB + (i & 1), (i >> 1) & 1, 6);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {                      // w V of the pieces this thread has fetched
+          const int r = j * 8 + (t >> 4), at = tile_at(r, (t & 15) * 8);
+          const float w = vec[B::kWrite + r];
+          const uint4 x = *reinterpret_cast<const uint4*>(st + St::kV + at);
+          const uint32_t xs[4] = {x.x, x.y, x.z, x.w};
+          uint32_t hi[4], lo[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xs[e]));
+            split2(f.x * w, f.y * w, hi[e], lo[e]);
+          }
+          *reinterpret_cast<uint4*>(st + St::kW + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          *reinterpret_cast<uint4*>(st + St::kW + kWalkV + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        }
+      }
+      tc::fence_async_proxy();
+      tc::mbar_arrive(bar(WB_FULL + (i & 1)));
+      if (kState && first_block) {
+        wait(WB_BLOB + (i & 1), (i >> 1) & 1, 7);
+        if (t < K) prod *= kMem ? vec[B::kDecay] : vec[t];
+      }
+      if constexpr (kMem) {
+        if (keeps_n) {
+          constexpr int kPer = K / 32;
+          if (!kState) {
+            asm volatile("bar.sync 2, 128;" ::: "memory");               // Q is here
+            // sixteen tokens a warp: partial sums over a lane's channels, then halves change hands until a lane has one token
+            float d[16];
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+              const unsigned char* qr = st + St::kQ + tile_at(lw * 16 + r, lane * kPer);
+              d[r] = 0.f;
+#pragma unroll
+              for (int e = 0; e < kPer; e += 2) {
+                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(qr + e * 2));
+                d[r] = fmaf(n[e + 1], f.y, fmaf(n[e], f.x, d[r]));
+              }
+            }
+#pragma unroll
+            for (int half = 8; half >= 1; half >>= 1) {
+              const bool up = lane & (2 * half);
+#pragma unroll
+              for (int r = 0; r < half; ++r) {
+                const float keep = up ? d[r + half] : d[r], give = up ? d[r] : d[r + half];
+                d[r] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * half);
+              }
+            }
+            const float dot = d[0] + __shfl_xor_sync(0xffffffffu, d[0], 1);
+            const int tok = lw * 16 + (lane >> 1);
+            if (!(lane & 1) && tok < min(kChunk, n_tok - i * kChunk))
+              p.den[(static_cast<int64_t>(first) + i * kChunk + tok) * p.heads + h] =
+                  fmaxf(fabsf(fmaf(vec[B::kAlpha + tok], dot, vec[B::kRow + tok])), vec[B::kFloor + tok]) + kMemFloor;
+          }
+#pragma unroll
+          for (int e = 0; e < kPer; ++e) n[e] = fmaf(vec[B::kDecay], n[e], vec[B::kSum + lane * kPer + e]);
+        }
+      }
+    }
+    cp_async_wait<0>();
+    if (kState && first_block && t < p.K) p.seg_decay[seg_pair * p.K + t] = prod;
+    if constexpr (kMem) {
+      if (keeps_n && lw == 0 && (kState || (last_seg && live))) {
+        float* dst = kState ? p.seg_n + seg_pair * p.K : p.n_state + pair * p.K;
+#pragma unroll
+        for (int e = 0; e < K / 32; ++e)
+          if (lane * (K / 32) + e < p.K) dst[lane * (K / 32) + e] = n[e];
+      }
+    }
+    if (s_abort && t == 0)                                 // a bulk copy may still be on its way
+      for (int i = max(0, chunks - 2); i < chunks; ++i) tc::mbar_wait_timed(bar(WB_BLOB + (i & 1)), (i >> 1) & 1);
+  } else {
+    // ---------------------------------------------------------------- products
+    constexpr uint32_t kMN = 1u << 15;                     // A is MN-major
+    constexpr uint32_t kUpdate = tc::instr_desc_f16(1, 1, true, 128, K) | kMN, kRead = tc::instr_desc_f16(1, 1, false, 128, kChunk),
+                       kLocal = kRead | kMN;
+    auto mn = [&](uint32_t at) { return tc::desc64(tc::desc_lo(at, kSlab), tc::kDescHiSw128Sbo1024); };
+    auto km = [&](uint32_t at) { return tc::desc64(tc::desc_lo(at, 16), tc::kDescHiSw128Sbo1024); };
+    for (int i = 0; i < chunks; ++i) {
+      const uint32_t st = base + stage_at(i);
+      wait(WB_BLOB + (i & 1), (i >> 1) & 1, 8);
+      wait(WB_FULL + (i & 1), (i >> 1) & 1, 9);
+      wait(WB_SREADY, i & 1, 10);
+      __syncwarp();
+      tc::fence_after_sync();
+      if constexpr (kMem) {
+        tc::mma_ss_4<128, 128>(tS, mn(st + St::kW), mn(st + St::kK), kUpdate, true);
+        tc::mma_ss_4<128, 128>(tS, mn(st + St::kW + kWalkV), mn(st + St::kK), kUpdate, true);
+      } else {
+        tc::mma_ss_4<128, 128>(tS, mn(st + St::kV), mn(st + B::kK), kUpdate, true);
+        tc::mma_ss_4<128, 128>(tS, mn(st + St::kV), mn(st + B::kK + B::kT), kUpdate, true);
+      }
+      if constexpr (kState) {
+        tc::commit_elected(bar(WB_SDONE), bar(WB_EMPTY + (i & 1)), true);
+      } else {
+        tc::commit_elected(bar(WB_SDONE), 0, false);
+        if (i > 0) wait(WB_OFREE, (i - 1) & 1, 11);
+        __syncwarp();
+        tc::fence_after_sync();
+        const uint32_t hi = tHL + (i & 1) * 128, lo = hi + 64, q = kMem ? st + St::kQ : st + B::kQ;
+#pragma unroll
+        for (int k = 0; k < K / 64; ++k) {
+          tc::mma_ts_4<2>(tO, hi + k * 32, km(q + k * kSlab), kRead, k > 0);
+          tc::mma_ts_4<2>(tO, lo + k * 32, km(q + k * kSlab), kRead, true);
+          if (!kMem) tc::mma_ts_4<2>(tO, hi + k * 32, km(q + B::kT + k * kSlab), kRead, true);
+        }
+        const uint32_t o2 = kMem ? tO + 64 : tO;
+        tc::mma_ss_4<128, 2>(o2, mn(st + St::kV), km(st + B::kA), kLocal, !kMem);
+        tc::mma_ss_4<128, 2>(o2, mn(st + St::kV), km(st + B::kA + kSlab), kLocal, true);
+        tc::commit_elected(bar(WB_ODONE), bar(WB_EMPTY + (i & 1)), true);
+      }
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 16) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, 512);
+  }
+}
+
+// The segments' own states become the states in front of them: per sequence, head and eight channels.
+constexpr int kJoinThreads = 256, kJoinBatch = 8;
+template <bool kMem>
+__global__ void __launch_bounds__(kJoinThreads) chunk_join_kernel(const WalkParams p) {
+  const int s = blockIdx.x, h = blockIdx.y, ch = blockIdx.z * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int n_tok = p.cu[s + 1] - p.cu[s];
+  if (n_tok <= 0) return;
+  const int per = p.seg_chunks * kChunk, segs = (n_tok + per - 1) / per, u0 = segments_before(p.cu, s, p.seg_chunks);
+  if (ch >= p.K) return;
+  const int slot = p.slots[s], st0 = p.start[s];
+  const bool has = slot >= 0 && slot < p.num_slots && st0 > 0;
+  const int64_t pair = static_cast<int64_t>(has ? slot : 0) * p.heads + h, step = static_cast<int64_t>(p.heads) * p.K * p.V;
+  auto join = [&](float first, float* at, int64_t stride) {
+    float x = first;
+    for (int g0 = 0; g0 < segs; g0 += kJoinBatch) {
+      float own[kJoinBatch], d[kJoinBatch];
+#pragma unroll
+      for (int j = 0; j < kJoinBatch; ++j) {
+        const bool ok = g0 + j < segs - 1;
+        own[j] = ok ? at[(g0 + j) * stride] : 0.f;
+        d[j] = ok ? p.seg_decay[(static_cast<int64_t>(u0 + g0 + j) * p.heads + h) * p.K + ch] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < kJoinBatch; ++j)
+        if (g0 + j < segs) {
+          at[(g0 + j) * stride] = x;
+          x = fmaf(x, d[j], own[j]);
+        }
+    }
+  };
+  for (int v = lane; v < p.V; v += 32)
+    join(has ? p.state[(pair * p.K + ch) * p.V + v] : 0.f,
+         p.seg_state + ((static_cast<int64_t>(u0) * p.heads + h) * p.K + ch) * p.V + v, step);
+  if (kMem && lane == 0)
+    join(has ? p.n_state[pair * p.K + ch] : 0.f, p.seg_n + (static_cast<int64_t>(u0) * p.heads + h) * p.K + ch,
+         static_cast<int64_t>(p.heads) * p.K);
+}
+
+// The sizes the walk takes; the register form (state_chunk.cuh) keeps the narrow ones, where most of 128 lanes would idle.
+inline bool walk_takes(int K, int V) { return K > 32 && V > 64; }
+// Chunks of a segment, or 0 for whole sequences.  A segment costs a second, lighter pass, so sequences are cut only where that
+// brings at least three times as many CTAs, none shorter than four chunks, all of them within one wave.
+inline int walk_segment(int64_t tokens, int num_seqs, int heads, int V) {
+  const int64_t blocks = static_cast<int64_t>(heads) * ((V + kWalkCols - 1) / kWalkCols);
+  const int64_t all = kNumSMs / blocks;                     // segments there is room for
+  if (num_seqs <= 0 || all < 3 * num_seqs) return 0;
+  const int64_t room = num_seqs > 1 ? all - num_seqs : all; // each sequence's last segment may be a short one
+  const int64_t chunks = (tokens + kChunk - 1) / kChunk, per = std::max<int64_t>(4, (chunks + room - 1) / room);
+  return chunks > per * num_seqs ? static_cast<int>(per) : 0;
+}
+inline int64_t walk_segments(int64_t tokens, int num_seqs, int per) { return per ? tokens / (per * kChunk) + std::min<int64_t>(num_seqs, tokens) : 0; }
+// Floats of the segments' states, n and decays.
+inline int64_t walk_segment_floats(int64_t tokens, int num_seqs, int heads, int K, int V) {
+  return walk_segments(tokens, num_seqs, walk_segment(tokens, num_seqs, heads, V)) * heads * (static_cast<int64_t>(K) * V + 2 * K);
+}
+
+// scratch holds the chunks' blobs, `segments` (16-byte aligned) walk_segment_floats.
+template <int K, bool kMem>
+int run_walk(const char* what, WalkParams p, int64_t tokens, float* segments, cudaStream_t st) {
+  p.seg_chunks = walk_segment(tokens, p.num_seqs, p.heads, p.V);
+  const int64_t units = p.seg_chunks ? walk_segments(tokens, p.num_seqs, p.seg_chunks) : p.num_seqs;
+  p.seg_state = segments;
+  p.seg_n = segments + units * p.heads * p.K * p.V;
+  p.seg_decay = p.seg_n + units * p.heads * p.K;
+  constexpr int smem = WalkStage<K, kMem>::kSmem;
+  static_assert(smem + 256 <= 227 * 1024, "a CTA's shared memory");
+  const dim3 grid(static_cast<unsigned>(units), p.heads, (p.V + kWalkCols - 1) / kWalkCols);
+  auto launch = [&](auto kernel, dim3 g) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return fail(MV_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+    kernel<<<g, kWalkThreads, smem, st>>>(p);
+    return check_launch(what);
+  };
+  if (p.seg_chunks) {
+    int rc = launch(chunk_walk_kernel<K, kMem, true>, grid);
+    if (rc) return rc;
+    chunk_join_kernel<kMem><<<dim3(p.num_seqs, p.heads, (p.K + 7) / 8), kJoinThreads, 0, st>>>(p);
+    rc = check_launch(what);
+    if (rc) return rc;
+  }
+  return launch(chunk_walk_kernel<K, kMem, false>, grid);
+}
+
+}  // namespace mv

@@ -7,13 +7,14 @@
 //                     against b at one token, on tensor cores in two terms each.  Below the diagonal that is the last token
 //                     before the block's rows, and every power of two is at most one.  On the diagonal it is the block's
 //                     middle; a block in which some channel forgets more than 2^-60 is summed channel by channel instead.
+// The walk over a sequence's chunks is chunk_walk.cuh's, or for narrow heads:
 // gla_chunk_kernel    per sequence, head and block of value columns: see state_chunk.cuh
 // V enters as the projection left it; the decayed operands, A and S in two terms.
-#include "state_chunk.cuh"
+#include "chunk_walk.cuh"
 
 namespace mv {
 
-constexpr int kGpThreads = 256;
+constexpr int kGpThreads = 512;
 
 struct GlaChunkParams {
   __nv_bfloat16* out; int64_t out_stride;
@@ -25,6 +26,7 @@ struct GlaChunkParams {
   int num_seqs;
   float* state; int num_slots, heads, K, V;
   unsigned char* scratch;                       // [chunk][head][Q hi, Q lo, K hi, K lo, A hi, A lo, 2^b_last]
+  bool z_vec;                                   // z's rows are whole 16-byte pieces
 };
 
 template <int K> struct GlaScratch {
@@ -33,65 +35,121 @@ template <int K> struct GlaScratch {
 };
 
 template <int K> struct GlaPrepShape {
-  static constexpr int kRow = K + 8, kB = K + 4;
-  static constexpr int kBytes = 2 * kChunk * kRow * 2 + (kChunk + 1) * kB * 4 + kChunk * 4;
+  static constexpr int kRow = K + 8;                     // bf16 rows of q and k, then fp32 rows of k's factors in the same place
+  // tables (block, channel): sum of a block's logarithms, and 2 to the power of what is in front of the block, of what follows it
+  // up to the chunk's end, and of the ways from its edges to its middle
+  enum { kTot, kFront, kBehind, kMidQ, kMidK, kTables };
+  static constexpr int kBytes = 2 * kChunk * kRow * 2 + (kChunk + 1) * kRow * 4 + kTables * 4 * K * 4 + kChunk * 4;
 };
 
-template <int K, bool kTime>
-__global__ void __launch_bounds__(kGpThreads) gla_prepare_kernel(const GlaChunkParams p) {
+// Two CTAs of 16 warps per SM.  A channel's two powers of a token, from the token to the edge of its block of 16, are formed once;
+// everything else is products with a block's: the operands relative to the chunk's ends, and A's blocks.
+// 1 x 16,384 tokens, 8 heads of 128: 168 us with powers formed per pair of blocks and logits read one by one
+template <int K, bool kTime, bool kWalk>
+__global__ void __launch_bounds__(kGpThreads, 2) gla_prepare_kernel(const GlaChunkParams p) {
   using Sh = GlaPrepShape<K>;
   using Sc = GlaScratch<K>;
+  constexpr int R = Sh::kRow, kPairs = K / 16;           // pairs of channels per thread
+  static_assert(kGpThreads == 512 && kChunk * K / 2 == kPairs * kGpThreads && 4 * K <= kGpThreads, "the split among threads");
   extern __shared__ __align__(16) unsigned char smem[];
-  __nv_bfloat16 *sQ = reinterpret_cast<__nv_bfloat16*>(smem), *sK = sQ + kChunk * Sh::kRow;
-  float* sB = reinterpret_cast<float*>(sK + kChunk * Sh::kRow) + Sh::kB;     // a row of zeros in front of token 0
-  float* sOwn = sB + kChunk * Sh::kB;                                        // A's diagonal, time mixing
+  __nv_bfloat16 *sQ = reinterpret_cast<__nv_bfloat16*>(smem), *sK = sQ + kChunk * R;
+  float* sKt = reinterpret_cast<float*>(smem);           // k 2^(end of its block - b), over sQ and sK
+  float* sB = reinterpret_cast<float*>(sK + kChunk * R) + R;       // a row of zeros in front of token 0
+  float* sQt = sB;                                       // q 2^(b - end of the block before), over sB
+  float* sTab = sB + kChunk * R;
+  float* sOwn = sTab + Sh::kTables * 4 * K;              // A's diagonal, time mixing
+  auto tab = [&](int which, int blk) { return sTab + (which * 4 + blk) * K; };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, h = blockIdx.y;
   int seq, chunk;
   if (!find_chunk(p.cu, p.num_seqs, blockIdx.x, seq, chunk)) return;     // uniform: the grid is an upper bound
   const int64_t first = p.cu[seq] + static_cast<int64_t>(chunk) * kChunk;
   const int nt = min(kChunk, static_cast<int>(p.cu[seq + 1] - first));
-  __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.scratch + (static_cast<int64_t>(blockIdx.x) * p.heads + h) * Sc::kBytes);
+  using Wb = WalkBlob<K, false>;
+  constexpr int64_t kBlob = kWalk ? Wb::kBytes : Sc::kBytes, kABytes = kWalk ? Wb::kA : Sc::kA * 2;
+  unsigned char* dst = p.scratch + (static_cast<int64_t>(blockIdx.x) * p.heads + h) * kBlob;
+  // columns c and c + 1 of tile x (Q hi, Q lo, K hi, K lo), and of A's term x
+  auto tile = [&](int x, int r, int c) -> uint32_t& {
+    return *reinterpret_cast<uint32_t*>(dst + (kWalk ? x * Wb::kT + tile_at(r, c) : (x * Sc::kVec + r * K + c) * 2));
+  };
+  auto local = [&](int x, int r, int c) -> uint32_t& {
+    return *reinterpret_cast<uint32_t*>(dst + kABytes + (kWalk ? x * kSlab + tile_at(r, c) : ((x * kChunk + r) * kChunk + c) * 2));
+  };
   {
     const uint32_t qd = smem_u32(sQ), kd = smem_u32(sK);
     for (int i = tid; i < kChunk * (K / 8); i += kGpThreads) {
       const int r = i / (K / 8), c = (i % (K / 8)) * 8;
       const bool ok = r < nt && c < p.K;
       const int64_t off = ok ? (first + r) * p.stride + h * p.K + c : 0;
-      cp_async16(qd + (r * Sh::kRow + c) * 2, p.q + off, ok ? 16 : 0);
-      cp_async16(kd + (r * Sh::kRow + c) * 2, p.k + off, ok ? 16 : 0);
+      cp_async16(qd + (r * R + c) * 2, p.q + off, ok ? 16 : 0);
+      cp_async16(kd + (r * R + c) * 2, p.k + off, ok ? 16 : 0);
     }
     cp_async_commit();
   }
-  for (int i = tid; i < kChunk * K; i += kGpThreads) {
-    const int r = i / K, c = i % K;
-    const int64_t at = (first + r) * p.z_stride + h * p.K + c;
-    float b = 0.f;
-    if (r < nt && c < p.K)
-      b = kTime ? time_log_decay(p.zf[at] + __bfloat162float(p.w0[h * p.K + c])) : channel_log_decay(__bfloat162float(p.z[at]), p.inv_tau);
-    sB[r * Sh::kB + c] = b * kLog2e;
-  }
-  for (int c = tid; c < Sh::kB; c += kGpThreads) sB[c - Sh::kB] = 0.f;
-  __syncthreads();
-  for (int i = tid; i < 4 * K; i += kGpThreads) {        // running sums of 16 tokens
-    float* b = sB + (i / K) * 16 * Sh::kB + i % K;
-    float run = 0.f;
+  auto log_decay = [&](float z, int c) {
+    return (kTime ? time_log_decay(z + __bfloat162float(p.w0[h * p.K + c])) : channel_log_decay(z, p.inv_tau)) * kLog2e;
+  };
+  if (p.z_vec) {                                         // rows of z on 16-byte boundaries, K a multiple of eight
+    for (int i = tid; i < kChunk * (K / 8); i += kGpThreads) {
+      const int r = i / (K / 8), c = (i % (K / 8)) * 8;
+      float b[8] = {};
+      if (r < nt && c < p.K) {
+        const int64_t at = (first + r) * p.z_stride + h * p.K + c;
+        float z[8];
+        if constexpr (kTime) {
+          const float4 x = *reinterpret_cast<const float4*>(p.zf + at), y = *reinterpret_cast<const float4*>(p.zf + at + 4);
+          z[0] = x.x; z[1] = x.y; z[2] = x.z; z[3] = x.w; z[4] = y.x; z[5] = y.y; z[6] = y.z; z[7] = y.w;
+        } else {
+          const uint4 raw = *reinterpret_cast<const uint4*>(p.z + at);
+          const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      run += b[r * Sh::kB];
-      b[r * Sh::kB] = run;
+          for (int e = 0; e < 4; ++e) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[e]));
+            z[2 * e] = f.x;
+            z[2 * e + 1] = f.y;
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) b[e] = log_decay(z[e], c + e);
+      }
+      float4* to = reinterpret_cast<float4*>(sB + r * R + c);
+      to[0] = make_float4(b[0], b[1], b[2], b[3]);
+      to[1] = make_float4(b[4], b[5], b[6], b[7]);
+    }
+  } else {
+    for (int i = tid; i < kChunk * K; i += kGpThreads) {
+      const int r = i / K, c = i % K;
+      const int64_t at = (first + r) * p.z_stride + h * p.K + c;
+      sB[r * R + c] = r < nt && c < p.K ? log_decay(kTime ? p.zf[at] : __bfloat162float(p.z[at]), c) : 0.f;
     }
   }
+  for (int c = tid; c < R; c += kGpThreads) sB[c - R] = 0.f;
   __syncthreads();
-  for (int c = tid; c < K; c += kGpThreads) {            // ... joined
-    float run = sB[15 * Sh::kB + c];
+  {                                                      // running sums: of 16 tokens, joined through the blocks' totals
+    const int blk = tid / K, c = tid % K;
+    float run[16], sum = 0.f;
+    if (blk < 4) {
 #pragma unroll
-    for (int blk = 1; blk < 4; ++blk) {
-      const float mine = sB[(blk * 16 + 15) * Sh::kB + c];
-#pragma unroll
-      for (int r = 0; r < 16; ++r) sB[(blk * 16 + r) * Sh::kB + c] += run;
-      run += mine;
+      for (int r = 0; r < 16; ++r) run[r] = sum += sB[(blk * 16 + r) * R + c];
+      tab(Sh::kTot, blk)[c] = sum;
     }
-    reinterpret_cast<float*>(dst + Sc::kDecay)[c] = fast_exp2(sB[(kChunk - 1) * Sh::kB + c]);
+    __syncthreads();
+    if (blk < 4) {
+      float front = 0.f, all = 0.f;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const float t = tab(Sh::kTot, x)[c];
+        if (x < blk) front += t;
+        all += t;
+      }
+#pragma unroll
+      for (int r = 0; r < 16; ++r) sB[(blk * 16 + r) * R + c] = front + run[r];
+      const float end = front + sum;
+      tab(Sh::kFront, blk)[c] = fast_exp2(front);
+      tab(Sh::kBehind, blk)[c] = fast_exp2(all - end);
+      tab(Sh::kMidQ, blk)[c] = fast_exp2(-run[7]);
+      tab(Sh::kMidK, blk)[c] = fast_exp2(run[7] - sum);
+      if (blk == 3) reinterpret_cast<float*>(dst + (kWalk ? Wb::kVec : Sc::kDecay * 2))[c] = fast_exp2(all);
+    }
   }
   cp_async_wait<0>();
   __syncthreads();
@@ -99,103 +157,124 @@ __global__ void __launch_bounds__(kGpThreads) gla_prepare_kernel(const GlaChunkP
     for (int t = warp; t < kChunk; t += kGpThreads / 32) {
       float own = 0.f;
       for (int c = lane; c < p.K; c += 32)
-        own = fmaf(__bfloat162float(sQ[t * Sh::kRow + c]) * __bfloat162float(p.bonus[h * p.K + c]), __bfloat162float(sK[t * Sh::kRow + c]), own);
+        own = fmaf(__bfloat162float(sQ[t * R + c]) * __bfloat162float(p.bonus[h * p.K + c]), __bfloat162float(sK[t * R + c]), own);
       own = warp_sum(own);
       if (lane == 0) sOwn[t] = own;
     }
     __syncthreads();
   }
-  const float* sE = kTime ? sB - Sh::kB : sB;            // exponents beside q
-  {
-    uint32_t* o = reinterpret_cast<uint32_t*>(dst);
-    for (int i = tid; i < kChunk * K / 2; i += kGpThreads) {
-      const int r = i / (K / 2), c = (i % (K / 2)) * 2;
-      const float2 b = *reinterpret_cast<const float2*>(sB + r * Sh::kB + c), e = *reinterpret_cast<const float2*>(sE + r * Sh::kB + c);
-      const float2 last = *reinterpret_cast<const float2*>(sB + (kChunk - 1) * Sh::kB + c);
-      const float2 q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sQ + r * Sh::kRow + c));
-      const float2 k = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sK + r * Sh::kRow + c));
-      uint32_t hi, lo;
-      split2(q.x * p.q_scale * fast_exp2(e.x), q.y * p.q_scale * fast_exp2(e.y), hi, lo);
-      o[i] = hi;
-      o[Sc::kVec / 2 + i] = lo;
-      split2(k.x * fast_exp2(last.x - b.x), k.y * fast_exp2(last.y - b.y), hi, lo);
-      o[Sc::kVec + i] = hi;
-      o[Sc::kVec * 3 / 2 + i] = lo;
-    }
-  }
-  uint32_t* gA = reinterpret_cast<uint32_t*>(dst + Sc::kA);
+  const float* sE = kTime ? sB - R : sB;                 // exponents beside q
   auto put = [&](int t, int j, float x, float y) {
     uint32_t hi, lo;
     split2(x, y, hi, lo);
-    gA[(t * kChunk + j) / 2] = hi;
-    gA[kChunk * kChunk / 2 + (t * kChunk + j) / 2] = lo;
+    local(0, t, j) = hi;
+    local(1, t, j) = lo;
   };
-  const int g = lane >> 2, c2 = (lane & 3) * 2;
-  // blocks 0 .. 5 below the diagonal, (1,0) (2,0) (2,1) (3,0) (3,1) (3,2), then the four on it
-#pragma unroll 1
-  for (int blk = warp; blk < 10; blk += kGpThreads / 32) {
-    const bool diag = blk >= 6;
-    const int bi = diag ? blk - 6 : blk == 0 ? 1 : blk < 3 ? 2 : 3, bj = diag ? bi : blk - bi * (bi - 1) / 2;
-    const float* ref = sB + (diag ? bi * 16 + 7 : bi * 16 - 1) * Sh::kB;
-    if (diag) {
-      float least = 0.f;
-      for (int c = lane; c < K; c += 32)
-        least = fminf(least, sB[(bi * 16 + 15) * Sh::kB + c] - (bi ? sB[(bi * 16 - 1) * Sh::kB + c] : 0.f));
-      if (__any_sync(0xffffffffu, least < -60.f)) {
-        for (int i = lane; i < 16 * 8; i += 32) {        // two neighbouring keys of one token
-          const int t = bi * 16 + (i >> 3), j = bi * 16 + (i & 7) * 2;
-          const int j_end = kTime ? t - 1 : t;
-          float x = 0.f, y = 0.f;
-          for (int c = 0; j <= j_end && c < K; ++c) {
-            const float q = __bfloat162float(sQ[t * Sh::kRow + c]), bt = sE[t * Sh::kB + c];
-            x = fmaf(q * __bfloat162float(sK[j * Sh::kRow + c]), fast_exp2(bt - sB[j * Sh::kB + c]), x);
-            if (j + 1 <= j_end) y = fmaf(q * __bfloat162float(sK[(j + 1) * Sh::kRow + c]), fast_exp2(bt - sB[(j + 1) * Sh::kB + c]), y);
-          }
-          if (kTime) {
-            if (j == t) x = sOwn[t];
-            if (j + 1 == t) y = sOwn[t];
-          }
-          put(t, j, x * p.q_scale, y * p.q_scale);
+  // Blocks 0 .. 5 of A below the diagonal, (1,0) (2,0) (2,1) (3,0) (3,1) (3,2), then the four on it: one per warp.
+  const bool diag = warp >= 6;
+  const int bi = diag ? warp - 6 : warp == 0 ? 1 : warp < 3 ? 2 : 3, bj = diag ? bi : warp - bi * (bi - 1) / 2;
+  bool mine = warp < 10;
+  if (mine && diag) {
+    float least = 0.f;
+    for (int c = lane; c < K; c += 32) least = fminf(least, tab(Sh::kTot, bi)[c]);
+    if (__any_sync(0xffffffffu, least < -60.f)) {        // more than a block's factors can hold: channel by channel
+      mine = false;
+      for (int i = lane; i < 16 * 8; i += 32) {          // two neighbouring keys of one token
+        const int t = bi * 16 + (i >> 3), j = bi * 16 + (i & 7) * 2;
+        const int j_end = kTime ? t - 1 : t;
+        float x = 0.f, y = 0.f;
+        for (int c = 0; j <= j_end && c < K; ++c) {
+          const float q = __bfloat162float(sQ[t * R + c]), bt = sE[t * R + c];
+          x = fmaf(q * __bfloat162float(sK[j * R + c]), fast_exp2(bt - sB[j * R + c]), x);
+          if (j + 1 <= j_end) y = fmaf(q * __bfloat162float(sK[(j + 1) * R + c]), fast_exp2(bt - sB[(j + 1) * R + c]), y);
         }
-        continue;
-      }
-    }
-    float acc[2][4] = {};
-#pragma unroll 2
-    for (int kb = 0; kb < K; kb += 16) {
-      uint32_t ah[4], al[4], bh[4], bl[4];
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        // A: rows g, g + 8 of the block's tokens, channels c2 and c2 + 8;  B: n-tiles of eight keys each
-        const int c = kb + c2 + (x >> 1) * 8, t = bi * 16 + g + (x & 1) * 8;
-        const float2 r = *reinterpret_cast<const float2*>(ref + c), b = *reinterpret_cast<const float2*>(sE + t * Sh::kB + c);
-        const float2 q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sQ + t * Sh::kRow + c));
-        split2(q.x * fast_exp2(b.x - r.x), q.y * fast_exp2(b.y - r.y), ah[x], al[x]);
-        const int cj = kb + c2 + (x & 1) * 8, j = bj * 16 + g + (x >> 1) * 8;
-        const float2 rj = *reinterpret_cast<const float2*>(ref + cj), bb = *reinterpret_cast<const float2*>(sB + j * Sh::kB + cj);
-        const float2 k = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sK + j * Sh::kRow + cj));
-        split2(k.x * fast_exp2(rj.x - bb.x), k.y * fast_exp2(rj.y - bb.y), bh[x], bl[x]);
-      }
-#pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        Mma::run(acc[n], ah, bh[2 * n], bh[2 * n + 1]);
-        Mma::run(acc[n], al, bh[2 * n], bh[2 * n + 1]);
-        Mma::run(acc[n], ah, bl[2 * n], bl[2 * n + 1]);
-      }
-    }
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int t = bi * 16 + g + half * 8, j = bj * 16 + n * 8 + c2;
-        float x = acc[n][2 * half], y = acc[n][2 * half + 1];
         if (kTime) {
           if (j == t) x = sOwn[t];
           if (j + 1 == t) y = sOwn[t];
         }
-        put(t, j, j <= t ? x * p.q_scale : 0.f, j + 1 <= t ? y * p.q_scale : 0.f);
+        put(t, j, x * p.q_scale, y * p.q_scale);
       }
+    }
   }
+  float2 qt[kPairs], kt[kPairs];
+#pragma unroll
+  for (int m = 0; m < kPairs; ++m) {
+    const int i = tid + m * kGpThreads, r = i / (K / 2), c = (i % (K / 2)) * 2, blk = r >> 4;
+    const float2 b = *reinterpret_cast<const float2*>(sB + r * R + c), e = *reinterpret_cast<const float2*>(sE + r * R + c);
+    const float2 ref = *reinterpret_cast<const float2*>(sB + (blk * 16 - 1) * R + c), end = *reinterpret_cast<const float2*>(sB + (blk * 16 + 15) * R + c);
+    const float2 front = *reinterpret_cast<const float2*>(tab(Sh::kFront, blk) + c), behind = *reinterpret_cast<const float2*>(tab(Sh::kBehind, blk) + c);
+    const float2 q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sQ + r * R + c));
+    const float2 k = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sK + r * R + c));
+    qt[m] = make_float2(q.x * fast_exp2(e.x - ref.x), q.y * fast_exp2(e.y - ref.y));
+    kt[m] = make_float2(k.x * fast_exp2(end.x - b.x), k.y * fast_exp2(end.y - b.y));
+    uint32_t hi, lo;
+    split2(qt[m].x * p.q_scale * front.x, qt[m].y * p.q_scale * front.y, hi, lo);
+    tile(0, r, c) = hi;
+    tile(1, r, c) = lo;
+    split2(kt[m].x * behind.x, kt[m].y * behind.y, hi, lo);
+    tile(2, r, c) = hi;
+    tile(3, r, c) = lo;
+  }
+  if (kWalk) zero_upper(tid, kGpThreads, [&](int r, int c, int x) -> uint32_t& { return local(x, r, c); });
+  __syncthreads();                                       // q, k and b are read
+#pragma unroll
+  for (int m = 0; m < kPairs; ++m) {
+    const int i = tid + m * kGpThreads, r = i / (K / 2), c = (i % (K / 2)) * 2;
+    *reinterpret_cast<float2*>(sQt + r * R + c) = qt[m];
+    *reinterpret_cast<float2*>(sKt + r * R + c) = kt[m];
+  }
+  __syncthreads();
+  if (!mine) return;
+  const int g = lane >> 2, c2 = (lane & 3) * 2;
+  const bool far = !diag && bj + 1 < bi;                 // blocks between the two
+  float acc[2][4] = {};
+#pragma unroll 2
+  for (int kb = 0; kb < K; kb += 16) {
+    uint32_t ah[4], al[4], bh[4], bl[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      // A: rows g, g + 8 of the block's tokens, channels c2 and c2 + 8;  B: n-tiles of eight keys each
+      const int c = kb + c2 + (x >> 1) * 8, t = bi * 16 + g + (x & 1) * 8;
+      float2 q = *reinterpret_cast<const float2*>(sQt + t * R + c);
+      if (diag) {
+        const float2 f = *reinterpret_cast<const float2*>(tab(Sh::kMidQ, bi) + c);
+        q.x *= f.x; q.y *= f.y;
+      } else if (far) {
+        float2 f = *reinterpret_cast<const float2*>(tab(Sh::kTot, bi - 1) + c);
+        if (bi - bj == 3) {
+          const float2 f2 = *reinterpret_cast<const float2*>(tab(Sh::kTot, 1) + c);
+          f.x += f2.x; f.y += f2.y;
+        }
+        q.x *= fast_exp2(f.x); q.y *= fast_exp2(f.y);
+      }
+      split2(q.x, q.y, ah[x], al[x]);
+      const int cj = kb + c2 + (x & 1) * 8, j = bj * 16 + g + (x >> 1) * 8;
+      float2 k = *reinterpret_cast<const float2*>(sKt + j * R + cj);
+      if (diag) {
+        const float2 f = *reinterpret_cast<const float2*>(tab(Sh::kMidK, bi) + cj);
+        k.x *= f.x; k.y *= f.y;
+      }
+      split2(k.x, k.y, bh[x], bl[x]);
+    }
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+      Mma::run(acc[n], ah, bh[2 * n], bh[2 * n + 1]);
+      Mma::run(acc[n], al, bh[2 * n], bh[2 * n + 1]);
+      Mma::run(acc[n], ah, bl[2 * n], bl[2 * n + 1]);
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int t = bi * 16 + g + half * 8, j = bj * 16 + n * 8 + c2;
+      float x = acc[n][2 * half], y = acc[n][2 * half + 1];
+      if (kTime) {
+        if (j == t) x = sOwn[t];
+        if (j + 1 == t) y = sOwn[t];
+      }
+      put(t, j, j <= t ? x * p.q_scale : 0.f, j + 1 <= t ? y * p.q_scale : 0.f);
+    }
 }
 
 template <int K> struct GlaChunkShape {
@@ -327,34 +406,50 @@ static int64_t gla_scratch_bytes(int K) {
 extern "C" int64_t mv_gla_chunk_workspace_bytes(int64_t tokens, int num_seqs, int heads, int dim, int vdim) {
   using namespace mv;
   if (tokens < 0 || num_seqs < 0 || heads <= 0 || !chunk_takes(dim, vdim)) return -1;
-  return chunk_bound(tokens, num_seqs) * heads * gla_scratch_bytes(dim);
+  const int64_t chunks = chunk_bound(tokens, num_seqs) * heads;
+  if (!walk_takes(dim, vdim)) return chunks * gla_scratch_bytes(dim);
+  return chunks * (dim <= 64 ? WalkBlob<64, false>::kBytes : WalkBlob<128, false>::kBytes) +
+         walk_segment_floats(tokens, num_seqs, heads, dim, vdim) * 4;
 }
 
 // Both recurrences; kTime: p.zf, p.w0 and p.bonus, else p.z and p.inv_tau.
 template <bool kTime>
-static int run_chunks(const char* what, const mv::GlaChunkParams& p, int64_t tokens, int64_t workspace_bytes, cudaStream_t st) {
+static int run_chunks(const char* what, const mv::GlaChunkParams& p, int64_t tokens, int64_t workspace_bytes, int* error_word, cudaStream_t st) {
   using namespace mv;
   const int num_seqs = p.num_seqs, heads = p.heads, dim = p.K, vdim = p.V;
   if (num_seqs < 0 || tokens < 0 || heads <= 0 || heads > 65535 || !chunk_takes(dim, vdim))
     return fail(MV_ERR_SHAPE, "%s: heads %d, dim %d, vdim %d", what, heads, dim, vdim);
   if (num_seqs == 0 || tokens == 0) return MV_OK;
-  if (!p.out || !p.q || !p.k || !p.v || !(kTime ? p.zf && p.w0 && p.bonus : p.z != nullptr) || !p.cu || !p.slots || !p.start || !p.state)
+  if (!p.out || !p.q || !p.k || !p.v || !(kTime ? p.zf && p.w0 && p.bonus : p.z != nullptr) || !p.cu || !p.slots || !p.start || !p.state || !error_word)
     return fail(MV_ERR_NULL, "%s: null pointer", what);
   if (!vec8_ok(p.out, p.out_stride, 2) || !vec8_ok(p.q, p.stride, 2) || !vec8_ok(p.k, p.stride, 2) || !vec8_ok(p.v, p.stride, 2))
     return fail(MV_ERR_ALIGN, "%s: rows must start on 16-byte boundaries", what);
   const int64_t chunks = chunk_bound(tokens, num_seqs);
-  if (!p.scratch || !aligned16(p.scratch) || workspace_bytes < chunks * heads * gla_scratch_bytes(dim))
+  if (!p.scratch || !aligned16(p.scratch) || workspace_bytes < mv_gla_chunk_workspace_bytes(tokens, num_seqs, heads, dim, vdim))
     return fail(MV_ERR_WORKSPACE, "%s: workspace", what);
+  auto prepare = [&](auto kernel, int bytes) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return fail(MV_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+    kernel<<<dim3(static_cast<unsigned>(chunks), heads), kGpThreads, bytes, st>>>(p);
+    return check_launch(what);
+  };
+  if (walk_takes(dim, vdim)) {
+    auto walk = [&](auto kk) {
+      constexpr int K = decltype(kk)::value;
+      const int rc = prepare(gla_prepare_kernel<K, kTime, true>, GlaPrepShape<K>::kBytes);
+      if (rc) return rc;
+      const WalkParams w{p.out, p.out_stride, nullptr, nullptr, nullptr, p.v, p.stride, p.cu, p.slots, p.start, num_seqs, p.state, nullptr,
+                         p.num_slots, heads, dim, vdim, p.scratch, 0, nullptr, nullptr, nullptr, error_word};
+      return run_walk<K, false>(what, w, tokens, reinterpret_cast<float*>(p.scratch + chunks * heads * WalkBlob<K, false>::kBytes), st);
+    };
+    return dim <= 64 ? walk(std::integral_constant<int, 64>{}) : walk(std::integral_constant<int, 128>{});
+  }
   return chunk_dispatch(dim, [&](auto kk) {
     constexpr int K = decltype(kk)::value;
-    constexpr int prep = GlaPrepShape<K>::kBytes;
-    cudaError_t e = cudaFuncSetAttribute(gla_prepare_kernel<K, kTime>, cudaFuncAttributeMaxDynamicSharedMemorySize, prep);
-    if (e != cudaSuccess) return fail(MV_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-    gla_prepare_kernel<K, kTime><<<dim3(static_cast<unsigned>(chunks), heads), kGpThreads, prep, st>>>(p);
-    int rc = check_launch(what);
+    const int rc = prepare(gla_prepare_kernel<K, kTime, false>, GlaPrepShape<K>::kBytes);
     if (rc) return rc;
     const int pb = chunk_columns(static_cast<int64_t>(num_seqs) * heads, vdim), smem = 2 * GlaChunkShape<K>::stage(pb);
-    e = cudaFuncSetAttribute(gla_chunk_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = cudaFuncSetAttribute(gla_chunk_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return fail(MV_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
     gla_chunk_kernel<K><<<dim3(num_seqs, heads, (vdim + pb - 1) / pb), kChunkThreads, smem, st>>>(p, pb);
     return check_launch(what);
@@ -365,25 +460,25 @@ extern "C" int mv_gla_chunk_scan(void* out, int64_t out_stride, const void* q, c
                                  const void* z, int64_t z_stride, float tau, const int32_t* cu, int num_seqs,
                                  int64_t tokens, const int32_t* slots, const int32_t* start, float* state, int num_slots,
                                  int heads, int dim, int vdim, float q_scale, void* workspace, int64_t workspace_bytes,
-                                 void* stream) {
+                                 int* error_word, void* stream) {
   using namespace mv;
   if (!(tau > 0.f)) return fail(MV_ERR_SHAPE, "gla_chunk_scan: tau %f", tau);
   auto c = [](const void* x) { return static_cast<const __nv_bfloat16*>(x); };
   const GlaChunkParams p{static_cast<__nv_bfloat16*>(out), out_stride, c(q), c(k), c(v), stride, c(z), z_stride, 1.f / tau, q_scale,
                          nullptr, nullptr, nullptr,
-                         cu, slots, start, num_seqs, state, num_slots, heads, dim, vdim, static_cast<unsigned char*>(workspace)};
-  return run_chunks<false>("gla_chunk_scan", p, tokens, workspace_bytes, static_cast<cudaStream_t>(stream));
+                         cu, slots, start, num_seqs, state, num_slots, heads, dim, vdim, static_cast<unsigned char*>(workspace), vec8_ok(z, z_stride, 2)};
+  return run_chunks<false>("gla_chunk_scan", p, tokens, workspace_bytes, error_word, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int mv_time_chunk_scan(void* out, int64_t out_stride, const void* r, const void* k, const void* v, int64_t stride,
                                   const float* z, int64_t z_stride, const void* w0, const void* bonus, const int32_t* cu,
                                   int num_seqs, int64_t tokens, const int32_t* slots, const int32_t* start, float* state,
                                   int num_slots, int heads, int dim, int vdim, void* workspace, int64_t workspace_bytes,
-                                  void* stream) {
+                                  int* error_word, void* stream) {
   using namespace mv;
   auto c = [](const void* x) { return static_cast<const __nv_bfloat16*>(x); };
   const GlaChunkParams p{static_cast<__nv_bfloat16*>(out), out_stride, c(r), c(k), c(v), stride, nullptr, z_stride, 1.f, 1.f,
                          z, c(w0), c(bonus),
-                         cu, slots, start, num_seqs, state, num_slots, heads, dim, vdim, static_cast<unsigned char*>(workspace)};
-  return run_chunks<true>("time_chunk_scan", p, tokens, workspace_bytes, static_cast<cudaStream_t>(stream));
+                         cu, slots, start, num_seqs, state, num_slots, heads, dim, vdim, static_cast<unsigned char*>(workspace), vec8_ok(z, z_stride, 4)};
+  return run_chunks<true>("time_chunk_scan", p, tokens, workspace_bytes, error_word, static_cast<cudaStream_t>(stream));
 }

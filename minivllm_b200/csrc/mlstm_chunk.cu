@@ -5,10 +5,11 @@
 //   S = e^(-M_last) S_0 + (w K)^T V,     w_j = e^(a_j - M_last);     n the same with V = 1
 //   denominator of t = max(|alpha_t q_t n_0 + sum_j A[t, j]|, e^-m_t) + 1e-6
 // mlstm_prepare_kernel  per chunk and head: the factors, A in two terms, its row sums, sum_j w_j k_j
+// The walk over a sequence's chunks is chunk_walk.cuh's, or for narrow heads:
 // mlstm_chunk_kernel    per sequence, head and block of value columns: see state_chunk.cuh.  The first block of columns also
 //                       carries n and writes the denominators.
 // Q, K and V enter as the projection left them, their factors as fp32 on accumulators or, w, on V^T in two terms.
-#include "state_chunk.cuh"
+#include "chunk_walk.cuh"
 
 namespace mv {
 
@@ -33,7 +34,7 @@ template <int K> struct MemVec {
   static constexpr int64_t kA = 2 * kChunk * kChunk * 2, kBytes = kA + kCount * 4;
 };
 
-template <int K>
+template <int K, bool kWalk>
 __global__ void __launch_bounds__(kMpThreads) mlstm_prepare_kernel(const MemChunkParams p) {
   using Vc = MemVec<K>;
   constexpr int ROW = K + 8;
@@ -99,7 +100,10 @@ __global__ void __launch_bounds__(kMpThreads) mlstm_prepare_kernel(const MemChun
   cp_async_wait<0>();
   __syncthreads();
   const LaneAt at(lane);
-  uint32_t* gA = reinterpret_cast<uint32_t*>(dst);
+  auto local = [&](int x, int r, int c) -> uint32_t& {     // columns c and c + 1 of A's term x
+    return *reinterpret_cast<uint32_t*>(dst + (kWalk ? x * kSlab + tile_at(r, c) : ((x * kChunk + r) * kChunk + c) * 2));
+  };
+  if (kWalk) zero_upper(tid, kMpThreads, [&](int r, int c, int x) -> uint32_t& { return local(x, r, c); });
   const int g = lane >> 2, c2 = (lane & 3) * 2;
   // blocks 0 .. 5 below the diagonal, (1,0) (2,0) (2,1) (3,0) (3,1) (3,2), then the four on it
 #pragma unroll 1
@@ -130,8 +134,8 @@ __global__ void __launch_bounds__(kMpThreads) mlstm_prepare_kernel(const MemChun
         sum += x + y;
         uint32_t hi, lo;
         split2(x, y, hi, lo);
-        gA[(t * kChunk + j) / 2] = hi;
-        gA[kChunk * kChunk / 2 + (t * kChunk + j) / 2] = lo;
+        local(0, t, j) = hi;
+        local(1, t, j) = lo;
       }
       sum += __shfl_xor_sync(0xffffffffu, sum, 1);
       sum += __shfl_xor_sync(0xffffffffu, sum, 2);
@@ -324,31 +328,50 @@ static int64_t mlstm_scratch_bytes(int K) {
 extern "C" int64_t mv_mlstm_chunk_workspace_bytes(int64_t tokens, int num_seqs, int heads, int dim, int vdim) {
   using namespace mv;
   if (tokens < 0 || num_seqs < 0 || heads <= 0 || !chunk_takes(dim, vdim)) return -1;
-  return chunk_bound(tokens, num_seqs) * heads * mlstm_scratch_bytes(dim);
+  const int64_t chunks = chunk_bound(tokens, num_seqs) * heads;
+  if (!walk_takes(dim, vdim)) return chunks * mlstm_scratch_bytes(dim);
+  return chunks * (dim <= 64 ? WalkBlob<64, true>::kBytes : WalkBlob<128, true>::kBytes) +
+         walk_segment_floats(tokens, num_seqs, heads, dim, vdim) * 4;
 }
 
 extern "C" int mv_mlstm_chunk_scan(void* out, int64_t out_stride, float* den, const void* q, const void* k, const void* v,
                                    int64_t stride, const float* chain, const int32_t* cu, int num_seqs, int64_t tokens,
                                    const int32_t* slots, const int32_t* start, float* S, float* n, int num_slots, int heads,
-                                   int dim, int vdim, float q_scale, void* workspace, int64_t workspace_bytes, void* stream) {
+                                   int dim, int vdim, float q_scale, void* workspace, int64_t workspace_bytes, int* error_word, void* stream) {
   using namespace mv;
   if (num_seqs < 0 || tokens < 0 || heads <= 0 || heads > 65535 || !chunk_takes(dim, vdim))
     return fail(MV_ERR_SHAPE, "mlstm_chunk_scan: heads %d, dim %d, vdim %d", heads, dim, vdim);
   if (num_seqs == 0 || tokens == 0) return MV_OK;
-  if (!out || !den || !q || !k || !v || !chain || !cu || !slots || !start || !S || !n) return fail(MV_ERR_NULL, "mlstm_chunk_scan: null pointer");
+  if (!out || !den || !q || !k || !v || !chain || !cu || !slots || !start || !S || !n || !error_word) return fail(MV_ERR_NULL, "mlstm_chunk_scan: null pointer");
   if (!vec8_ok(out, out_stride, 2) || !vec8_ok(q, stride, 2) || !vec8_ok(k, stride, 2) || !vec8_ok(v, stride, 2) || !aligned16(chain))
     return fail(MV_ERR_ALIGN, "mlstm_chunk_scan: rows must start on 16-byte boundaries");
   const int64_t chunks = chunk_bound(tokens, num_seqs);
-  if (!workspace || !aligned16(workspace) || workspace_bytes < chunks * heads * mlstm_scratch_bytes(dim))
+  if (!workspace || !aligned16(workspace) || workspace_bytes < mv_mlstm_chunk_workspace_bytes(tokens, num_seqs, heads, dim, vdim))
     return fail(MV_ERR_WORKSPACE, "mlstm_chunk_scan: workspace");
   auto c = [](const void* x) { return static_cast<const __nv_bfloat16*>(x); };
   const MemChunkParams p{static_cast<__nv_bfloat16*>(out), out_stride, den, c(q), c(k), c(v), stride, reinterpret_cast<const float4*>(chain),
                          q_scale, cu, slots, start, num_seqs, S, n, num_slots, heads, dim, vdim, static_cast<unsigned char*>(workspace)};
   auto st = static_cast<cudaStream_t>(stream);
+  if (walk_takes(dim, vdim)) {
+    auto walk = [&](auto kk) {
+      constexpr int K = decltype(kk)::value;
+      using Vc = MemVec<K>;
+      using Wb = WalkBlob<K, true>;
+      static_assert(Vc::kBytes == Wb::kBytes && Vc::kA == Wb::kVec && Vc::kWrite == Wb::kWrite && Vc::kFloor == Wb::kFloor && Vc::kDecay == Wb::kDecay,
+                    "both walks read the same scratch");
+      mlstm_prepare_kernel<K, true><<<dim3(static_cast<unsigned>(chunks), heads), kMpThreads, 2 * kChunk * (K + 8) * 2, st>>>(p);
+      const int rc = check_launch("mlstm_prepare");
+      if (rc) return rc;
+      const WalkParams w{p.out, p.out_stride, p.den, p.q, p.k, p.v, p.stride, p.cu, p.slots, p.start, num_seqs, p.state, p.n_state,
+                         p.num_slots, heads, dim, vdim, p.scratch, 0, nullptr, nullptr, nullptr, error_word};
+      return run_walk<K, true>("mlstm_chunk", w, tokens, reinterpret_cast<float*>(p.scratch + chunks * heads * Wb::kBytes), st);
+    };
+    return dim <= 64 ? walk(std::integral_constant<int, 64>{}) : walk(std::integral_constant<int, 128>{});
+  }
   return chunk_dispatch(dim, [&](auto kk) {
     constexpr int K = decltype(kk)::value;
     constexpr int prep = 2 * kChunk * (K + 8) * 2;
-    mlstm_prepare_kernel<K><<<dim3(static_cast<unsigned>(chunks), heads), kMpThreads, prep, st>>>(p);
+    mlstm_prepare_kernel<K, false><<<dim3(static_cast<unsigned>(chunks), heads), kMpThreads, prep, st>>>(p);
     int rc = check_launch("mlstm_prepare");
     if (rc) return rc;
     const int pb = chunk_columns(static_cast<int64_t>(num_seqs) * heads, vdim), smem = 2 * MemChunkShape<K>::stage(pb);

@@ -140,6 +140,16 @@ __device__ __forceinline__ void load_lower(uint32_t dst, const __nv_bfloat16* sr
   }
 }
 
+// Zeros in the 16 x 16 blocks above the diagonal of a 64 x 64 tile in two terms; at(row, column, term) is the word of two columns.
+template <typename F> __device__ __forceinline__ void zero_upper(int tid, int threads, F&& at) {
+  constexpr int kWords = 6 * 16 * 8;             // of a term: six blocks, 16 rows, 8 words
+  for (int i = tid; i < 2 * kWords; i += threads) {
+    const int x = i / kWords, blk = i % kWords / 128, r = i % 128 / 8, c = i % 8 * 2;
+    const int bj = blk == 0 ? 1 : blk < 3 ? 2 : 3, bi = blk - bj * (bj - 1) / 2;
+    at(bi * 16 + r, bj * 16 + c, x) = 0u;
+  }
+}
+
 // The warp's 16 x 64 transposed results to rows of `tile` (its own 16 columns), then to `dst` in 32-byte pieces.
 __device__ __forceinline__ void store_out(const float (&o)[8][4], __nv_bfloat16* tile, int stride, __nv_bfloat16* dst,
                                           int64_t dst_stride, int nt, int cols, int lane) {

@@ -7,6 +7,7 @@ import torch.nn.functional as F
 
 from .. import _cabi
 from ..utils.context import get_context
+from .attention import _error_word
 from .group_norm import head_norm_gate
 from .linear import StackedLinear
 
@@ -33,7 +34,8 @@ def gla_scan(q, k, v, z, tau, cu, slots, starts, state, heads, dim, vdim, gate=N
         _cabi.check(L.mv_gla_chunk_scan(
             out.data_ptr(), out.stride(0), q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), z.data_ptr(), z.stride(0),
             tau, cu.data_ptr(), slots.numel(), tokens, slots.data_ptr(), starts.data_ptr(), state.data_ptr(), state.shape[0],
-            heads, dim, vdim, dim ** -0.5, ws.data_ptr(), ws.numel(), _cabi.stream_ptr()))
+            heads, dim, vdim, dim ** -0.5, ws.data_ptr(), ws.numel(), _error_word(q.device).data_ptr(),
+            _cabi.stream_ptr()))
         return out
     _cabi.check(L.mv_gla_scan(
         out.data_ptr(), out.stride(0), q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), z.data_ptr(), z.stride(0),

@@ -8,6 +8,7 @@ import torch.nn.functional as F
 
 from .. import _cabi
 from ..utils.context import get_context
+from .attention import _error_word
 from .gla import CHUNK_FROM
 from .group_norm import head_norm_gate
 from .linear import StackedLinear, router_logits
@@ -43,7 +44,8 @@ def mlstm_scan(q, k, v, chain, cu, slots, starts, S, n, heads, dim, vdim, chunke
     state = (slots.data_ptr(), starts.data_ptr(), S.data_ptr(), n.data_ptr(), S.shape[0], heads, dim, vdim, dim ** -0.5)
     if chunked:
         ws = torch.empty(max(need, 1), dtype=torch.uint8, device=q.device)
-        _cabi.check(L.mv_mlstm_chunk_scan(*head, tokens, *state, ws.data_ptr(), ws.numel(), _cabi.stream_ptr()))
+        _cabi.check(L.mv_mlstm_chunk_scan(*head, tokens, *state, ws.data_ptr(), ws.numel(), _error_word(q.device).data_ptr(),
+                                    _cabi.stream_ptr()))
     else:
         _cabi.check(L.mv_mlstm_scan(*head, *state, _cabi.layer_dtype_code(q.dtype), _cabi.stream_ptr()))
     return out, den

@@ -8,6 +8,7 @@ import torch.nn.functional as F
 
 from .. import _cabi
 from ..utils.context import get_context
+from .attention import _error_word
 from .gla import CHUNK_FROM, DEFAULT_RANK
 from .group_norm import head_norm_gate
 from .linear import router_logits
@@ -41,7 +42,8 @@ def time_scan(r, k, v, z, w0, bonus, cu, slots, starts, state, heads, dim, vdim,
     tail = (slots.data_ptr(), starts.data_ptr(), state.data_ptr(), state.shape[0], heads, dim, vdim)
     if chunked:
         ws = torch.empty(max(need, 1), dtype=torch.uint8, device=r.device)
-        _cabi.check(L.mv_time_chunk_scan(*head, tokens, *tail, ws.data_ptr(), ws.numel(), _cabi.stream_ptr()))
+        _cabi.check(L.mv_time_chunk_scan(*head, tokens, *tail, ws.data_ptr(), ws.numel(), _error_word(r.device).data_ptr(),
+                                    _cabi.stream_ptr()))
         return out
     ptr = lambda t: t.data_ptr() if t is not None else None
     _cabi.check(L.mv_time_scan(*head, *tail, ptr(gate), gate.stride(0) if gate is not None else 0, ptr(norm_w), eps, out_scale,

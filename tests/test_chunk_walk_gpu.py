@@ -1,0 +1,76 @@
+"""The tensor-memory walk over chunks (csrc/chunk_walk.cuh) where sequences are cut into segments: few long sequences, ragged
+ends of segments and chunks, empty sequences, states that go on, narrow last column blocks."""
+import pytest
+import torch
+
+from oracle import dafotar_oracle, fozerax_oracle, subivik_oracle
+
+pytestmark = pytest.mark.gpu
+BF, F64 = torch.bfloat16, torch.float64
+
+
+def _rnd(seed, *shape, scale=1.0, mean=0.0):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale + mean
+
+
+def _i32(x):
+    return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+
+def _rel(got, want):
+    got, want = got.double().cpu(), want.double()
+    return float((got - want).norm() / want.norm())
+
+
+# heads, dim, vdim, lengths of the first and the second portion of each sequence
+CASES = [(1, 128, 256, [700], [513]), (2, 64, 128, [1025, 0, 300], [1, 640, 0]), (1, 96, 136, [64 * 9], [64 * 5 + 1]),
+         (3, 40, 72, [899, 257], [63, 64]), (1, 128, 128, [3001], [17])]
+
+
+@pytest.mark.parametrize("kind", ["gla", "time", "mlstm"])
+@pytest.mark.parametrize("H,K,V,first,second", CASES, ids=str)
+def test_segments(kind, H, K, V, first, second):
+    """Read-outs within the rounding of bf16 results and operands, states within that of operands in two terms, as for whole
+    sequences (tests of the chunked kernels)."""
+    from minivllm_b200.layers import gla, mlstm, time_mix
+    n, lens = len(first), [a + b for a, b in zip(first, second)]
+    q, k, v = ([_rnd(10 * s + i, lens[s], H, D).to(BF) for s in range(n)] for i, D in enumerate((K, K, V)))
+    S = torch.full((n, H, K, V), float("nan"), device="cuda")
+    d = lambda t: t.double()
+    if kind == "gla":
+        z = [_rnd(10 * s + 5, lens[s], H, K, mean=3.0).to(BF) for s in range(n)]
+        ref = [fozerax_oracle.gla_scan(d(a) * K ** -0.5, d(b), d(c), fozerax_oracle.channel_decay(d(x), 4.0)) for a, b, c, x in zip(q, k, v, z)]
+    elif kind == "time":
+        z, w0, bonus = [_rnd(10 * s + 5, lens[s], H, K, mean=-3.0) for s in range(n)], _rnd(3, H * K).to(BF), _rnd(4, H, K).to(BF)
+        ref = [subivik_oracle.bonus_scan(d(a), d(b), d(c), torch.exp(-torch.exp(d(x) + d(w0).view(H, K))), d(bonus)) for a, b, c, x in zip(q, k, v, z)]
+    else:
+        z, zero = [_rnd(10 * s + 5, lens[s], 2 * H, mean=0.0) for s in range(n)], torch.zeros(H)
+        f_b = torch.full((H,), 3.0)
+        cap = lambda x: 9.0 * torch.tanh(x / 9.0)
+        ref = [dafotar_oracle.mlstm_scan(d(a) * K ** -0.5, d(b), d(c), cap(d(x[:, :H])), torch.nn.functional.logsigmoid(cap(d(x[:, H:]) + 3.0)))
+               for a, b, c, x in zip(q, k, v, z)]
+        nv, m = torch.full((n, H, K), float("nan"), device="cuda"), torch.full((n, H), float("nan"), device="cuda")
+    slots, at = _i32(list(range(n))), [0] * n
+    for part in (first, second):
+        cut = lambda x: torch.cat([x[s][at[s]:at[s] + part[s]].flatten(1) for s in range(n)]).cuda()
+        p = torch.cat([cut(q), cut(k), cut(v)], 1)
+        a, b, c = p.split([H * K, H * K, H * V], 1)
+        cu, starts = _i32([0] + torch.tensor(part).cumsum(0).tolist()), _i32(at)
+        if kind == "gla":
+            got = gla.gla_scan(a, b, c, cut(z), 4.0, cu, slots, starts, S, H, K, V, chunked=True).view(-1, H, V)
+        elif kind == "time":
+            got = time_mix.time_scan(a, b, c, cut(z), w0.cuda(), bonus.cuda(), cu, slots, starts, S, H, K, V, chunked=True).view(-1, H, V)
+        else:
+            chain = mlstm.mlstm_gates(cut(z), zero.to(BF).cuda(), f_b.to(BF).cuda(), 9.0, cu, slots, starts, m, H)
+            o, den = mlstm.mlstm_scan(a, b, c, chain, cu, slots, starts, S, nv, H, K, V, chunked=True)
+            got = o.view(-1, H, V).double() / den.double()[..., None]
+        want = torch.cat([ref[s][0][at[s]:at[s] + part[s]] for s in range(n)])
+        assert _rel(got, want) < 6e-3, part
+        at = [x + y for x, y in zip(at, part)]
+    for s in range(n):
+        if kind == "mlstm":
+            want = ref[s][1]
+            shift = torch.exp(m[s].cpu().double() - want[2])
+            assert _rel(S[s].cpu().double() * shift[:, None, None], want[0]) < 1e-4 and _rel(nv[s].cpu().double() * shift[:, None], want[1]) < 1e-4
+        else:
+            assert _rel(S[s], ref[s][1]) < 2e-4, s
