@@ -11,7 +11,6 @@ constexpr int kDecWarps = 4;
 constexpr int kDecThreads = kDecWarps * 32;
 constexpr int kDecStages = 3;
 constexpr int kTileTok = 16;                    // tokens per warp tile
-constexpr int kCtaTok = kTileTok * kDecWarps;   // tokens per CTA step
 constexpr int kDecCtasPerSM = 2;
 constexpr int kDecWaves = 1;                    // work units per resident CTA: units are equal in length, so one each
                                                 // is balanced; 2 and 4 measured slower (more pieces to merge)
@@ -73,11 +72,13 @@ __device__ __forceinline__ int load_ctx(const DecodeParams& p, int b) {
 struct DecodePlan {
   int seg_len, n_seg;
 };
+template <int kWarps = kDecWarps>
 __device__ inline DecodePlan build_plan(const DecodeParams& p, int* s_tok, long long* s_red) {
+  constexpr int kStep = kTileTok * kWarps;               // tokens per CTA step
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int carry = 0;
   if (tid == 0) s_tok[0] = 0;
-  for (int base = 0; base < p.batch; base += kDecThreads) {
+  for (int base = 0; base < p.batch; base += kWarps * 32) {
     const int b = base + tid;
     const int n = b < p.batch ? load_ctx(p, b) : 0;
     int incl = n;
@@ -90,7 +91,7 @@ __device__ inline DecodePlan build_plan(const DecodeParams& p, int* s_tok, long 
     __syncthreads();
     int wofs = 0, tot = 0;
 #pragma unroll
-    for (int w = 0; w < kDecWarps; ++w) {
+    for (int w = 0; w < kWarps; ++w) {
       const int v = static_cast<int>(s_red[w]);
       if (w < warp) wofs += v;
       tot += v;
@@ -102,8 +103,8 @@ __device__ inline DecodePlan build_plan(const DecodeParams& p, int* s_tok, long 
   const int total = carry;
   DecodePlan plan;
   int seg = (total + p.target_items - 1) / p.target_items;
-  seg = ((seg + kCtaTok - 1) / kCtaTok) * kCtaTok;
-  if (seg < kCtaTok) seg = kCtaTok;
+  seg = ((seg + kStep - 1) / kStep) * kStep;
+  if (seg < kStep) seg = kStep;
   plan.seg_len = seg;
   plan.n_seg = (total + seg - 1) / seg;   // <= target_items
   return plan;
@@ -177,7 +178,7 @@ __device__ __forceinline__ void zero_empty_sequences(const DecodeParams& p, cons
   for (int b = blockIdx.x; b < p.batch; b += gridDim.x) {
     if (s_tok[b + 1] != s_tok[b]) continue;
     T* row = static_cast<T*>(p.out) + static_cast<int64_t>(b) * p.num_heads * D;
-    for (int i = threadIdx.x; i < p.num_heads * D; i += kDecThreads) row[i] = Elem<T>::from_f(0.f);
+    for (int i = threadIdx.x; i < p.num_heads * D; i += blockDim.x) row[i] = Elem<T>::from_f(0.f);
   }
 }
 
@@ -185,17 +186,17 @@ __device__ __forceinline__ void zero_empty_sequences(const DecodeParams& p, cons
 // floats) and its (m, l) pairs (sML) to shared memory: combine the warps and
 // write either the final output (sequence not split) or the partial result.
 // A warp's rows sit at (warp * rpw + row): rpw = 16 (the whole MMA tile) or fewer when only the first rows exist.
-template <typename T, int D>
+template <typename T, int D, int kWarps = kDecWarps>
 __device__ __forceinline__ void merge_and_write(const DecodeParams& p, const float* sO, const float* sML, int stride,
                                                 int rows_valid, int h0, int b, int item, int nsplit, int rpw = 16) {
-  for (int idx = threadIdx.x; idx < rows_valid * D; idx += kDecThreads) {
+  for (int idx = threadIdx.x; idx < rows_valid * D; idx += kWarps * 32) {
     const int row = idx / D, d = idx - row * D;
     float M = kNegBig;
 #pragma unroll
-    for (int ww = 0; ww < kDecWarps; ++ww) M = fmaxf(M, sML[(ww * rpw + row) * 2]);
+    for (int ww = 0; ww < kWarps; ++ww) M = fmaxf(M, sML[(ww * rpw + row) * 2]);
     float acc = 0.f, L = 0.f;
 #pragma unroll
-    for (int ww = 0; ww < kDecWarps; ++ww) {
+    for (int ww = 0; ww < kWarps; ++ww) {
       const float wgt = fast_exp2(sML[(ww * rpw + row) * 2] - M);
       acc += wgt * sO[(ww * rpw + row) * stride + d];
       L += wgt * sML[(ww * rpw + row) * 2 + 1];
@@ -233,7 +234,7 @@ __device__ __forceinline__ void combine_if_last(const DecodeParams& p, const int
   __syncthreads();
   if (*s_last) {
     const int2 info = seq_items(s_tok, plan, b);
-    for (int idx = threadIdx.x; idx < rows_valid * D; idx += kDecThreads) {
+    for (int idx = threadIdx.x; idx < rows_valid * D; idx += blockDim.x) {
       const int h = h0 + idx / D, d = idx % D;
       float M = kNegBig;
       for (int s = 0; s < info.y; ++s)

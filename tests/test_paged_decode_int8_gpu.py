@@ -62,6 +62,8 @@ def test_int8_decode_config_shape(dtype):
     dict(batch=3, ctx_lo=10, ctx_hi=500, num_heads=32, num_kv_heads=1, block_size=48),   # two row tiles; odd scale indices
     dict(batch=40, ctx_lo=1, ctx_hi=700, num_heads=4, num_kv_heads=1, block_size=256),
     dict(batch=4, ctx_lo=200, ctx_hi=900, num_heads=9, num_kv_heads=3, block_size=32),   # odd kv head count
+    dict(batch=7, ctx_lo=1, ctx_hi=900, num_heads=16, num_kv_heads=2, block_size=64),    # eight heads a group: the last on the N side
+    dict(batch=7, ctx_lo=1, ctx_hi=900, num_heads=18, num_kv_heads=2, block_size=64),    # nine: heads on the M side
 ])
 def test_int8_decode_shape_sweep(kw):
     _check(synth.decode_inputs(seed=50, head_dim=128, **kw), torch.float16)
