@@ -82,6 +82,12 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+__device__ __forceinline__ float max_nan(float a, float b) {       // NaN if either is
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
+
 // Blackwell packed fp32 pairs: one issue slot for two lanes of work.
 __device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
   float2 d;

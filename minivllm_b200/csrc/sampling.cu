@@ -204,9 +204,9 @@ __device__ __forceinline__ float race_noise(uint32_t bits) {
 // Bound: instruction issue (a column's share of Philox is 15 slots).  A score is only formed where it can win.  With E = -log u
 // >= 1 - u a score is at most v / T - log(1 - u), so a column whose 1 - u exceeds e^(v / T - best) is passed over for one
 // ex2.approx instead of two logarithms; `best` is the warp's, which moves about ten times in a row.  The test errs on the side
-// of forming the score: `slack` covers the roundings of the exponent (a few 2^-23 of best, and those of the noise itself),
+// of forming the score: aim()'s slack covers the roundings of the exponent (a few 2^-23 of best, and those of the noise itself),
 // kEdge those of u, and a NaN or an infinity fails the comparison.  Every score that is formed is the same as before, so are the
-// tokens.  512 x 151,936 bf16: 236 us when every score was formed, 132 us now.
+// tokens.  512 x 151,936 bf16: 236 us when every score was formed, 107 us now.
 template <typename T, bool kVec>
 __global__ void __launch_bounds__(kArgmaxThreads)
 sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t cols, uint32_t index_offset, bool aligned,
@@ -229,65 +229,97 @@ sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t col
   constexpr int kPiece = kVec && sizeof(T) == 2 ? 8 : 4;
   constexpr float kLog2 = 1.4426950408889634f, kEdge = 2.f - 0x1p-21f;
   const float slope = inv_t * kLog2;
-  float shift = INFINITY;                        // (slack - best) in base 2: everything may win at first
-  // Global columns base .. base + kPiece - 1 of piece p; the first piece may begin before the shard.
-  const uint32_t base0 = index_offset & ~3u;
-  const int64_t lead = static_cast<int64_t>(index_offset) - base0, pieces = (cols + lead + kPiece - 1) / kPiece;
-  const int64_t rounds = (pieces + my.threads - 1) / my.threads;
-  for (int64_t it = 0; it < rounds; ++it) {      // the same number for all lanes: they vote
-    const int64_t p = it * my.threads + my.at, i0 = p * kPiece - lead;
-    float v[kPiece];
-    bool live = false;                           // some column of the piece exists
-    if constexpr (kVec) {
-      live = p < pieces;
-      if (live) {
-        if (i0 + kPiece <= cols) {
-          const uint4 raw = ld_stream16(row + i0);
-          if constexpr (sizeof(T) == 2) {
-            const typename Elem<T>::T2* p2 = reinterpret_cast<const typename Elem<T>::T2*>(&raw);
+  float shift = INFINITY;                        // (slack - best) in base 2
+  // Piece p has the global columns base0 + p * kPiece and on; the first piece may begin before the shard, the last end behind it.
+  const uint32_t n_cols = static_cast<uint32_t>(cols), base0 = index_offset & ~3u, lead = index_offset - base0;
+  const uint32_t skip = lead ? 1u : 0u, whole = (n_cols + lead) / kPiece, pieces = whole + ((n_cols + lead) % kPiece ? 1u : 0u);
+  auto draw = [&](uint32_t p, uint32_t (&bits)[kPiece]) {
+    const uint32_t group = (base0 >> 2) + p * (kPiece / 4);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float2 f = Elem<T>::to_f2(p2[j]);
-              v[2 * j] = f.x;
-              v[2 * j + 1] = f.y;
-            }
-          } else {
-            const float4 f = *reinterpret_cast<const float4*>(&raw);
-            v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < kPiece; ++j) v[j] = i0 + j < cols ? Elem<T>::to_f(row[i0 + j]) : -INFINITY;
-        }
-      }
-    } else {
-      live = p < pieces;
-#pragma unroll
-      for (int j = 0; j < kPiece; ++j) v[j] = live && i0 + j >= 0 && i0 + j < cols ? Elem<T>::to_f(row[i0 + j]) : -INFINITY;
+    for (int q = 0; q < kPiece / 4; ++q) {
+      const Philox a = philox4x32_10(Philox{group + q, rowi, s0, s1}, k0, k1);
+      bits[4 * q] = a.x; bits[4 * q + 1] = a.y; bits[4 * q + 2] = a.z; bits[4 * q + 3] = a.w;
     }
-    uint32_t bits[kPiece], may = 0;
-    if (live) {
-      const uint32_t group = (base0 >> 2) + static_cast<uint32_t>(p * (kPiece / 4));
-#pragma unroll
-      for (int q = 0; q < kPiece / 4; ++q) {
-        const Philox a = philox4x32_10(Philox{group + q, rowi, s0, s1}, k0, k1);
-        bits[4 * q] = a.x; bits[4 * q + 1] = a.y; bits[4 * q + 2] = a.z; bits[4 * q + 3] = a.w;
-      }
-#pragma unroll
-      for (int j = 0; j < kPiece; ++j) {
-        const float e = fast_exp2(fmaf(v[j], slope, shift)), u1 = __uint_as_float((bits[j] >> 9) | 0x3f800000u);     // 1 + u
-        may |= u1 + e < kEdge ? 0u : 1u << j;
-      }
-    }
-    if (!__any_sync(0xffffffffu, may != 0)) continue;
-#pragma unroll
-    for (int j = 0; j < kPiece; ++j)
-      if ((may >> j & 1) && i0 + j >= 0 && i0 + j < cols) best.offer(v[j] * inv_t + race_noise(bits[j]), static_cast<uint32_t>(i0 + j));
-    float top = best.v;                          // a NaN leaves the others' maximum
+  };
+  auto aim = [&] {                               // the warp's best so far sets the test; a NaN leaves the others' maximum
+    float top = best.v;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
-    const float slack = 0.02f + 4e-6f * fabsf(top);
-    shift = (slack - top) * kLog2;
+    // behind an infinite score only infinities and NaN are looked at
+    shift = top == INFINITY ? -INFINITY : (0.02f + 4e-6f * fabsf(top) - top) * kLog2;
+  };
+  // The whole warp; lanes that are not `live` have nothing to offer, nor have columns outside the shard.
+  auto consider = [&](const float (&v)[kPiece], uint32_t p, bool live, bool inside) {
+    uint32_t bits[kPiece];
+    draw(p, bits);
+    float2 x[kPiece / 2];
+    float most = -INFINITY;
+#pragma unroll
+    for (int j = 0; j < kPiece / 2; ++j) {
+      x[j] = fma_f32x2(make_float2(v[2 * j], v[2 * j + 1]), make_float2(slope, slope), make_float2(shift, shift));
+      x[j] = add_f32x2(make_float2(fast_exp2(x[j].x), fast_exp2(x[j].y)),
+                       make_float2(__uint_as_float((bits[2 * j] >> 9) | 0x3f800000u), __uint_as_float((bits[2 * j + 1] >> 9) | 0x3f800000u)));
+      most = max_nan(max_nan(most, x[j].x), x[j].y);
+    }
+    if (!__any_sync(0xffffffffu, live && !(most < kEdge))) return;
+#pragma unroll
+    for (int j = 0; j < kPiece; ++j) {
+      const uint32_t i = p * kPiece + j - lead;  // wraps below zero: not below n_cols
+      if (live && !((j & 1 ? x[j / 2].y : x[j / 2].x) < kEdge) && (inside || i < n_cols)) best.offer(v[j] * inv_t + race_noise(bits[j]), i);
+    }
+    aim();
+  };
+  auto fetch = [&](uint32_t p, float (&v)[kPiece]) {       // a whole piece inside the shard
+    const T* at = row + (p * kPiece - lead);
+    if constexpr (kVec) {
+      const uint4 raw = ld_stream16(at);
+      if constexpr (sizeof(T) == 2) {
+        const typename Elem<T>::T2* p2 = reinterpret_cast<const typename Elem<T>::T2*>(&raw);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 f = Elem<T>::to_f2(p2[j]);
+          v[2 * j] = f.x;
+          v[2 * j + 1] = f.y;
+        }
+      } else {
+        const float4 f = *reinterpret_cast<const float4*>(&raw);
+        v[0] = f.x; v[1] = f.y; v[2] = f.z; v[3] = f.w;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < kPiece; ++j) v[j] = Elem<T>::to_f(at[j]);
+    }
+  };
+  const uint32_t rounds = whole > skip ? (whole - skip) / my.threads : 0;
+  uint32_t p = skip + my.at;
+  if (rounds) {
+    // one score per lane to begin with, so that the test has something to go by (the same column again is no gain over itself)
+    float v[kPiece];
+    uint32_t bits[kPiece];
+    fetch(p, v);
+    draw(p, bits);
+    best.offer(v[0] * inv_t + race_noise(bits[0]), p * kPiece - lead);
+    aim();
+    for (uint32_t it = 0; it < rounds; ++it, p += my.threads) {
+      float now[kPiece];
+#pragma unroll
+      for (int j = 0; j < kPiece; ++j) now[j] = v[j];
+      if (it + 1 < rounds) fetch(p + my.threads, v);
+      consider(now, p, true, true);
+    }
+  }
+  // what is left: less than a round of whole pieces, and the pieces over the shard's edges
+  const uint32_t left = pieces - rounds * my.threads;      // the first piece of a shard that begins inside it among them
+  for (uint32_t it = 0; it * my.threads < left; ++it) {
+    const uint32_t k = it * my.threads + my.at, q = k < skip ? 0 : k + rounds * my.threads;
+    const bool live = k < left;
+    float v[kPiece];
+#pragma unroll
+    for (int j = 0; j < kPiece; ++j) {
+      const uint32_t i = q * kPiece + j - lead;
+      v[j] = live && i < n_cols ? Elem<T>::to_f(row[i]) : -INFINITY;
+    }
+    consider(v, q, live, false);
   }
   finish_row(best, index_offset, my, rowi, keys, tokens);
 }
