@@ -7,21 +7,30 @@
 // scratch that lies there as the swizzled tiles want it, so a chunk is one bulk copy and its V.  mLSTM (kMem): Q and K are the
 // projection's rows; alpha is applied to O^T's first product, and w V is split into two terms here.
 //
-// 17 warps: 0-7 own the state (a thread has a value column and half of the channels: scales, splits and writes it back),
-// 8-11 read O and store rows, 12-15 load (and form w V, n and the denominators), 16 issues the products.  The chain of a chunk
-// is state -> update -> state; O's products run beside the next chunk's scaling and splitting.
+// 18 warps: 0-7 own the state (a thread has a value column and half of the channels: scales, splits and writes it back),
+// 8-11 read O and store rows (and carry n and the denominators), 12-15 form w V, 16 issues the products, 17 loads.  The chain of a chunk
+// is state -> update -> state; O's products run beside the next chunk's scaling and splitting.  Whole chunks
+// come by TMA; a sequence's ragged last chunk is copied by warps 12-15 with zeros past its end, and so are all chunks of rows
+// that are not made of whole slabs.
 //
-// Bound: that chain (about 1,500 cycles a chunk, 512 of them the update's products), so a sequence's chunks take their time one
-// after the other.  Where sequences, heads and column blocks are too few for the SMs, sequences are cut into segments: a pass
-// over each segment from a zero state (kState: no O), a join that turns the segments' own states into the states in front of
-// them, and the full pass over all segments at once.
+// The roles' loops are rolled: unrolled, five of them pushed one another out of the instruction cache (a fourth of the stalls),
+// and a chunk of mLSTM took 4.1 us instead of 3.6.
+// Bound: gla and time mixing read 98 KB a chunk, two column blocks of a head the same 82 KB of it, at about 6 TB/s over all SMs
+// (L2); mLSTM the chain of w V, state and update.  Before (register MMAs): 885 and 242 us for the two walks below.
+//   1 x 16,384 tokens, 8 heads of 128 x 256 (gla, 9 segments): 38 us own states, 11 us join, 74 to 84 us walk
+//   16 x 512-1536 tokens, 8 heads of 128 x 256 (mLSTM): 138 us
+//
+// A sequence's chunks take their time one after the other.  Where sequences, heads and column blocks are too few for the SMs,
+// sequences are cut into segments: a pass over each segment from a zero state (kState: no O), a join that turns the segments'
+// own states into the states in front of them, and the full pass over all segments at once.
 #pragma once
 #include "state_chunk.cuh"
 #include "tcgen05.cuh"
+#include "tmap.cuh"
 
 namespace mv {
 
-constexpr int kWalkThreads = 17 * 32, kWalkCols = 128;
+constexpr int kWalkThreads = 18 * 32, kWalkCols = 128;
 constexpr int kSlab = kChunk * 128;                       // bytes of 64 rows of 64 bf16 values
 constexpr int kWalkV = 2 * kSlab;
 
@@ -58,6 +67,7 @@ struct WalkParams {
   int seg_chunks;                                         // chunks of a segment, 0: sequences are whole
   float *seg_state, *seg_n, *seg_decay;                   // per segment and head: K x V, K (kMem), K
   int* error_word;
+  bool tma;                                               // whole chunks by TMA
 };
 
 // Segment x of the batch: its sequence and its place in it.  Whole warp; false past the last.
@@ -137,7 +147,9 @@ __device__ __forceinline__ void mma_ts_4(uint32_t d_tmem, uint32_t a_tmem, uint6
 enum WalkBar { WB_BLOB = 0, WB_FULL = 2, WB_EMPTY = 4, WB_SREADY = 6, WB_SDONE, WB_ODONE, WB_OFREE, WB_COUNT };
 
 template <int K, bool kMem, bool kState>
-__global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const WalkParams p) {
+__global__ void __launch_bounds__(kWalkThreads, 1)
+chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                  const __grid_constant__ CUtensorMap map_v) {
   using B = WalkBlob<K, kMem>;
   using St = WalkStage<K, kMem>;
   extern __shared__ unsigned char smem_raw[];
@@ -172,7 +184,7 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const WalkP
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(bar(WB_BLOB + i), 1);
       tc::mbar_init(bar(WB_FULL + i), 128);
-      tc::mbar_init(bar(WB_EMPTY + i), kMem && !kState ? 1 + 128 : 1);
+      tc::mbar_init(bar(WB_EMPTY + i), 1 + 128);
     }
     tc::mbar_init(bar(WB_SREADY), 256);
     tc::mbar_init(bar(WB_SDONE), 1);
@@ -193,56 +205,62 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const WalkP
   const uint32_t tS = tmem, tHL = tmem + 128, tO = tmem + 384;
   auto wait = [&](int b, int parity, int where) { tc::mbar_wait(bar(b), parity, &s_abort, p.error_word, where); };
   auto stage_at = [&](int i) { return (i & 1) * St::kBytes; };
+  auto whole = [&](int i) { return p.tma && n_tok - i * kChunk >= kChunk; };    // chunk i comes by TMA
 
   if (warp < 8) {
     // ---------------------------------------------------------------- the state
     const int row = (warp & 3) * 32 + lane, ch0 = (warp >> 2) * (K / 2);
     const bool on = row < pw;
     const uint32_t lanes = static_cast<uint32_t>(warp & 3) << 21;
-    float S[K / 2];
+    const uint32_t own = tS + lanes + ch0;
     {
-      const float* src = p.seg_chunks ? p.seg_state + seg_pair * p.K * p.V : p.state + pair * p.K * p.V;
+      const float* src = (p.seg_chunks ? p.seg_state + seg_pair * p.K * p.V : p.state + pair * p.K * p.V) + p0 + row;
       const bool has = !kState && on && (p.seg_chunks || (live && st0 > 0));
+#pragma unroll 1
+      for (int c = 0; c < K / 2; c += 16) {
+        uint32_t x[16];
 #pragma unroll
-      for (int c = 0; c < K / 2; ++c)
-        S[c] = has && ch0 + c < p.K ? src[static_cast<int64_t>(ch0 + c) * p.V + p0 + row] : 0.f;
+        for (int e = 0; e < 16; ++e)
+          x[e] = has && ch0 + c + e < p.K ? __float_as_uint(src[static_cast<int64_t>(ch0 + c + e) * p.V]) : 0u;
+        tc::tmem_st16(own + c, x);
+      }
+      tc::wait_st();
     }
-    auto read_state = [&] {
-#pragma unroll
-      for (int c = 0; c < K / 2; c += 32) tc::tmem_ld32(tS + lanes + ch0 + c, *reinterpret_cast<uint32_t(*)[32]>(S + c));
-      tc::wait_ld();
-    };
     for (int i = 0; i < chunks; ++i) {
       const unsigned char* st = smem + stage_at(i);
       if (i > 0) {
         wait(WB_SDONE, (i - 1) & 1, 1);
         tc::fence_after_sync();
-        read_state();
       }
       wait(WB_BLOB + (i & 1), (i >> 1) & 1, 2);
       const float* vec = reinterpret_cast<const float*>(st + B::kVec);
       const uint32_t hl = tHL + (i & 1) * 128 + lanes + ch0 / 2;
+#pragma unroll 1
+      for (int c = 0; c < K / 2; c += 32) {
+        uint32_t x[32];
+        tc::tmem_ld32(own + c, x);
+        tc::wait_ld();
 #pragma unroll
-      for (int c = 0; c < K / 2; c += 16) {
-        if (!kState) {
-          uint32_t hi[8], lo[8];
+        for (int half = 0; half < 32; half += 16) {
+          if (!kState) {
+            uint32_t hi[8], lo[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) split2(S[c + 2 * e], S[c + 2 * e + 1], hi[e], lo[e]);
-          tc::tmem_st8(hl + c / 2, hi);
-          tc::tmem_st8(hl + 64 + c / 2, lo);
-        }
-        if constexpr (kMem) {
-          const float d = vec[B::kDecay];
-#pragma unroll
-          for (int e = 0; e < 16; ++e) S[c + e] *= d;
-        } else {
+            for (int e = 0; e < 8; ++e) split2(__uint_as_float(x[half + 2 * e]), __uint_as_float(x[half + 2 * e + 1]), hi[e], lo[e]);
+            tc::tmem_st8(hl + (c + half) / 2, hi);
+            tc::tmem_st8(hl + 64 + (c + half) / 2, lo);
+          }
 #pragma unroll
           for (int e = 0; e < 16; e += 4) {
-            const float4 d = *reinterpret_cast<const float4*>(vec + ch0 + c + e);
-            S[c + e] *= d.x; S[c + e + 1] *= d.y; S[c + e + 2] *= d.z; S[c + e + 3] *= d.w;
+            float4 d;
+            if constexpr (kMem) d = make_float4(vec[B::kDecay], vec[B::kDecay], vec[B::kDecay], vec[B::kDecay]);
+            else d = *reinterpret_cast<const float4*>(vec + ch0 + c + half + e);
+            const float2 lo2 = mul_f32x2(make_float2(__uint_as_float(x[half + e]), __uint_as_float(x[half + e + 1])), make_float2(d.x, d.y));
+            const float2 hi2 = mul_f32x2(make_float2(__uint_as_float(x[half + e + 2]), __uint_as_float(x[half + e + 3])), make_float2(d.z, d.w));
+            x[half + e] = __float_as_uint(lo2.x); x[half + e + 1] = __float_as_uint(lo2.y);
+            x[half + e + 2] = __float_as_uint(hi2.x); x[half + e + 3] = __float_as_uint(hi2.y);
           }
         }
-        tc::tmem_st16(tS + lanes + ch0 + c, *reinterpret_cast<const uint32_t(*)[16]>(S + c));
+        tc::tmem_st32(own + c, x);
       }
       tc::wait_st();
       tc::fence_before_sync();
@@ -250,103 +268,139 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const WalkP
     }
     wait(WB_SDONE, (chunks - 1) & 1, 3);
     tc::fence_after_sync();
-    read_state();
-    if (on && (kState || (last_seg && live))) {
-      float* dst = kState ? p.seg_state + seg_pair * p.K * p.V : p.state + pair * p.K * p.V;
+    const bool keep = on && (kState || (last_seg && live));
+    float* dst = (kState ? p.seg_state + seg_pair * p.K * p.V : p.state + pair * p.K * p.V) + p0 + row;
+#pragma unroll 1
+    for (int c = 0; c < K / 2; c += 16) {
+      uint32_t x[16];
+      tc::tmem_ld16(own + c, x);
+      tc::wait_ld();
+      if (keep) {
 #pragma unroll
-      for (int c = 0; c < K / 2; ++c)
-        if (ch0 + c < p.K) dst[static_cast<int64_t>(ch0 + c) * p.V + p0 + row] = S[c];
+        for (int e = 0; e < 16; ++e)
+          if (ch0 + c + e < p.K) dst[static_cast<int64_t>(ch0 + c + e) * p.V] = __uint_as_float(x[e]);
+      }
     }
   } else if (warp < 12) {
     // ---------------------------------------------------------------- results
-    if constexpr (!kState) {
-      const int t4 = tid - 256, row = (warp & 3) * 32 + lane;
-      const uint32_t lanes = static_cast<uint32_t>(warp & 3) << 21;
-      __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(smem + 2 * St::kBytes);
-      for (int i = 0; i < chunks; ++i) {
-        wait(WB_ODONE, i & 1, 4);
-        tc::fence_after_sync();
-        const float* vec = reinterpret_cast<const float*>(smem + stage_at(i) + B::kVec);
-        uint32_t o[64];
-#pragma unroll
-        for (int c = 0; c < 64; c += 32) tc::tmem_ld32(tO + lanes + c, *reinterpret_cast<uint32_t(*)[32]>(o + c));
-        tc::wait_ld();
-        if constexpr (kMem) {
-#pragma unroll
-          for (int c = 0; c < 64; c += 16) {
-            uint32_t a[16];
-            tc::tmem_ld16(tO + 64 + lanes + c, a);
-            tc::wait_ld();
-#pragma unroll
-            for (int e = 0; e < 16; e += 4) {
-              const float4 al = *reinterpret_cast<const float4*>(vec + B::kAlpha + c + e);
-              o[c + e] = __float_as_uint(fmaf(__uint_as_float(o[c + e]), al.x, __uint_as_float(a[e])));
-              o[c + e + 1] = __float_as_uint(fmaf(__uint_as_float(o[c + e + 1]), al.y, __uint_as_float(a[e + 1])));
-              o[c + e + 2] = __float_as_uint(fmaf(__uint_as_float(o[c + e + 2]), al.z, __uint_as_float(a[e + 2])));
-              o[c + e + 3] = __float_as_uint(fmaf(__uint_as_float(o[c + e + 3]), al.w, __uint_as_float(a[e + 3])));
-            }
-          }
-          tc::mbar_arrive(bar(WB_EMPTY + (i & 1)));        // the stage's alpha is read
-        }
-        tc::fence_before_sync();
-        tc::mbar_arrive(bar(WB_OFREE));
-        asm volatile("bar.sync 1, 128;" ::: "memory");     // the rows of the chunk before are stored
-#pragma unroll
-        for (int t = 0; t < kChunk; ++t) rows[t * kWalkCols + row] = __float2bfloat16_rn(__uint_as_float(o[t]));
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        const int nt = min(kChunk, n_tok - i * kChunk);
-        __nv_bfloat16* dst = p.out + (static_cast<int64_t>(first) + i * kChunk) * p.out_stride + static_cast<int64_t>(h) * p.V + p0;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int r = j * 8 + (t4 >> 4), c = (t4 & 15) * 8;
-          if (r < nt && c < pw)
-            *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(r) * p.out_stride + c) = *reinterpret_cast<const uint4*>(rows + r * kWalkCols + c);
-        }
-      }
-    }
-  } else if (warp < 16) {
-    // ---------------------------------------------------------------- loads
-    const int t = tid - 384, lw = warp - 12;
+    const int t = tid - 256, lw = warp - 8, row = lw * 32 + lane;
+    const uint32_t lanes = static_cast<uint32_t>(lw) << 21;
     const bool first_block = blockIdx.z == 0, keeps_n = kMem && first_block;
-    const __nv_bfloat16* v = p.v + static_cast<int64_t>(h) * p.V + p0;
-    float n[K / 32], prod = 1.f;                           // channels lane * (K / 32) ..; the segment's decay of channel t
+    constexpr int kPer = K / 32;
+    float n[kPer], prod = 1.f;                             // channels lane * kPer ..; the segment's decay of channel t
     if constexpr (kMem) {
       const float* src = p.seg_chunks ? p.seg_n + seg_pair * p.K : p.n_state + pair * p.K;
 #pragma unroll
-      for (int e = 0; e < K / 32; ++e) {
-        const int ch = lane * (K / 32) + e;
+      for (int e = 0; e < kPer; ++e) {
+        const int ch = lane * kPer + e;
         n[e] = !kState && keeps_n && ch < p.K && (p.seg_chunks || (live && st0 > 0)) ? src[ch] : 0.f;
       }
     }
-    auto issue = [&](int i) {
+    __nv_bfloat16* rows = reinterpret_cast<__nv_bfloat16*>(smem + 2 * St::kBytes);
+    for (int i = 0; i < chunks; ++i) {
+      unsigned char* st = smem + stage_at(i);
+      const float* vec = reinterpret_cast<const float*>(st + B::kVec);
+      const int nt = min(kChunk, n_tok - i * kChunk);
+      if (kState) {
+        wait(WB_BLOB + (i & 1), (i >> 1) & 1, 7);
+        if (first_block && t < K) prod *= kMem ? vec[B::kDecay] : vec[t];
+      }
+      if constexpr (kMem) {
+        if (keeps_n) {
+          if constexpr (!kState) {
+            wait(WB_FULL + (i & 1), (i >> 1) & 1, 6);
+#pragma unroll 2
+            for (int r = 0; r < 16; r += 2) {              // two tokens at a time, each half of the warp ends with one
+              float d[2];
+#pragma unroll
+              for (int x = 0; x < 2; ++x) {
+                const unsigned char* qr = st + St::kQ + tile_at(lw * 16 + r + x, lane * kPer);
+                d[x] = 0.f;
+#pragma unroll
+                for (int e = 0; e < kPer; e += 2) {
+                  const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(qr + e * 2));
+                  d[x] = fmaf(n[e + 1], f.y, fmaf(n[e], f.x, d[x]));
+                }
+              }
+              float dot = (lane & 16 ? d[1] : d[0]) + __shfl_xor_sync(0xffffffffu, lane & 16 ? d[0] : d[1], 16);
+#pragma unroll
+              for (int o = 8; o >= 1; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+              const int tok = lw * 16 + r + (lane >> 4);
+              if (!(lane & 15) && tok < nt)
+                p.den[(static_cast<int64_t>(first) + i * kChunk + tok) * p.heads + h] =
+                    fmaxf(fabsf(fmaf(vec[B::kAlpha + tok], dot, vec[B::kRow + tok])), vec[B::kFloor + tok]) + kMemFloor;
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < kPer; ++e) n[e] = fmaf(vec[B::kDecay], n[e], vec[B::kSum + lane * kPer + e]);
+        }
+      }
+      if constexpr (kState) {
+        tc::mbar_arrive(bar(WB_EMPTY + (i & 1)));
+        continue;
+      }
+      wait(WB_ODONE, i & 1, 4);
+      tc::fence_after_sync();
+      asm volatile("bar.sync 1, 128;" ::: "memory");       // the rows of the chunk before are stored
+#pragma unroll 1
+      for (int c = 0; c < kChunk; c += 16) {
+        uint32_t o[16];
+        tc::tmem_ld16(tO + lanes + c, o);
+        if constexpr (kMem) {
+          uint32_t a[16];
+          tc::tmem_ld16(tO + 64 + lanes + c, a);
+          tc::wait_ld();
+#pragma unroll
+          for (int e = 0; e < 16; e += 2) {
+            const float2 x = fma_f32x2(make_float2(__uint_as_float(o[e]), __uint_as_float(o[e + 1])), *reinterpret_cast<const float2*>(vec + B::kAlpha + c + e),
+                                       make_float2(__uint_as_float(a[e]), __uint_as_float(a[e + 1])));
+            o[e] = __float_as_uint(x.x);
+            o[e + 1] = __float_as_uint(x.y);
+          }
+        } else {
+          tc::wait_ld();
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) rows[(c + e) * kWalkCols + row] = __float2bfloat16_rn(__uint_as_float(o[e]));
+      }
+      tc::fence_before_sync();
+      tc::mbar_arrive(bar(WB_EMPTY + (i & 1)));            // the stage's vectors and Q are read
+      tc::mbar_arrive(bar(WB_OFREE));
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      __nv_bfloat16* dst = p.out + (static_cast<int64_t>(first) + i * kChunk) * p.out_stride + static_cast<int64_t>(h) * p.V + p0;
+#pragma unroll 2
+      for (int j = 0; j < 8; ++j) {
+        const int r = j * 8 + (t >> 4), c = (t & 15) * 8;
+        if (r < nt && c < pw)
+          *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(r) * p.out_stride + c) = *reinterpret_cast<const uint4*>(rows + r * kWalkCols + c);
+      }
+    }
+    if (kState && first_block && t < p.K) p.seg_decay[seg_pair * p.K + t] = prod;
+    if constexpr (kMem) {
+      if (keeps_n && lw == 0 && (kState || (last_seg && live))) {
+        float* dst = kState ? p.seg_n + seg_pair * p.K : p.n_state + pair * p.K;
+#pragma unroll
+        for (int e = 0; e < kPer; ++e)
+          if (lane * kPer + e < p.K) dst[lane * kPer + e] = n[e];
+      }
+    }
+  } else if (warp < 16) {
+    // ---------------------------------------------------------------- w V, ragged chunks
+    const int t = tid - 384;
+    const __nv_bfloat16* v = p.v + static_cast<int64_t>(h) * p.V + p0;
+    auto copy = [&](int i) {
       const int s2 = i & 1, nt = min(kChunk, n_tok - i * kChunk);
       const uint32_t st = base + stage_at(i);
       if (i >= 2) wait(WB_EMPTY + s2, ((i >> 1) - 1) & 1, 5);
-      if ((kMem || kState) && i >= 2) asm volatile("bar.sync 2, 128;" ::: "memory");       // no loader reads the stage any more
-      if (t == 0) {
-        const unsigned char* src = p.scratch + (static_cast<int64_t>(chunk0 + i) * p.heads + h) * B::kBytes;
-        const uint32_t b = bar(WB_BLOB + s2);
-        if (kState && !kMem) {
-          tc::mbar_expect_tx(b, 2 * B::kT + B::kFloats * 4);
-          tc::bulk_load(st + B::kK, src + B::kK, 2 * B::kT, b);
-          tc::bulk_load(st + B::kVec, src + B::kVec, B::kFloats * 4, b);
-        } else if (kState) {
-          tc::mbar_expect_tx(b, B::kFloats * 4);
-          tc::bulk_load(st + B::kVec, src + B::kVec, B::kFloats * 4, b);
-        } else {
-          tc::mbar_expect_tx(b, static_cast<uint32_t>(B::kBytes));
-          tc::bulk_load(st, src, static_cast<uint32_t>(B::kBytes), b);
-        }
-      }
       const int64_t row0 = static_cast<int64_t>(first) + i * kChunk;
-#pragma unroll
+#pragma unroll 2
       for (int j = 0; j < 8; ++j) {
         const int r = j * 8 + (t >> 4), c = (t & 15) * 8;
         const bool ok = r < nt && c < pw;
         cp_async16(st + St::kV + tile_at(r, c), ok ? v + (row0 + r) * p.stride + c : p.v, ok ? 16 : 0);
       }
       if constexpr (kMem) {
-#pragma unroll 4
+#pragma unroll 2
         for (int j = t; j < kChunk * (K / 8); j += 128) {
           const int r = j / (K / 8), c = (j % (K / 8)) * 8;
           const bool ok = r < nt && c < p.K;
@@ -356,18 +410,18 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const WalkP
         }
       }
     };
-    issue(0);
+    if (!whole(0)) copy(0);
     cp_async_commit();
     for (int i = 0; i < chunks; ++i) {
-      if (i + 1 < chunks) issue(i + 1);
+      if (i + 1 < chunks && !whole(i + 1)) copy(i + 1);
       cp_async_commit();
-      cp_async_wait<1>();
-      unsigned char* st = smem + stage_at(i);
-      const float* vec = reinterpret_cast<const float*>(st + B::kVec);
+      cp_async_wait<1>();                                  // empty groups where chunks come by TMA
+      wait(WB_BLOB + (i & 1), (i >> 1) & 1, 12);
       if constexpr (kMem) {
-        wait(WB_BLOB + (i & 1), (i >> 1) & 1, 6);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {                      // w V of the pieces this thread has fetched
+        unsigned char* st = smem + stage_at(i);
+        const float* vec = reinterpret_cast<const float*>(st + B::kVec);
+#pragma unroll 2
+        for (int j = 0; j < 8; ++j) {                      // w V; a thread takes the pieces that it may have copied
           const int r = j * 8 + (t >> 4), at = tile_at(r, (t & 15) * 8);
           const float w = vec[B::kWrite + r];
           const uint4 x = *reinterpret_cast<const uint4*>(st + St::kV + at);
@@ -376,7 +430,8 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const WalkP
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&xs[e]));
-            split2(f.x * w, f.y * w, hi[e], lo[e]);
+            const float2 y = mul_f32x2(f, make_float2(w, w));
+            split2(y.x, y.y, hi[e], lo[e]);
           }
           *reinterpret_cast<uint4*>(st + St::kW + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
           *reinterpret_cast<uint4*>(st + St::kW + kWalkV + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
@@ -384,59 +439,42 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const WalkP
       }
       tc::fence_async_proxy();
       tc::mbar_arrive(bar(WB_FULL + (i & 1)));
-      if (kState && first_block) {
-        wait(WB_BLOB + (i & 1), (i >> 1) & 1, 7);
-        if (t < K) prod *= kMem ? vec[B::kDecay] : vec[t];
-      }
-      if constexpr (kMem) {
-        if (keeps_n) {
-          constexpr int kPer = K / 32;
-          if (!kState) {
-            asm volatile("bar.sync 2, 128;" ::: "memory");               // Q is here
-            // sixteen tokens a warp: partial sums over a lane's channels, then halves change hands until a lane has one token
-            float d[16];
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-              const unsigned char* qr = st + St::kQ + tile_at(lw * 16 + r, lane * kPer);
-              d[r] = 0.f;
-#pragma unroll
-              for (int e = 0; e < kPer; e += 2) {
-                const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(qr + e * 2));
-                d[r] = fmaf(n[e + 1], f.y, fmaf(n[e], f.x, d[r]));
-              }
-            }
-#pragma unroll
-            for (int half = 8; half >= 1; half >>= 1) {
-              const bool up = lane & (2 * half);
-#pragma unroll
-              for (int r = 0; r < half; ++r) {
-                const float keep = up ? d[r + half] : d[r], give = up ? d[r] : d[r + half];
-                d[r] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * half);
-              }
-            }
-            const float dot = d[0] + __shfl_xor_sync(0xffffffffu, d[0], 1);
-            const int tok = lw * 16 + (lane >> 1);
-            if (!(lane & 1) && tok < min(kChunk, n_tok - i * kChunk))
-              p.den[(static_cast<int64_t>(first) + i * kChunk + tok) * p.heads + h] =
-                  fmaxf(fabsf(fmaf(vec[B::kAlpha + tok], dot, vec[B::kRow + tok])), vec[B::kFloor + tok]) + kMemFloor;
-          }
-#pragma unroll
-          for (int e = 0; e < kPer; ++e) n[e] = fmaf(vec[B::kDecay], n[e], vec[B::kSum + lane * kPer + e]);
-        }
-      }
     }
     cp_async_wait<0>();
-    if (kState && first_block && t < p.K) p.seg_decay[seg_pair * p.K + t] = prod;
-    if constexpr (kMem) {
-      if (keeps_n && lw == 0 && (kState || (last_seg && live))) {
-        float* dst = kState ? p.seg_n + seg_pair * p.K : p.n_state + pair * p.K;
+  } else if (warp == 17) {
+    // ---------------------------------------------------------------- loads
+    if (lane == 0) {
+      for (int i = 0; i < chunks; ++i) {
+        const uint32_t st = base + stage_at(i), b = bar(WB_BLOB + (i & 1));
+        const bool rows = whole(i);
+        if (i >= 2) wait(WB_EMPTY + (i & 1), ((i >> 1) - 1) & 1, 13);
+        const unsigned char* src = p.scratch + (static_cast<int64_t>(chunk0 + i) * p.heads + h) * B::kBytes;
+        constexpr uint32_t kBlob = kState ? (kMem ? 0 : 2 * B::kT) + B::kFloats * 4 : static_cast<uint32_t>(B::kBytes);
+        constexpr uint32_t kRows = kWalkV + (kMem ? (kState ? 1 : 2) * B::kT : 0);
+        tc::mbar_expect_tx(b, kBlob + (rows ? kRows : 0));
+        if (kState) {
+          if (!kMem) tc::bulk_load(st + B::kK, src + B::kK, 2 * B::kT, b);
+          tc::bulk_load(st + B::kVec, src + B::kVec, B::kFloats * 4, b);
+        } else {
+          tc::bulk_load(st, src, static_cast<uint32_t>(B::kBytes), b);
+        }
+        if (rows) {
+          const int row0 = first + i * kChunk;
 #pragma unroll
-        for (int e = 0; e < K / 32; ++e)
-          if (lane * (K / 32) + e < p.K) dst[lane * (K / 32) + e] = n[e];
+          for (int c = 0; c < kWalkCols; c += 64) tc::tma_load_3d(st + St::kV + c / 64 * kSlab, &map_v, h * p.V + p0 + c, row0, 0, b);
+          if constexpr (kMem) {
+#pragma unroll
+            for (int c = 0; c < K; c += 64) {
+              if (!kState) tc::tma_load_3d(st + St::kQ + c / 64 * kSlab, &map_q, h * p.K + c, row0, 0, b);
+              tc::tma_load_3d(st + St::kK + c / 64 * kSlab, &map_k, h * p.K + c, row0, 0, b);
+            }
+          }
+        }
       }
+      if (s_abort)                                         // a copy may still be on its way
+        for (int i = max(0, chunks - 2); i < chunks; ++i) tc::mbar_wait_timed(bar(WB_BLOB + (i & 1)), (i >> 1) & 1);
     }
-    if (s_abort && t == 0)                                 // a bulk copy may still be on its way
-      for (int i = max(0, chunks - 2); i < chunks; ++i) tc::mbar_wait_timed(bar(WB_BLOB + (i & 1)), (i >> 1) & 1);
+    __syncwarp();
   } else {
     // ---------------------------------------------------------------- products
     constexpr uint32_t kMN = 1u << 15;                     // A is MN-major
@@ -487,42 +525,39 @@ __global__ void __launch_bounds__(kWalkThreads, 1) chunk_walk_kernel(const WalkP
   }
 }
 
-// The segments' own states become the states in front of them: per sequence, head and eight channels.
+// The segments' own states become the states in front of them, a thread per element of a sequence's and head's state; kMem: n
+// behind them.  Loads of eight segments are in flight at a time.
 constexpr int kJoinThreads = 256, kJoinBatch = 8;
 template <bool kMem>
 __global__ void __launch_bounds__(kJoinThreads) chunk_join_kernel(const WalkParams p) {
-  const int s = blockIdx.x, h = blockIdx.y, ch = blockIdx.z * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int s = blockIdx.x, h = blockIdx.y, at = blockIdx.z * kJoinThreads + threadIdx.x, size = p.K * p.V;
   const int n_tok = p.cu[s + 1] - p.cu[s];
   if (n_tok <= 0) return;
   const int per = p.seg_chunks * kChunk, segs = (n_tok + per - 1) / per, u0 = segments_before(p.cu, s, p.seg_chunks);
-  if (ch >= p.K) return;
+  if (at >= size + (kMem ? p.K : 0)) return;
   const int slot = p.slots[s], st0 = p.start[s];
-  const bool has = slot >= 0 && slot < p.num_slots && st0 > 0;
-  const int64_t pair = static_cast<int64_t>(has ? slot : 0) * p.heads + h, step = static_cast<int64_t>(p.heads) * p.K * p.V;
-  auto join = [&](float first, float* at, int64_t stride) {
-    float x = first;
-    for (int g0 = 0; g0 < segs; g0 += kJoinBatch) {
-      float own[kJoinBatch], d[kJoinBatch];
+  const bool has = slot >= 0 && slot < p.num_slots && st0 > 0, in_n = at >= size;
+  const int64_t pair = static_cast<int64_t>(has ? slot : 0) * p.heads + h, unit = static_cast<int64_t>(u0) * p.heads + h;
+  const int ch = in_n ? at - size : at / p.V;
+  float* own_at = in_n ? p.seg_n + unit * p.K + ch : p.seg_state + unit * size + at;
+  const int64_t step = static_cast<int64_t>(p.heads) * (in_n ? p.K : size);
+  const float* decay = p.seg_decay + unit * p.K + ch;
+  float x = !has ? 0.f : in_n ? p.n_state[pair * p.K + ch] : p.state[pair * size + at];
+  for (int g0 = 0; g0 < segs; g0 += kJoinBatch) {
+    float own[kJoinBatch], d[kJoinBatch];
 #pragma unroll
-      for (int j = 0; j < kJoinBatch; ++j) {
-        const bool ok = g0 + j < segs - 1;
-        own[j] = ok ? at[(g0 + j) * stride] : 0.f;
-        d[j] = ok ? p.seg_decay[(static_cast<int64_t>(u0 + g0 + j) * p.heads + h) * p.K + ch] : 0.f;
-      }
-#pragma unroll
-      for (int j = 0; j < kJoinBatch; ++j)
-        if (g0 + j < segs) {
-          at[(g0 + j) * stride] = x;
-          x = fmaf(x, d[j], own[j]);
-        }
+    for (int j = 0; j < kJoinBatch; ++j) {
+      const bool ok = g0 + j < segs - 1;
+      own[j] = ok ? own_at[(g0 + j) * step] : 0.f;
+      d[j] = ok ? decay[static_cast<int64_t>(g0 + j) * p.heads * p.K] : 0.f;
     }
-  };
-  for (int v = lane; v < p.V; v += 32)
-    join(has ? p.state[(pair * p.K + ch) * p.V + v] : 0.f,
-         p.seg_state + ((static_cast<int64_t>(u0) * p.heads + h) * p.K + ch) * p.V + v, step);
-  if (kMem && lane == 0)
-    join(has ? p.n_state[pair * p.K + ch] : 0.f, p.seg_n + (static_cast<int64_t>(u0) * p.heads + h) * p.K + ch,
-         static_cast<int64_t>(p.heads) * p.K);
+#pragma unroll
+    for (int j = 0; j < kJoinBatch; ++j)
+      if (g0 + j < segs) {
+        own_at[(g0 + j) * step] = x;
+        x = fmaf(x, d[j], own[j]);
+      }
+  }
 }
 
 // The sizes the walk takes; the register form (state_chunk.cuh) keeps the narrow ones, where most of 128 lanes would idle.
@@ -554,16 +589,24 @@ int run_walk(const char* what, WalkParams p, int64_t tokens, float* segments, cu
   constexpr int smem = WalkStage<K, kMem>::kSmem;
   static_assert(smem + 256 <= 227 * 1024, "a CTA's shared memory");
   const dim3 grid(static_cast<unsigned>(units), p.heads, (p.V + kWalkCols - 1) / kWalkCols);
+  CUtensorMap maps[3] = {};
+  p.tma = !kMem || p.K % 64 == 0;                          // a box of 64 columns of q or k stays within its head
+  const __nv_bfloat16* from[3] = {kMem ? p.q : p.v, kMem ? p.k : p.v, p.v};
+  for (int i = 0; i < 3 && p.tma; ++i) {
+    const int64_t cols = static_cast<int64_t>(p.heads) * (i < 2 && kMem ? p.K : p.V);
+    const int rc = make_tmap_bf16(&maps[i], from[i], cols, tokens, 1, p.stride, p.stride * tokens, kChunk, 1, what);
+    if (rc) return rc;
+  }
   auto launch = [&](auto kernel, dim3 g) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return fail(MV_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-    kernel<<<g, kWalkThreads, smem, st>>>(p);
+    kernel<<<g, kWalkThreads, smem, st>>>(p, maps[0], maps[1], maps[2]);
     return check_launch(what);
   };
   if (p.seg_chunks) {
     int rc = launch(chunk_walk_kernel<K, kMem, true>, grid);
     if (rc) return rc;
-    chunk_join_kernel<kMem><<<dim3(p.num_seqs, p.heads, (p.K + 7) / 8), kJoinThreads, 0, st>>>(p);
+    chunk_join_kernel<kMem><<<dim3(p.num_seqs, p.heads, (p.K * (p.V + (kMem ? 1 : 0)) + kJoinThreads - 1) / kJoinThreads), kJoinThreads, 0, st>>>(p);
     rc = check_launch(what);
     if (rc) return rc;
   }

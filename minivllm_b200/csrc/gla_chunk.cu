@@ -34,6 +34,23 @@ template <int K> struct GlaScratch {
   static constexpr int64_t kBytes = kDecay * 2 + K * 4;
 };
 
+// -log(sigmoid(z)) = max(-z, 0) + log(1 + e), e = e^-|z|, in 32-bit: e from ex2.approx with the rounding of its argument put
+// back, log(1 + e) = 2 artanh(e / (2 + e)) by the series of artanh up to the 13th power (the next is below 2^-26 of it at e = 1).
+// A third of the instructions of log1pf(expf(-z)), of which this kernel needs one per channel and token.
+__device__ __forceinline__ float neg_log_sigmoid(float z) {
+  constexpr float kHi = 1.44269502f, kLo = 1.92596303e-8f;         // log2(e) in two terms
+  const float a = fmaxf(-fabsf(z), -200.f), t = a * kHi, r = fmaf(a, kLo, fmaf(a, kHi, -t));
+  const float e = fast_exp2(t) * fmaf(r, 0.693147182f, 1.f);
+  const float s = __fdividef(e, 2.f + e), q = s * s;
+  float x = fmaf(q, 1.f / 13.f, 1.f / 11.f);
+  x = fmaf(x, q, 1.f / 9.f);
+  x = fmaf(x, q, 1.f / 7.f);
+  x = fmaf(x, q, 1.f / 5.f);
+  x = fmaf(x, q, 1.f / 3.f);
+  x = fmaf(x, q, 1.f);
+  return fmaf(2.f * s, x, max_nan(-z, 0.f));
+}
+
 template <int K> struct GlaPrepShape {
   static constexpr int kRow = K + 8;                     // bf16 rows of q and k, then fp32 rows of k's factors in the same place
   // tables (block, channel): sum of a block's logarithms, and 2 to the power of what is in front of the block, of what follows it
@@ -44,7 +61,7 @@ template <int K> struct GlaPrepShape {
 
 // Two CTAs of 16 warps per SM.  A channel's two powers of a token, from the token to the edge of its block of 16, are formed once;
 // everything else is products with a block's: the operands relative to the chunk's ends, and A's blocks.
-// 1 x 16,384 tokens, 8 heads of 128: 168 us with powers formed per pair of blocks and logits read one by one
+// 1 x 16,384 tokens, 8 heads of 128: 168 us with powers formed per pair of blocks and logits read one by one, 105 us now
 template <int K, bool kTime, bool kWalk>
 __global__ void __launch_bounds__(kGpThreads, 2) gla_prepare_kernel(const GlaChunkParams p) {
   using Sh = GlaPrepShape<K>;
@@ -86,7 +103,7 @@ __global__ void __launch_bounds__(kGpThreads, 2) gla_prepare_kernel(const GlaChu
     cp_async_commit();
   }
   auto log_decay = [&](float z, int c) {
-    return (kTime ? time_log_decay(z + __bfloat162float(p.w0[h * p.K + c])) : channel_log_decay(z, p.inv_tau)) * kLog2e;
+    return (kTime ? time_log_decay(z + __bfloat162float(p.w0[h * p.K + c])) : -neg_log_sigmoid(z) * p.inv_tau) * kLog2e;
   };
   if (p.z_vec) {                                         // rows of z on 16-byte boundaries, K a multiple of eight
     for (int i = tid; i < kChunk * (K / 8); i += kGpThreads) {
@@ -197,23 +214,35 @@ __global__ void __launch_bounds__(kGpThreads, 2) gla_prepare_kernel(const GlaChu
     }
   }
   float2 qt[kPairs], kt[kPairs];
+  // the rows of one step of a thread lie in one block of 16 when 512 threads cover 8 or 16 of them: its edges are read once
+  constexpr int kRows = kGpThreads / (K / 2), kStep = kGpThreads % (K / 2) || kRows > 16 ? 1 : 16 / kRows;
 #pragma unroll
-  for (int m = 0; m < kPairs; ++m) {
-    const int i = tid + m * kGpThreads, r = i / (K / 2), c = (i % (K / 2)) * 2, blk = r >> 4;
-    const float2 b = *reinterpret_cast<const float2*>(sB + r * R + c), e = *reinterpret_cast<const float2*>(sE + r * R + c);
-    const float2 ref = *reinterpret_cast<const float2*>(sB + (blk * 16 - 1) * R + c), end = *reinterpret_cast<const float2*>(sB + (blk * 16 + 15) * R + c);
-    const float2 front = *reinterpret_cast<const float2*>(tab(Sh::kFront, blk) + c), behind = *reinterpret_cast<const float2*>(tab(Sh::kBehind, blk) + c);
-    const float2 q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sQ + r * R + c));
-    const float2 k = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sK + r * R + c));
-    qt[m] = make_float2(q.x * fast_exp2(e.x - ref.x), q.y * fast_exp2(e.y - ref.y));
-    kt[m] = make_float2(k.x * fast_exp2(end.x - b.x), k.y * fast_exp2(end.y - b.y));
-    uint32_t hi, lo;
-    split2(qt[m].x * p.q_scale * front.x, qt[m].y * p.q_scale * front.y, hi, lo);
-    tile(0, r, c) = hi;
-    tile(1, r, c) = lo;
-    split2(kt[m].x * behind.x, kt[m].y * behind.y, hi, lo);
-    tile(2, r, c) = hi;
-    tile(3, r, c) = lo;
+  for (int m0 = 0; m0 < kPairs; m0 += kStep) {
+    float2 ref, end, front, behind;
+#pragma unroll
+    for (int m = m0; m < m0 + kStep; ++m) {
+      const int i = tid + m * kGpThreads, r = i / (K / 2), c = (i % (K / 2)) * 2;
+      if (m == m0) {
+        const int blk = r >> 4;
+        ref = *reinterpret_cast<const float2*>(sB + (blk * 16 - 1) * R + c), end = *reinterpret_cast<const float2*>(sB + (blk * 16 + 15) * R + c);
+        front = *reinterpret_cast<const float2*>(tab(Sh::kFront, blk) + c), behind = *reinterpret_cast<const float2*>(tab(Sh::kBehind, blk) + c);
+        front.x *= p.q_scale; front.y *= p.q_scale;
+      }
+      const float2 b = *reinterpret_cast<const float2*>(sB + r * R + c), e = *reinterpret_cast<const float2*>(sE + r * R + c);
+      const float2 q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sQ + r * R + c));
+      const float2 k = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(sK + r * R + c));
+      const float2 ex = add_f32x2(e, make_float2(-ref.x, -ref.y)), ey = add_f32x2(end, make_float2(-b.x, -b.y));
+      qt[m] = mul_f32x2(q, make_float2(fast_exp2(ex.x), fast_exp2(ex.y)));
+      kt[m] = mul_f32x2(k, make_float2(fast_exp2(ey.x), fast_exp2(ey.y)));
+      uint32_t hi, lo;
+      const float2 qo = mul_f32x2(qt[m], front), ko = mul_f32x2(kt[m], behind);
+      split2(qo.x, qo.y, hi, lo);
+      tile(0, r, c) = hi;
+      tile(1, r, c) = lo;
+      split2(ko.x, ko.y, hi, lo);
+      tile(2, r, c) = hi;
+      tile(3, r, c) = lo;
+    }
   }
   if (kWalk) zero_upper(tid, kGpThreads, [&](int r, int c, int x) -> uint32_t& { return local(x, r, c); });
   __syncthreads();                                       // q, k and b are read
@@ -439,7 +468,7 @@ static int run_chunks(const char* what, const mv::GlaChunkParams& p, int64_t tok
       const int rc = prepare(gla_prepare_kernel<K, kTime, true>, GlaPrepShape<K>::kBytes);
       if (rc) return rc;
       const WalkParams w{p.out, p.out_stride, nullptr, nullptr, nullptr, p.v, p.stride, p.cu, p.slots, p.start, num_seqs, p.state, nullptr,
-                         p.num_slots, heads, dim, vdim, p.scratch, 0, nullptr, nullptr, nullptr, error_word};
+                         p.num_slots, heads, dim, vdim, p.scratch, 0, nullptr, nullptr, nullptr, error_word, false};
       return run_walk<K, false>(what, w, tokens, reinterpret_cast<float*>(p.scratch + chunks * heads * WalkBlob<K, false>::kBytes), st);
     };
     return dim <= 64 ? walk(std::integral_constant<int, 64>{}) : walk(std::integral_constant<int, 128>{});

@@ -363,7 +363,7 @@ extern "C" int mv_mlstm_chunk_scan(void* out, int64_t out_stride, float* den, co
       const int rc = check_launch("mlstm_prepare");
       if (rc) return rc;
       const WalkParams w{p.out, p.out_stride, p.den, p.q, p.k, p.v, p.stride, p.cu, p.slots, p.start, num_seqs, p.state, p.n_state,
-                         p.num_slots, heads, dim, vdim, p.scratch, 0, nullptr, nullptr, nullptr, error_word};
+                         p.num_slots, heads, dim, vdim, p.scratch, 0, nullptr, nullptr, nullptr, error_word, false};
       return run_walk<K, true>("mlstm_chunk", w, tokens, reinterpret_cast<float*>(p.scratch + chunks * heads * Wb::kBytes), st);
     };
     return dim <= 64 ? walk(std::integral_constant<int, 64>{}) : walk(std::integral_constant<int, 128>{});
