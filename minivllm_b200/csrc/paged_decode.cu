@@ -72,13 +72,13 @@ paged_decode_kernel(const DecodeParams p) {
   const int g = lane >> 2, t = lane & 3;
 
   const DecodePlan plan = build_plan(p, s_start, s_red);
-  if (blockIdx.x == 0) {
+  if (p.arrivals == nullptr && blockIdx.x == 0) {
     for (int b = tid; b < p.batch; b += kDecThreads) p.binfo[b] = seq_items(s_start, plan, b);
   }
   zero_empty_sequences<T, D>(p, s_start);
 
   const int ydim = p.num_kv_heads * p.mtiles;
-  const long long n_units = static_cast<long long>(plan.n_seg) * ydim;
+  const int n_units = plan.n_seg * ydim;
   const uint32_t ring = smem_u32(smem) + warp * S::kWarpBytes;
   const T* kc = static_cast<const T*>(p.k_cache);
   const T* vc = static_cast<const T*>(p.v_cache);
@@ -93,7 +93,7 @@ paged_decode_kernel(const DecodeParams p) {
     if (at.b < 0) return false;
     it.kvh = at.y / p.mtiles;
     it.mt = at.y - it.kvh * p.mtiles;
-    const DecodeItem di = piece_of(s_start, plan, at.b, at.seg);
+    const DecodeItem di = piece_of(p, s_start, plan, at.b, at.seg);
     it.item = di.item;
     it.b = di.b; it.nsplit = di.nsplit; it.tok_begin = di.tok_begin; it.tok_end = di.tok_end;
     it.table = p.block_tables + static_cast<int64_t>(di.b) * p.bt_stride;
@@ -103,19 +103,24 @@ paged_decode_kernel(const DecodeParams p) {
     it.my_tiles = cta_tiles > warp ? (cta_tiles - warp + kDecWarps - 1) / kDecWarps : 0;
     return true;
   };
-  // ring stage <- tile i of this warp within item `it` (no commit)
-  auto issue_tile = [&](const Item& it, int i, int stage) {
+  // Tile i of this warp within item `it`, first half: lane r (r < 16) asks the block table for row r, others mirror it.
+  struct Row {
+    int block, off;
+  };
+  auto look_up = [&](const Item& it, int i) {
     const int tok0 = it.tok_begin + (i * kDecWarps + warp) * kTileTok;
     const int blk0 = tok0 / bs, off0 = tok0 - blk0 * bs;
-    // lane r (r < 16) resolves row r; others mirror it
     const int r_me = lane & 15;
-    int off = off0 + r_me, blk = blk0;
-    while (off >= bs) { off -= bs; ++blk; }
-    int slot = -1;
-    if (tok0 + r_me < it.tok_end) {
-      const int pb = __ldg(it.table + blk);
-      if (pb >= 0 && pb < p.num_blocks) slot = pb * bs + off;
-    }
+    Row row;
+    row.off = off0 + r_me;
+    int blk = blk0;
+    while (row.off >= bs) { row.off -= bs; ++blk; }
+    row.block = tok0 + r_me < it.tok_end ? __ldg(it.table + blk) : -1;
+    return row;
+  };
+  // second half: ring stage <- the rows looked up (no commit)
+  auto issue_tile = [&](int kvh, const Row& row, int stage) {
+    const int slot = row.block >= 0 && row.block < p.num_blocks ? row.block * bs + row.off : -1;
     const uint32_t live = __ballot_sync(0xffffffffu, slot >= 0) & 0xffffu;
     if (lane == 0) s_mask[warp][stage] = live;
     const uint32_t kdst = ring + stage * S::kStageBytes;
@@ -125,7 +130,7 @@ paged_decode_kernel(const DecodeParams p) {
     for (int li = 0; li < LOAD_ITERS; ++li) {
       const int r = r0 + li * RPI;
       const int s = __shfl_sync(0xffffffffu, slot, r);
-      const int64_t eoff = s >= 0 ? (static_cast<int64_t>(s) * p.num_kv_heads + it.kvh) * D + c * 8 : 0;
+      const int64_t eoff = s >= 0 ? (static_cast<int64_t>(s) * p.num_kv_heads + kvh) * D + c * 8 : 0;
       const uint32_t doff = r * S::kRowBytes + ((c ^ (r & 7)) << 4);
       cp_async16(kdst + doff, kc + eoff, s >= 0 ? 16 : 0);
       cp_async16(vdst + doff, vc + eoff, s >= 0 ? 16 : 0);
@@ -138,37 +143,62 @@ paged_decode_kernel(const DecodeParams p) {
   Item load_it;
   bool load_valid = false;
   int load_tile = 0, load_slot = 0, use_slot = 0;
-  auto issue_next = [&]() {
+  Row load_row = {-1, 0};
+  auto next_tile = [&]() {                  // to the next tile there is, and asks for its rows
     while (load_valid && load_tile >= load_it.my_tiles) {
       walk_next(p, s_start, plan, ydim, n_units, gridDim.x, load_at);
       load_valid = load_item(load_at, load_it);
       load_tile = 0;
     }
+    if (load_valid) load_row = look_up(load_it, load_tile);
+  };
+  auto issue_next = [&]() {
     if (load_valid) {
-      issue_tile(load_it, load_tile, load_slot % kDecStages);
+      const Row row = load_row;             // asked for a tile ago
+      const int kvh = load_it.kvh;
       ++load_tile;
+      next_tile();
+      issue_tile(kvh, row, load_slot % kDecStages);
     }
     cp_async_commit();
     ++load_slot;
   };
+  // Q fragments: rows g and g+8 of the 16-row tile, zero past the group (the streaming form has no rows above 8).
+  uint32_t qa[KSTEPS][4];
+  auto load_q = [&](const Item& it) {
+    const int h0 = it.kvh * p.group + it.mt * 16, rows = min(16, p.group - it.mt * 16);
+    const T* qbase = static_cast<const T*>(p.q) + (static_cast<int64_t>(it.b) * p.num_heads + h0) * D;
+    const bool v0 = g < rows, v1 = !kStream && g + 8 < rows;
+    const uint32_t* q0 = reinterpret_cast<const uint32_t*>(qbase + static_cast<int64_t>(g) * D);
+    const uint32_t* q1 = reinterpret_cast<const uint32_t*>(qbase + static_cast<int64_t>(g + 8) * D);
+#pragma unroll
+    for (int ks = 0; ks < KSTEPS; ++ks) {
+      qa[ks][0] = v0 ? __ldg(q0 + ks * 8 + t) : 0u;
+      qa[ks][1] = v1 ? __ldg(q1 + ks * 8 + t) : 0u;
+      qa[ks][2] = v0 ? __ldg(q0 + ks * 8 + 4 + t) : 0u;
+      qa[ks][3] = v1 ? __ldg(q1 + ks * 8 + 4 + t) : 0u;
+    }
+  };
   if constexpr (kStream) {
     walk_start(p, s_start, plan, ydim, n_units, blockIdx.x, load_at);
     load_valid = load_item(load_at, load_it);
-#pragma unroll
+    if (load_valid) load_q(load_it);
+    next_tile();
+#pragma unroll 1
     for (int i = 0; i < kDecStages - 1; ++i) issue_next();
   }
 
   ItemWalk at;
-  for (walk_start(p, s_start, plan, ydim, n_units, blockIdx.x, at); at.b >= 0;
-       walk_next(p, s_start, plan, ydim, n_units, gridDim.x, at)) {
-    Item cur;
-    load_item(at, cur);
+  walk_start(p, s_start, plan, ydim, n_units, blockIdx.x, at);
+  Item cur;
+  load_item(at, cur);
+  while (at.b >= 0) {
     const int item = cur.item, kvh = cur.kvh, mt = cur.mt, b = cur.b, nsplit = cur.nsplit, my_tiles = cur.my_tiles;
     const int rows_valid = min(16, p.group - mt * 16);
     const int h0 = kvh * p.group + mt * 16;
 
     auto issue = [&](int i) {   // not streaming: stage i % kDecStages <- tile i of this item (or nothing past its end)
-      if (i < my_tiles) issue_tile(cur, i, i % kDecStages);
+      if (i < my_tiles) issue_tile(kvh, look_up(cur, i), i % kDecStages);
       cp_async_commit();
     };
 
@@ -177,21 +207,7 @@ paged_decode_kernel(const DecodeParams p) {
       for (int i = 0; i < kDecStages - 1; ++i) issue(i);
     }
 
-    // Q fragments: rows g and g+8 of the 16-row tile, zero past the group.
-    uint32_t qa[KSTEPS][4];
-    {
-      const T* qbase = static_cast<const T*>(p.q) + (static_cast<int64_t>(b) * p.num_heads + h0) * D;
-      const bool v0 = g < rows_valid, v1 = g + 8 < rows_valid;
-      const uint32_t* q0 = reinterpret_cast<const uint32_t*>(qbase + static_cast<int64_t>(g) * D);
-      const uint32_t* q1 = reinterpret_cast<const uint32_t*>(qbase + static_cast<int64_t>(g + 8) * D);
-#pragma unroll
-      for (int ks = 0; ks < KSTEPS; ++ks) {
-        qa[ks][0] = v0 ? __ldg(q0 + ks * 8 + t) : 0u;
-        qa[ks][1] = v1 ? __ldg(q1 + ks * 8 + t) : 0u;
-        qa[ks][2] = v0 ? __ldg(q0 + ks * 8 + 4 + t) : 0u;
-        qa[ks][3] = v1 ? __ldg(q1 + ks * 8 + 4 + t) : 0u;
-      }
-    }
+    if constexpr (!kStream) load_q(cur);
 
     float o[NT][4];
 #pragma unroll
@@ -231,23 +247,27 @@ paged_decode_kernel(const DecodeParams p) {
         for (int e = 0; e < 4; ++e) {
           const int col = n * 8 + 2 * t + (e & 1);
           const bool ok = (live >> col) & 1u;
+          if (kStream && e > 1) continue;
           s[n][e] = ok ? s[n][e] * p.scale_log2 : -INFINITY;
         }
         mx0 = fmaxf(mx0, fmaxf(s[n][0], s[n][1]));
-        mx1 = fmaxf(mx1, fmaxf(s[n][2], s[n][3]));
+        if (!kStream) mx1 = fmaxf(mx1, fmaxf(s[n][2], s[n][3]));
       }
       mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
       mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-      mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-      const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
-      const float a0 = fast_exp2(m0 - mn0), a1 = fast_exp2(m1 - mn1);
+      if (!kStream) {
+        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+      }
+      const float mn0 = fmaxf(m0, mx0), mn1 = kStream ? m1 : fmaxf(m1, mx1);
+      const float a0 = fast_exp2(m0 - mn0), a1 = kStream ? 1.f : fast_exp2(m1 - mn1);
       m0 = mn0; m1 = mn1;
       float ps0 = 0.f, ps1 = 0.f;
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
         s[n][0] = fast_exp2(s[n][0] - mn0); s[n][1] = fast_exp2(s[n][1] - mn0);
-        s[n][2] = fast_exp2(s[n][2] - mn1); s[n][3] = fast_exp2(s[n][3] - mn1);
+        s[n][2] = kStream ? 0.f : fast_exp2(s[n][2] - mn1);
+        s[n][3] = kStream ? 0.f : fast_exp2(s[n][3] - mn1);
         ps0 += s[n][0] + s[n][1];
         ps1 += s[n][2] + s[n][3];
       }
@@ -267,6 +287,10 @@ paged_decode_kernel(const DecodeParams p) {
         for (int n = 0; n < 2; ++n) {
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
+            if (kStream && hh) {
+              pl[2 * n + hh] = 0u;
+              continue;
+            }
             const float2 hi = Elem<T>::to_f2(*reinterpret_cast<const typename Elem<T>::T2*>(&pa[2 * n + hh]));
             pl[2 * n + hh] = pack2<T>(s[n][2 * hh] - hi.x, s[n][2 * hh + 1] - hi.y);
           }
@@ -275,7 +299,10 @@ paged_decode_kernel(const DecodeParams p) {
       // the running maximum rarely moves after the first tiles: rescale only when some row of the warp needs it
       if (__any_sync(0xffffffffu, a0 != 1.f || a1 != 1.f)) {
 #pragma unroll
-        for (int j = 0; j < NT; ++j) { o[j][0] *= a0; o[j][1] *= a0; o[j][2] *= a1; o[j][3] *= a1; }
+        for (int j = 0; j < NT; ++j) {
+          o[j][0] *= a0; o[j][1] *= a0;
+          if (!kStream) { o[j][2] *= a1; o[j][3] *= a1; }
+        }
       }
       {
         const int row = (lane & 7) + (((lane >> 3) & 1) << 3);
@@ -301,6 +328,12 @@ paged_decode_kernel(const DecodeParams p) {
     l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
     l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+
+    ItemWalk next_at = at;
+    walk_next(p, s_start, plan, ydim, n_units, gridDim.x, next_at);
+    Item next;
+    const bool more = load_item(next_at, next);
+    if (kStream && more) load_q(next);        // on its way during the merge
 
     // ---- merge the four warps through shared memory ----
     if constexpr (kStream) {
@@ -344,6 +377,8 @@ paged_decode_kernel(const DecodeParams p) {
       __syncthreads();  // the ring is handed back to the pipelines
       combine_if_last<T, D>(p, s_start, plan, b, b * ydim + kvh * p.mtiles + mt, h0, rows_valid, nsplit, &s_last);
     }
+    at = next_at;
+    cur = next;
   }
   if constexpr (kStream) cp_async_wait<0>();   // only empty groups are left
 }

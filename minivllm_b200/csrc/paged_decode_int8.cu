@@ -79,13 +79,13 @@ paged_decode_int8_kernel(const DecodeParams p) {
   const int g = lane >> 2, t = lane & 3;
 
   const DecodePlan plan = build_plan(p, s_start, s_red);
-  if (blockIdx.x == 0) {
+  if (p.arrivals == nullptr && blockIdx.x == 0) {
     for (int b = tid; b < p.batch; b += kDecThreads) p.binfo[b] = seq_items(s_start, plan, b);
   }
   zero_empty_sequences<T, D>(p, s_start);
 
   const int ydim = p.num_kv_heads * p.mtiles;
-  const long long n_units = static_cast<long long>(plan.n_seg) * ydim;
+  const int n_units = plan.n_seg * ydim;
   const uint32_t ring = smem_u32(smem) + warp * S::kWarpBytes;
   const int8_t* kc = static_cast<const int8_t*>(p.k_cache);
   const int8_t* vc = static_cast<const int8_t*>(p.v_cache);
@@ -95,7 +95,7 @@ paged_decode_int8_kernel(const DecodeParams p) {
   for (walk_start(p, s_start, plan, ydim, n_units, blockIdx.x, at); at.b >= 0;
        walk_next(p, s_start, plan, ydim, n_units, gridDim.x, at)) {
     const int kvh = at.y / p.mtiles, mt = at.y - kvh * p.mtiles;
-    const DecodeItem di = piece_of(s_start, plan, at.b, at.seg);
+    const DecodeItem di = piece_of(p, s_start, plan, at.b, at.seg);
     const int item = di.item, b = di.b, nsplit = di.nsplit, tok_begin = di.tok_begin, tok_end = di.tok_end;
     const int32_t* table = p.block_tables + static_cast<int64_t>(b) * p.bt_stride;
     const int rows_valid = min(16, p.group - mt * 16);
@@ -376,12 +376,12 @@ paged_decode_int8_tok_kernel(const DecodeParams p) {
   const int g = lane >> 2, t = lane & 3;
 
   const DecodePlan plan = build_plan<kQ8Warps>(p, s_start, s_red);
-  if (blockIdx.x == 0) {
+  if (p.arrivals == nullptr && blockIdx.x == 0) {
     for (int b = tid; b < p.batch; b += kQ8Warps * 32) p.binfo[b] = seq_items(s_start, plan, b);
   }
   zero_empty_sequences<T, D>(p, s_start);
   const int ydim = p.num_kv_heads;
-  const long long n_units = static_cast<long long>(plan.n_seg) * ydim;
+  const int n_units = plan.n_seg * ydim;
   const uint32_t ring = smem_u32(smem) + warp * S::kWarpBytes;
   const int8_t* kc = static_cast<const int8_t*>(p.k_cache);
   const int8_t* vc = static_cast<const int8_t*>(p.v_cache);
@@ -391,7 +391,7 @@ paged_decode_int8_tok_kernel(const DecodeParams p) {
   for (walk_start(p, s_start, plan, ydim, n_units, blockIdx.x, at); at.b >= 0;
        walk_next(p, s_start, plan, ydim, n_units, gridDim.x, at)) {
     const int kvh = at.y;
-    const DecodeItem di = piece_of(s_start, plan, at.b, at.seg);
+    const DecodeItem di = piece_of(p, s_start, plan, at.b, at.seg);
     const int b = di.b, tok_begin = di.tok_begin, tok_end = di.tok_end;
     const int32_t* table = p.block_tables + static_cast<int64_t>(b) * p.bt_stride;
     const int rows_valid = p.group, h0 = kvh * p.group;

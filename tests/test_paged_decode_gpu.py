@@ -123,6 +123,24 @@ def test_decode_segment_cuts_on_and_off_sequence_boundaries(dtype):
         assert torch.count_nonzero(got[b]) == 0
 
 
+@pytest.mark.parametrize("kv,lens", [
+    (4, [63, 64, 65, 129, 0, 256, 257, 1, 190]),        # few sequences: each begins a segment of its own
+    (8, [64] * 36 + [65]),                              # one piece more than there is room for with the shortest segments
+    (8, [1500] * 30 + [1] * 7),                         # as many sequences as segments
+    (1, [9000, 40, 0, 700]),                            # more than eight pieces to reduce
+    (64, [300, 20, 128]),                               # one or no segment for a KV head
+])
+def test_decode_pieces_of_few_sequences(kv, lens):
+    d = synth.decode_inputs(seed=47, batch=len(lens), ctx_lo=max(lens), ctx_hi=max(lens), num_heads=2 * kv, num_kv_heads=kv,
+                            head_dim=128, block_size=64)
+    cl = torch.tensor(lens, dtype=d["context_lens"].dtype)
+    for dtype in (torch.float16, torch.bfloat16):
+        got, want = _gpu_decode(d, dtype, context_lens=cl), _oracle_decode(d, dtype, context_lens=cl)
+        _close(got, want, dtype)
+        for b, n in enumerate(lens):
+            assert n or torch.count_nonzero(got[b]) == 0
+
+
 def test_decode_long_context_is_split():
     """One sequence far longer than a chunk: exercises the partial-result path and the combine kernel."""
     d = synth.decode_inputs(seed=45, batch=2, ctx_lo=9000, ctx_hi=12000, num_heads=8, num_kv_heads=2, head_dim=128,

@@ -69,6 +69,16 @@ def test_int8_decode_shape_sweep(kw):
     _check(synth.decode_inputs(seed=50, head_dim=128, **kw), torch.float16)
 
 
+@pytest.mark.parametrize("kv,lens", [(4, [127, 128, 129, 0, 257, 1, 520]), (8, [1400] * 30 + [1] * 7), (1, [9000, 40, 700])])
+def test_int8_decode_pieces_of_few_sequences(kv, lens):
+    """Each sequence begins a segment of its own; with one head, more than eight pieces are reduced."""
+    d = synth.decode_inputs(seed=48, batch=len(lens), ctx_lo=max(lens), ctx_hi=max(lens), num_heads=2 * kv, num_kv_heads=kv,
+                            block_size=64)
+    got = _check(d, torch.float16, context_lens=torch.tensor(lens, dtype=d["context_lens"].dtype))
+    for b, n in enumerate(lens):
+        assert n or torch.count_nonzero(got[b]) == 0
+
+
 def test_int8_decode_long_context_split_and_holes():
     d = synth.decode_inputs(seed=51, batch=2, ctx_lo=5000, ctx_hi=9000, num_heads=8, num_kv_heads=2, block_size=256)
     bt = d["block_tables"].clone()
