@@ -255,7 +255,9 @@ def logits_dtype_code(dt):
 
 
 def stream_ptr():
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device.  Through torch.cuda.current_stream, which makes a Stream object, it took 3.3 us
+    of a call's 15.8; the handle alone takes 0.1 (and current_device, once CUDA is up, as much)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def require_cuda(*tensors):
