@@ -116,3 +116,53 @@ def test_plan_edge_cases():
     _check([1], 8, 1, 296)
     _check([100000], 1, 1, 296)                      # one sequence over all segments
     _check([0, 5, 0, 0, 70000, 0, 3, 0], 1, 1, 296)
+
+
+def padded_plan(ctx, target, step, threads):
+    """The plan of few sequences: (padded prefix sums, seg_len, n_seg), or None where the stream is cut as it is."""
+    _, seg, _ = build_plan(ctx, target)
+    seg = max(-(-(-(-sum(ctx) // target)) // step) * step, step)
+    if not 1 < len(ctx) <= min(target, threads):
+        return None
+    for seg_len in (seg, seg + step, seg + 2 * step, seg + 3 * step):
+        pieces = [-(-c // seg_len) for c in ctx]
+        assert sum(pieces) < 1 << 16                 # a 16-bit count
+        if sum(pieces) <= target:
+            s_tok = [0]
+            for n in pieces:
+                s_tok.append(s_tok[-1] + n * seg_len)
+            return s_tok, seg_len, sum(pieces)
+    return None
+
+
+def test_padded_plan_gives_every_unit_one_item():
+    rng = random.Random(1)
+    taken = 0
+    for _ in range(200):
+        batch, kvh, (step, threads) = rng.choice([2, 3, 16, 37, 100]), rng.choice([1, 2, 4, 8]), rng.choice([(64, 128), (128, 256)])
+        ctx = [rng.choice([0, 1, step, step + 1, rng.randint(1, 5000)]) for _ in range(batch)]
+        target = target_items(kvh, 1)
+        plan = padded_plan(ctx, target, step, threads)
+        if plan is None:
+            continue
+        taken += 1
+        s_tok, seg_len, n_seg = plan
+        assert n_seg * kvh <= NUM_SMS * CTAS_PER_SM
+        covered, items = {}, set()
+        for unit in range(n_seg * kvh):
+            visits = walk(s_tok, batch, seg_len, n_seg, kvh, unit, n_seg * kvh)
+            assert len(visits) == 1                  # nobody begins a second item
+            seg, y, p = visits[0]
+            end = min((seg + 1) * seg_len - s_tok[p["b"]], ctx[p["b"]])
+            assert 0 <= p["tok_begin"] < end
+            covered.setdefault((y, p["b"]), []).append((p["tok_begin"], end))
+            first, count = seq_items(s_tok, seg_len, p["b"])
+            assert count == p["nsplit"] and first <= p["item"] < first + count and p["item"] < items_max(batch, kvh, 1)
+            assert (y, p["item"]) not in items
+            items.add((y, p["item"]))
+        for y in range(kvh):
+            for b, c in enumerate(ctx):
+                iv = sorted(covered.get((y, b), []))
+                assert sum(e - a for a, e in iv) == c and all(a[1] == b_[0] for a, b_ in zip(iv, iv[1:]))
+                assert len(iv) == seq_items(s_tok, seg_len, b)[1]
+    assert taken > 100

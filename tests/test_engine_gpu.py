@@ -226,3 +226,18 @@ def test_two_prefill_waves_in_flight_keep_the_streams():
         two, eng = _run(False, max_tokens=24, config=dict(CONFIG, prefill_streams=2, **extra))
         assert eng.model_runner._prefill_at >= 3, "the prompts were meant to take several waves"
         _assert_same_up_to_near_ties(two, one, "two prefill streams against one", config=dict(CONFIG, **extra))
+
+
+def test_logits_cross_to_the_host_whole():
+    """step_logits's copy at the edges of its pieces: the values are those of `.float().cpu()`, and the error word comes along."""
+    from minivllm_b200.engine import model_runner
+    n = model_runner.SCORE_PIECE
+    for dtype, piece in ((torch.bfloat16, n), (torch.float16, n), (torch.float32, n)):
+        r = object.__new__(model_runner.ModelRunner)
+        r.max_num_seqs, r.dtype, r._score = 4, dtype, None
+        r.error_word = torch.full((1,), 7, dtype=torch.int32, device="cuda")
+        for shape in ((0, 32), (1, 1), (2, piece // 2), (1, piece + 1), (3, piece + 5), (7, 1001)):
+            x = torch.randn(shape, device="cuda").to(dtype)
+            r._score_buffers()["error"].zero_()
+            assert torch.equal(r._logits_to_host(x), x.float().cpu()), (dtype, shape)
+            assert int(r._score["error"]) == 7
