@@ -104,7 +104,6 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 // Four K = 16 steps, A and B in shared memory, by the elected lane of a converged warp; descriptors move by kA and kB units.
 template <int kA, int kB>
 __device__ __forceinline__ void mma_ss_4(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, bool accum) {

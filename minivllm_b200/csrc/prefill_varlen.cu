@@ -530,27 +530,34 @@ prefill_varlen_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
 //   live in shared memory behind the tile buffers) and publishes what the other roles need of it in a ring of
 //   descriptors (UFULL / UEMPTY), one unit ahead of the MMA warp.
 //   Q buffer: QEMPTY is committed behind the unit's last QK, the producer waits for it before the next Q.
-//   O accumulators: OFREE[t] gets 128 arrivals when head t's softmax warps have read O in the epilogue;
+//   O accumulators: OFREE[t] gets an arrival of each of head t's softmax warps when it has read O in the epilogue;
 //   the MMA warp waits for it before the first PV of head t's next unit.
-//   Output: each softmax warp transposes its 32 rows through a staging buffer so that a store instruction
-//   writes whole 128-byte lines (a thread storing its own row makes 32 lines per instruction, and the stores
-//   of one unit then hold up every shared-memory access of the SM for about 2,000 cycles).
+//   Softmax: eight warps a head, 16 rows each.  With four a head and a whole row a thread, the first tile of a unit took
+//   2,900 cycles behind its QK and the epilogue 2,000 during which the tensor cores idled: 4.3 us a unit beside its steps.  A
+//   warpgroup of its own for the epilogue was measured too: it takes issue slots from the softmax and gained half as much.
+//   Output: rows leave by TMA through each warp's staging buffer (a thread storing its own row makes 32 lines per
+//   instruction, and the stores of one unit then hold up every shared-memory access of the SM for about 2,000 cycles).
+//   32/8 heads, bf16: 32 sequences of 128 to 2048 tokens 422 -> 396 us; 16 portions behind cached halves 278 -> 243; 64 x 512
+//   tokens 306 -> 229 us.  Long sequences run at the power limit (56 % of the tensor cycles at 1.5 GHz, 1.2 PFLOP/s).
 //   Code size: the MMA warp shares an instruction cache with the large softmax loop.  Its waits are the compact
 //   form (rolled spin, the long-wait part a call) and the two warps with few registers keep their loops small;
 //   with unrolled waits the same kernel was 25 % slower on the 32-sequence benchmark.
 // ---------------------------------------------------------------------------------------------
 enum { PB_Q = 0, PB_QEMPTY = 1, PB_KFULL = 2, PB_KEMPTY = 4, PB_VFULL = 6, PB_VEMPTY = 8, PB_SFULL = 10, PB_PREADY = 12,
        PB_ODONE = 14, PB_OFREE = 16, PB_SPARE = 18, PB_DRAIN = 19, PB_UFULL = 20, PB_UEMPTY = 24, PB_COUNT = 28 };
-constexpr int kPfOutWarpBytes = 32 * 128;                    // output staging of one softmax warp: 32 rows x 64 outputs
-constexpr int kPfOutStageBytes = 8 * kPfOutWarpBytes;
-__device__ __forceinline__ void st_shared16(uint32_t addr, const uint4& v) {
-  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+constexpr int kPpSoftWarps = 16, kPpThreads = kPpSoftWarps * 32 + 128;      // registers: 512 x 104 + 128 x 64, launched with 640 x 96
+constexpr int kPfOutWarpBytes = 16 * 128;                    // output staging of one softmax warp: 16 rows x 64 outputs
+constexpr int kPfOutStageBytes = kPpSoftWarps * kPfOutWarpBytes;
+__device__ __forceinline__ void st_matrix4(uint32_t addr, const uint32_t (&r)[4]) {       // four 8 x 8 matrices of 16-bit values
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 __device__ __forceinline__ uint4 ld_shared16(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
   return v;
 }
+constexpr int kPfSortSeqs = 8;      // sequences up to which units are sorted: a lookup goes through them, several times where they
+                                    // have few tiles (at 32 sequences, 128 to 2048 tokens, 421 us instead of 395)
 constexpr int kPfUnitRing = 4;      // units handed from the producer warp to the other roles ahead of time
 constexpr int kPfSchedSlots = 1024;  // launches that can be in flight with a work counter of their own
 // Work counters of the persistent launches: [slot][0] = units handed out beyond the first one per CTA,
@@ -558,13 +565,14 @@ constexpr int kPfSchedSlots = 1024;  // launches that can be in flight with a wo
 static __device__ unsigned int g_pf_sched[kPfSchedSlots][2];
 
 template <typename T>
-__global__ void __launch_bounds__(kPfThreads, 1)
+__global__ void __launch_bounds__(kPpThreads, 1)
 prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                          const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p) {
+                          const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const PrefillParams p) {
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bars[PB_COUNT];
   __shared__ uint32_t s_tmem_base;
-  __shared__ int s_scan[16];
+  __shared__ int s_scan[kPpThreads / 32];
+  __shared__ int s_base[kPfSortSeqs];                    // KV tiles of a sequence's cached keys
   __shared__ int s_abort;
   __shared__ int s_sticky;
   __shared__ __align__(16) int s_unit[kPfUnitRing][8];   // unit descriptors, see UnitDesc
@@ -576,7 +584,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   const uint32_t q_smem = smem_base;                                  // [head 2][half 2][128][128B]
   const uint32_t k_smem = q_smem + 2 * kPfTileBytes;                  // [stage][half][128][128B]
   const uint32_t v_smem = k_smem + kPfStages * kPfTileBytes;
-  // output staging of the softmax warps (32 rows x 128 B each), then the tiles before sequence i (num_seqs + 1)
+  // output staging of the softmax warps (16 rows x 128 B each), then the tiles before sequence i (num_seqs + 1)
   const uint32_t o_smem = v_smem + kPfStages * kPfTileBytes;
   int* s_pref = reinterpret_cast<int*>(smem_raw + (smem_base - smem_u32(smem_raw)) + 2 * kPfTileBytes +
                                        2 * kPfStages * kPfTileBytes + kPfOutStageBytes);
@@ -592,12 +600,13 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   __syncthreads();
   {  // block-wide inclusive scan of the tiles per sequence
     int carry = 0;
-    for (int base = 0; base < p.num_seqs; base += kPfThreads) {
+    for (int base = 0; base < p.num_seqs; base += kPpThreads) {
       const int s = base + tid;
       int n = 0;
       if (s < p.num_seqs) {
         const int len = p.cu_seqlens[s + 1] - p.cu_seqlens[s];
         n = len > 0 ? (len + kPfTile - 1) / kPfTile : 0;
+        if (s < kPfSortSeqs) s_base[s] = p.paged ? (max(p.cu_seqlens_k[s + 1] - p.cu_seqlens_k[s] - len, 0) + kPfTile - 1) / kPfTile : 0;
       }
       int incl = n;
 #pragma unroll
@@ -609,7 +618,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
       __syncthreads();
       int wofs = 0, tot = 0;
 #pragma unroll
-      for (int w2 = 0; w2 < kPfThreads / 32; ++w2) {
+      for (int w2 = 0; w2 < kPpThreads / 32; ++w2) {
         const int v = s_scan[w2];
         if (w2 < warp) wofs += v;
         tot += v;
@@ -637,25 +646,67 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
     return;
   }
 
-  // Unit u = (head pair y, query tile x) in the order a grid of one CTA per unit would run them: x fastest, the
-  // tiles of a sequence in descending order.  CTAs that run at the same time then work on the query tiles of a
-  // few sequences for one KV head and share its K/V tiles in L2.  The first unit of a CTA is its block index;
-  // further ones come from a counter (whoever is free takes the next: the KV loops differ in length by up to
-  // the number of tiles of a sequence, and any fixed assignment leaves some SMs idle at the end).
+  // Units are (head pair y, query tile) and a CTA's first one is its block index; further ones come from a counter (whoever
+  // is free takes the next: the KV loops differ in length by up to the number of tiles of a sequence, and any fixed
+  // assignment leaves some SMs idle at the end).  Up to kPfSortSeqs sequences: longest KV loop first, so that what is left at
+  // the end is short.  A tile's place in that order is its level, the number of KV steps up to its diagonal; a sequence has
+  // one tile for each level from base + 1 on (base: KV tiles of its cached keys), so the tiles of a level are found by going
+  // through the sequences.  Head pairs are taken in as many groups as still leave the last group work for twice the
+  // longest loop on every SM: a group's K and V then stay in L2.  7 sequences of 5,142 tokens, 4/1 heads, bf16: 210 -> 181 us;
+  // one of 3,000, 32/8 heads: 99 -> 83 us.
+  // More sequences: y outermost, the tiles of a sequence in descending order (their loops are short against the whole).
   struct Unit {
     int seq, seq_start, seq_len, q0, first_pos, n_kv, kvh, head_a;
     bool has_b, split_p;
   };
-  auto get_unit = [&](long long u) {
+  const bool sorted = p.num_seqs <= kPfSortSeqs && total_units > gridDim.x && total_units <= 0x7fffffff;
+  auto tiles_of = [&](int q) { return s_pref[q + 1] - s_pref[q]; };
+  auto in_level = [&](int q, int level) { return level > s_base[q] && level <= s_base[q] + tiles_of(q); };
+  struct Order {                                       // where the producer is in the sorted order
+    int top;
+    unsigned groups;
+    int group, y0, ys, level, above, here;
+  };
+  auto get_unit = [&](long long u, Order& o) {
     Unit w;
-    const int y = static_cast<int>(u / n_tiles), x = static_cast<int>(u - static_cast<long long>(y) * n_tiles);
-    int lo = 0, hi = p.num_seqs - 1;                   // last sequence with s_pref[seq] <= x
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (s_pref[mid] <= x) lo = mid; else hi = mid - 1;
+    int y, qtile, lo = 0;
+    if (sorted) {
+      y = static_cast<int>(static_cast<unsigned>(u) / static_cast<unsigned>(n_tiles));
+      auto enter = [&](int level) {
+        o.level = level;
+        o.here = 0;
+        for (int q = 0; q < p.num_seqs; ++q) o.here += in_level(q, level) ? 1 : 0;
+      };
+      const int group = static_cast<int>((static_cast<unsigned>(y + 1) * o.groups - 1) / static_cast<unsigned>(ydim));   // ydim < 2^16
+      if (group != o.group) {
+        o.group = group;
+        o.y0 = static_cast<int>(static_cast<unsigned>(group) * ydim / o.groups);
+        o.ys = static_cast<int>(static_cast<unsigned>(group + 1) * ydim / o.groups) - o.y0;
+        o.above = 0;
+        enter(o.top);
+      }
+      const unsigned v = static_cast<unsigned>(u) - static_cast<unsigned>(o.y0) * n_tiles;
+      const int x = static_cast<int>(v / static_cast<unsigned>(o.ys));
+      y = o.y0 + static_cast<int>(v - static_cast<unsigned>(x) * o.ys);
+      while (x >= o.above + o.here && o.level > 1) {
+        o.above += o.here;
+        enter(o.level - 1);
+      }
+      int k = x - o.above;                             // the k-th sequence with a tile of this level
+      for (int q = 0; q < p.num_seqs; ++q)
+        if (in_level(q, o.level) && k-- == 0) lo = q;
+      qtile = o.level - 1 - s_base[lo];
+    } else {
+      y = static_cast<int>(u / n_tiles);
+      const int x = static_cast<int>(u - static_cast<long long>(y) * n_tiles);
+      int hi = p.num_seqs - 1;                         // last sequence with s_pref[seq] <= x
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (s_pref[mid] <= x) lo = mid; else hi = mid - 1;
+      }
+      qtile = tiles_of(lo) - 1 - (x - s_pref[lo]);
     }
     w.seq = lo;
-    const int qtile = (s_pref[lo + 1] - s_pref[lo]) - 1 - (x - s_pref[lo]);
     w.kvh = y / p.pairs;
     const int pair = y - w.kvh * p.pairs;
     w.head_a = w.kvh * p.group + 2 * pair;
@@ -696,19 +747,19 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
     }
     for (int t = 0; t < 2; ++t) {
       tc::mbar_init(bar(PB_SFULL + t), 1);
-      tc::mbar_init(bar(PB_PREADY + t), 128);
+      tc::mbar_init(bar(PB_PREADY + t), kPpSoftWarps / 2);
       tc::mbar_init(bar(PB_ODONE + t), 1);
-      tc::mbar_init(bar(PB_OFREE + t), 128);
+      tc::mbar_init(bar(PB_OFREE + t), kPpSoftWarps / 2);
     }
     tc::mbar_init(bar(PB_SPARE), 1);   // takes commits that nobody waits for
     tc::mbar_init(bar(PB_DRAIN), 1);
     for (int i = 0; i < kPfUnitRing; ++i) {
       tc::mbar_init(bar(PB_UFULL + i), 1);
-      tc::mbar_init(bar(PB_UEMPTY + i), 9);   // the MMA warp and the eight softmax warps
+      tc::mbar_init(bar(PB_UEMPTY + i), 1 + kPpSoftWarps);   // the MMA warp and the softmax warps
     }
     tc::mbar_fence_init();
   }
-  if (warp == 8) {
+  if (warp == kPpSoftWarps) {
     tc::tmem_alloc(smem_u32(&s_tmem_base), 512);
     tc::tmem_relinquish();
   }
@@ -718,10 +769,24 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   const uint32_t tmem = s_tmem_base;
   if (tid == 0) PF_STAMP(0, 31, 2);
 
-  if (warp >= 8) {
-    tc::setmaxnreg_dec_40();
-    if (warp == 8) {
+  if (warp >= kPpSoftWarps) {
+    tc::setmaxnreg_dec_64();
+    if (warp == kPpSoftWarps) {
       // ------------------------------ TMA producer ------------------------------
+      Order order = {1, 1u, -1, 0, 1, 0, 0, 0};
+      if (sorted) {
+        float steps = 0.f;
+        for (int q = lane; q < p.num_seqs; q += 32) {
+          const int n = tiles_of(q);
+          order.top = max(order.top, n > 0 ? s_base[q] + n : 1);
+          steps += static_cast<float>(n) * (static_cast<float>(s_base[q]) + 0.5f * static_cast<float>(n + 1));
+        }
+        order.top = __reduce_max_sync(0xffffffffu, order.top);
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) steps += __shfl_xor_sync(0xffffffffu, steps, o);
+        const float fit = steps * static_cast<float>(ydim) / (2.f * static_cast<float>(gridDim.x) * static_cast<float>(order.top));
+        order.groups = static_cast<unsigned>(max(1, min(p.num_kv_heads, static_cast<int>(fminf(fit, 65536.f)))));
+      }
       if (lane == 0) {
         tc::tma_prefetch_desc(&tmap_q);
         tc::tma_prefetch_desc(&tmap_k);
@@ -736,7 +801,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
           const bool live = u < total_units && !*abort_flag;
           Unit w;
           if (live) {
-            w = get_unit(u);
+            w = get_unit(u, order);
             *reinterpret_cast<int4*>(&s_unit[slot][0]) = make_int4(w.n_kv, w.first_pos, w.seq_start, w.seq_len);
             *reinterpret_cast<int4*>(&s_unit[slot][4]) = make_int4(w.q0, w.head_a, (w.has_b ? 1 : 0) | (w.split_p ? 2 : 0),
                                                                          w.n_kv | (w.has_b ? kUnitHasB : 0) | (w.split_p ? kUnitSplitP : 0));
@@ -802,7 +867,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
           }
         }
       }
-    } else if (warp == 9) {
+    } else if (warp == kPpSoftWarps + 1) {
       // ------------------------------- MMA issuer -------------------------------
       const uint32_t idesc_qk = tc::instr_desc_f16(p.fmt, p.fmt, false, 128, 128);
       const uint32_t idesc_pv = tc::instr_desc_f16(p.fmt, p.fmt, true, 128, 128);
@@ -913,213 +978,195 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
     }
   } else {
     // ------------------------------ softmax warps ------------------------------
-    tc::setmaxnreg_inc_232();
-    const int t = warp >> 2;                       // 0: head A, 1: head B
-    const int row = (warp & 3) * 32 + lane;        // row of the tile = TMEM lane
-    const uint32_t lane_addr = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    // Eight a head, two on each 32 lanes of tensor memory with 16 rows each, in the 16x256b layout: lane i holds columns
+    // 8g + 2 (i & 3) + {0, 1} of rows i / 4 and i / 4 + 8 (a and b below), so that a row's maximum is two shuffles away and
+    // nothing crosses warps.
+    tc::setmaxnreg_inc_104();
+    const int t = warp >> 3;                       // 0: head A, 1: head B
+    const int row0w = (warp & 3) * 32 + ((warp >> 2) & 1) * 16;      // first row of the warp = TMEM lane
+    const int row = row0w + (lane >> 2), colq = 2 * (lane & 3);
+    const uint32_t lane_addr = static_cast<uint32_t>(row0w) << 16;
     const uint32_t s_addr = tmem + lane_addr + t * 128;
     const uint32_t o_addr = tmem + lane_addr + 256 + t * 128;
+    const uint32_t o_stage = o_smem + warp * kPfOutWarpBytes;   // this warp's 16 rows x 128 B
+    auto arrive = [&](int i) {                     // for the warp
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(bar(i));
+    };
     int g = 0;                                     // KV steps of this head so far (barrier phases)
-    const uint32_t o_stage = o_smem + warp * kPfOutWarpBytes;   // this warp's 32 rows x 128 B
     for (int ku = 0;; ++ku) {
       const int slot = ku % kPfUnitRing;
       tc::mbar_wait_compact<false>(bar(PB_UFULL + slot), (ku / kPfUnitRing) & 1, abort_flag, p.error_word, 13);
       const int n_kv = *abort_flag ? 0 : s_unit[slot][0];
       if (n_kv == 0) break;
-      if ((warp & 3) == 0 && lane == 0) PF_STAMP(2 + t, ku, 0);
+      if ((warp & 7) == 0 && lane == 0) PF_STAMP(2 + t, ku, 0);
       const int first_pos = s_unit[slot][1], flags = s_unit[slot][6];
-      const bool split_p = (flags & 2) != 0;
       if (t == 1 && !(flags & 1)) {
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(bar(PB_UEMPTY + slot));
+        arrive(PB_UEMPTY + slot);
         continue;
       }
-      float m_used = -INFINITY, l = 0.f;
-      // Rare: the reference maximum of some row of this warp moved.  PV of the previous step must have landed
-      // in O before O is scaled; the next PV cannot start before this warp arrives at PREADY below.
-      auto rescale_o = [&](float alpha, int gg, float& l_ref) {
-        tc::mbar_wait_compact<false>(bar(PB_ODONE + t), (gg - 1) & 1, abort_flag, p.error_word, 9);
+      float m_a = -INFINITY, m_b = -INFINITY, l_a = 0.f, l_b = 0.f;
+      for (int j = 0; j < n_kv; ++j) {
+        tc::mbar_wait_compact<false>(bar(PB_SFULL + t), g & 1, abort_flag, p.error_word, 8);
+        if ((warp & 7) == 0 && lane == 0 && j == 0) PF_STAMP(2 + t, ku, 2);
+        if ((warp & 7) == 0 && lane == 0) PF_STEP(ku, 1 + t, j, 0);
         tc::fence_after_sync();
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t ov[32];
-          tc::tmem_ld32(o_addr + c * 32, ov);
-          tc::wait_ld();
+        uint32_t sv[2][32];                        // [half][4 group + {a, a, b, b}]
+        tc::tmem_ld16x256_x8(s_addr, sv[0]);
+        tc::tmem_ld16x256_x8(s_addr + 64, sv[1]);
+        tc::wait_ld();
+        // Keys of this tile sit at positions 128j + col, query row r at first_pos + r: a key is visible when
+        // col <= r + shift.  Tiles that end at or before the first row's position need no mask at all.
+        const int shift = first_pos - j * kPfTile;
+        if (shift < kPfTile - 1) {
+          const int vis = row + shift - colq;      // of row a; 8 more for row b
 #pragma unroll
-          for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-          tc::tmem_st32(o_addr + c * 32, ov);
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (h * 64 + (i >> 2) * 8 + (i & 1) > vis + ((i & 2) ? 8 : 0)) sv[h][i] = 0xff800000u;  // -inf
         }
-        tc::wait_st();
-        l_ref *= alpha;
-      };
-        for (int j = 0; j < n_kv; ++j) {
-          tc::mbar_wait_compact<false>(bar(PB_SFULL + t), g & 1, abort_flag, p.error_word, 8);
-          if ((warp & 3) == 0 && lane == 0 && j == 0) PF_STAMP(2 + t, ku, 2);
-          if ((warp & 3) == 0 && lane == 0) PF_STEP(ku, 1 + t, j, 0);
-          tc::fence_after_sync();
-          // Keys of this tile sit at positions 128j + col, query row r at first_pos + r: a key is visible when
-          // col <= r + shift.  Tiles that end at or before the first row's position need no mask at all.
-          const int shift = first_pos - j * kPfTile;
-          const bool diag = shift < kPfTile - 1;
-          const int vis = row + shift;            // last visible column of this thread's row
-          float sum = 0.f;
-          if (!split_p) {
-            // ---- fast path: the whole S row in registers, one wait for four loads ----
-            uint32_t sv[4][32];
-  #pragma unroll
-            for (int c = 0; c < 4; ++c) tc::tmem_ld32(s_addr + c * 32, sv[c]);
-            tc::wait_ld();
-            if (diag) {
-  #pragma unroll
-              for (int c = 0; c < 4; ++c)
-  #pragma unroll
-                for (int i = 0; i < 32; ++i)
-                  if (c * 32 + i > vis) sv[c][i] = 0xff800000u;  // -inf
-            }
-            // Row maximum: three-input max, eight independent chains (one chain of 128 dependent ops costs ~500 cycles).
-            float mxs[8];
-  #pragma unroll
-            for (int i = 0; i < 8; ++i) mxs[i] = -INFINITY;
-  #pragma unroll
-            for (int c = 0; c < 4; ++c)
-  #pragma unroll
-              for (int i = 0; i < 16; ++i)
-                mxs[i & 7] = tc::max3(mxs[i & 7], __uint_as_float(sv[c][2 * i]), __uint_as_float(sv[c][2 * i + 1]));
-            float mx = fmaxf(tc::max3(mxs[0], mxs[1], mxs[2]), tc::max3(mxs[3], mxs[4], mxs[5]));
-            mx = tc::max3(mx, mxs[6], mxs[7]);
-            mx *= p.scale_log2;  // scale > 0, so max commutes with it
-            const bool grow = mx > m_used + kRescaleThreshold;
-            if (j > 0 && __any_sync(0xffffffffu, grow)) rescale_o(grow ? ex2(m_used - mx) : 1.f, g, l);
-            if (grow) m_used = mx;
-            // exp2(s * scale - m) on packed pairs; a share of the pairs goes to the FMA-pipe polynomial so that
-            // the special-function unit (the slowest pipe of the tile) does not see every exponential
-            const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), nm2 = make_float2(-m_used, -m_used);
-            float2 sums[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-  #pragma unroll
-            for (int c2 = 0; c2 < 2; ++c2) {
-              uint32_t pk[32];
-  #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const int c = 2 * c2 + (i >> 4), k = (i & 15) * 2;
-                const float2 x = tc::fma2(make_float2(__uint_as_float(sv[c][k]), __uint_as_float(sv[c][k + 1])), sc2, nm2);
-                float2 e;
-                if (MV_PF_POLY_PRED(i)) {
-                  e = tc::ex2_poly2(x);
-                } else {
-                  e.x = tc::ex2_mufu(x.x);
-                  e.y = tc::ex2_mufu(x.y);
-                }
-                sums[i & 3] = tc::add2(sums[i & 3], e);
-                pk[i] = pack2<T>(e.x, e.y);
-              }
-              tc::tmem_st32(s_addr + c2 * 32, pk);   // P over the first 64 columns of S (all of S is in registers)
-            }
-            const float2 s01 = tc::add2(sums[0], sums[1]), s23 = tc::add2(sums[2], sums[3]);
-            sum = (s01.x + s01.y) + (s23.x + s23.y);
-          } else {
-            // ---- rows with few keys, bf16: two passes over S, P plus its rounding residue ----
-            float mx = -INFINITY;
-  #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              uint32_t sv[32];
-              tc::tmem_ld32(s_addr + c * 32, sv);
-              tc::wait_ld();
-  #pragma unroll
-              for (int i = 0; i < 32; ++i)
-                mx = fmaxf(mx, (diag && c * 32 + i > vis) ? -INFINITY : __uint_as_float(sv[i]));
-            }
-            mx *= p.scale_log2;
-            const bool grow = mx > m_used + kRescaleThreshold;
-            if (j > 0 && __any_sync(0xffffffffu, grow)) rescale_o(grow ? ex2(m_used - mx) : 1.f, g, l);
-            if (grow) m_used = mx;
-            uint32_t plo[32];
-  #pragma unroll
-            for (int c2 = 0; c2 < 2; ++c2) {
-              uint32_t sa[32], sb[32], pk[32];
-              tc::tmem_ld32(s_addr + c2 * 64, sa);
-              tc::tmem_ld32(s_addr + c2 * 64 + 32, sb);
-              tc::wait_ld();
-              // once the second half of S has been read, the residue of the first half can go over columns 64..95
-              if (c2 == 1) tc::tmem_st32(s_addr + 64, plo);
-  #pragma unroll
-              for (int i = 0; i < 32; ++i) {
-                const int k = (i & 15) * 2, col = c2 * 64 + 2 * i;
-                float s0 = __uint_as_float(i < 16 ? sa[k] : sb[k]);
-                float s1 = __uint_as_float(i < 16 ? sa[k + 1] : sb[k + 1]);
-                if (diag && col > vis) s0 = -INFINITY;
-                if (diag && col + 1 > vis) s1 = -INFINITY;
-                const float p0 = ex2(fmaf(s0, p.scale_log2, -m_used));
-                const float p1 = ex2(fmaf(s1, p.scale_log2, -m_used));
-                pk[i] = pack2<T>(p0, p1);
-                const float2 hi = Elem<T>::to_f2(*reinterpret_cast<typename Elem<T>::T2*>(&pk[i]));
-                plo[i] = pack2<T>(p0 - hi.x, p1 - hi.y);
-                sum += p0 + p1;
-              }
-              tc::tmem_st32(s_addr + c2 * 32, pk);
-            }
-            tc::tmem_st32(s_addr + 96, plo);
+        float mxa[2], mxb[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          mxa[h] = mxb[h] = -INFINITY;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            mxa[h] = tc::max3(mxa[h], __uint_as_float(sv[h][4 * i]), __uint_as_float(sv[h][4 * i + 1]));
+            mxb[h] = tc::max3(mxb[h], __uint_as_float(sv[h][4 * i + 2]), __uint_as_float(sv[h][4 * i + 3]));
           }
-          l += sum;
-          tc::wait_st();
-          tc::fence_before_sync();
-          if (!(p.inject == 1 && t == 0 && g == 0 && blockIdx.x == 0)) tc::mbar_arrive(bar(PB_PREADY + t));
-          if ((warp & 3) == 0 && lane == 0 && j == n_kv - 1) PF_STAMP(2 + t, ku, 3);
-          if ((warp & 3) == 0 && lane == 0) PF_STEP(ku, 1 + t, j, 1);
-          ++g;
         }
-
-      // ---- epilogue: O / l -> global.  All of O is read into registers so that the accumulator can be handed
-      // back (OFREE) at once.  The rows then go through this warp's staging buffer, 64 columns at a time, so that
-      // each store instruction writes four whole 128-byte lines instead of 32 bytes of 32 different rows. ----
-      tc::mbar_wait_compact<false>(bar(PB_ODONE + t), (g - 1) & 1, abort_flag, p.error_word, 10);
-      if ((warp & 3) == 0 && lane == 0) PF_STAMP(2 + t, ku, 4);
-      tc::fence_after_sync();
-      uint32_t ov[4][32];
+        float xa = fmaxf(mxa[0], mxa[1]), xb = fmaxf(mxb[0], mxb[1]);
+        xa = fmaxf(xa, __shfl_xor_sync(0xffffffffu, xa, 1));
+        xb = fmaxf(xb, __shfl_xor_sync(0xffffffffu, xb, 1));
+        xa = fmaxf(xa, __shfl_xor_sync(0xffffffffu, xa, 2));
+        xb = fmaxf(xb, __shfl_xor_sync(0xffffffffu, xb, 2));
+        xa *= p.scale_log2;                        // scale > 0, so max commutes with it
+        xb *= p.scale_log2;
+        const bool grow_a = xa > m_a + kRescaleThreshold, grow_b = xb > m_b + kRescaleThreshold;
+        if (j > 0 && __any_sync(0xffffffffu, grow_a || grow_b)) {
+          // Rare: the reference maximum of some row of this warp moved.  PV of the previous step must have landed in O before
+          // O is scaled; the next PV cannot start before this warp arrives at PREADY below.
+          const float fa = grow_a ? ex2(m_a - xa) : 1.f, fb = grow_b ? ex2(m_b - xb) : 1.f;
+          tc::mbar_wait_compact<false>(bar(PB_ODONE + t), (g - 1) & 1, abort_flag, p.error_word, 9);
+          tc::fence_after_sync();
+#pragma unroll 1
+          for (int cc = 0; cc < 4; ++cc) {
+            uint32_t ov[16];
+            tc::tmem_ld16x256_x4(o_addr + cc * 32, ov);
+            tc::wait_ld();
 #pragma unroll
-      for (int c = 0; c < 4; ++c) tc::tmem_ld32(o_addr + c * 32, ov[c]);
+            for (int i = 0; i < 16; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * ((i & 2) ? fb : fa));
+            tc::tmem_st16x256_x4(o_addr + cc * 32, ov);
+          }
+          l_a *= fa;
+          l_b *= fb;
+        }
+        if (grow_a) m_a = xa;
+        if (grow_b) m_b = xb;
+        // exp2(s * scale - m) on packed pairs; one pair in eight goes to the FMA-pipe polynomial so that
+        // the special-function unit does not see every exponential (of 0, 1/16, 1/8, 1/4 and 3/8 the best or within 1 %).  P lies over the first 64 columns of S: each warp's
+        // rows of S are in its registers.  kSplit: rows with few keys, bf16, whose rounding residue goes behind P.
+        const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), na2 = make_float2(-m_a, -m_a), nb2 = make_float2(-m_b, -m_b);
+        float2 sum_a[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, sum_b[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        auto weights = [&](auto split) {
+          constexpr bool kSplit = decltype(split)::value;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t pk[16], lo[kSplit ? 16 : 1];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {         // pair i: group i / 2, row a or b
+              const float2 x = tc::fma2(make_float2(__uint_as_float(sv[h][2 * i]), __uint_as_float(sv[h][2 * i + 1])), sc2, (i & 1) ? nb2 : na2);
+              float2 e;
+              if ((i & 7) == 5 && !kSplit) {
+                e = tc::ex2_poly2(x);
+              } else {
+                e.x = tc::ex2_mufu(x.x);
+                e.y = tc::ex2_mufu(x.y);
+              }
+              float2& acc = (i & 1) ? sum_b[h] : sum_a[h];
+              acc = tc::add2(acc, e);
+              pk[i] = pack2<T>(e.x, e.y);
+              if (kSplit) {
+                const float2 hi = Elem<T>::to_f2(*reinterpret_cast<typename Elem<T>::T2*>(&pk[i]));
+                lo[kSplit ? i : 0] = pack2<T>(e.x - hi.x, e.y - hi.y);
+              }
+            }
+            tc::tmem_st16x128_x8(s_addr + h * 32, pk);
+            if constexpr (kSplit) tc::tmem_st16x128_x8(s_addr + 64 + h * 32, lo);
+          }
+        };
+        if (std::is_same<T, __nv_bfloat16>::value && (flags & 2)) weights(std::integral_constant<bool, std::is_same<T, __nv_bfloat16>::value>{});
+        else weights(std::false_type{});
+        const float2 ta = tc::add2(sum_a[0], sum_a[1]), tb = tc::add2(sum_b[0], sum_b[1]);
+        l_a += ta.x + ta.y;
+        l_b += tb.x + tb.y;
+        tc::wait_st();
+        tc::fence_before_sync();
+        if (!(p.inject == 1 && t == 0 && g == 0 && blockIdx.x == 0 && warp == 0)) arrive(PB_PREADY + t);
+        if ((warp & 7) == 0 && lane == 0 && j == n_kv - 1) PF_STAMP(2 + t, ku, 3);
+        if ((warp & 7) == 0 && lane == 0) PF_STEP(ku, 1 + t, j, 1);
+        ++g;
+      }
+
+      // ---- epilogue: O / l -> global, by TMA from this warp's staging buffer, 64 columns at a time ----
+      l_a += __shfl_xor_sync(0xffffffffu, l_a, 1);
+      l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
+      l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
+      l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
+      const float inv_a = l_a > 0.f ? 1.f / l_a : 0.f, inv_b = l_b > 0.f ? 1.f / l_b : 0.f;
+      const int seq_start = s_unit[slot][2], seq_len = s_unit[slot][3], row0 = s_unit[slot][4] + row0w, head = s_unit[slot][5] + t;
+      arrive(PB_UEMPTY + slot);
+      tc::mbar_wait_compact<false>(bar(PB_ODONE + t), (g - 1) & 1, abort_flag, p.error_word, 10);
+      if ((warp & 7) == 0 && lane == 0) PF_STAMP(2 + t, ku, 4);
+      tc::fence_after_sync();
+      uint32_t ov[2][32];
+      tc::tmem_ld16x256_x8(o_addr, ov[0]);
+      tc::tmem_ld16x256_x8(o_addr + 64, ov[1]);
       tc::wait_ld();
       tc::fence_before_sync();
-      tc::mbar_arrive(bar(PB_OFREE + t));
-      if ((warp & 3) == 0 && lane == 0) PF_STAMP(2 + t, ku, 5);
-      const float inv_l = l > 0.f ? 1.f / l : 0.f;
-      const int2 pl0 = *reinterpret_cast<const int2*>(&s_unit[slot][2]);     // seq_start, seq_len
-      const int2 pl1 = *reinterpret_cast<const int2*>(&s_unit[slot][4]);     // q0, head_a
-      const int4 place = make_int4(pl0.x, pl0.y, pl1.x, pl1.y);
-      const int seq_len = place.y;
-      const int row0 = place.z + (warp & 3) * 32;              // first row of this warp within the sequence
-      T* obase = static_cast<T*>(p.out) + static_cast<int64_t>(place.x + row0) * p.out_stride_tok +
-                 static_cast<int64_t>(place.w + t) * kPfD;
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(bar(PB_UEMPTY + slot));
+      arrive(PB_OFREE + t);                        // the accumulator is read
+      if ((warp & 7) == 0 && lane == 0) PF_STAMP(2 + t, ku, 5);
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-#pragma unroll
-        for (int ch = 0; ch < 8; ++ch) {                       // this lane's row: eight chunks of eight outputs
-          const int c = half * 2 + (ch >> 2), i0 = (ch & 3) * 8;
-          uint4 x;
-          x.x = pack2<T>(__uint_as_float(ov[c][i0 + 0]) * inv_l, __uint_as_float(ov[c][i0 + 1]) * inv_l);
-          x.y = pack2<T>(__uint_as_float(ov[c][i0 + 2]) * inv_l, __uint_as_float(ov[c][i0 + 3]) * inv_l);
-          x.z = pack2<T>(__uint_as_float(ov[c][i0 + 4]) * inv_l, __uint_as_float(ov[c][i0 + 5]) * inv_l);
-          x.w = pack2<T>(__uint_as_float(ov[c][i0 + 6]) * inv_l, __uint_as_float(ov[c][i0 + 7]) * inv_l);
-          st_shared16(o_stage + lane * 128 + ((ch ^ (lane & 7)) << 4), x);   // chunks swizzled by row: no bank conflicts
-        }
+      for (int h = 0; h < 2; ++h) {
+        if (lane == 0) tc::bulk_wait_read();       // the copy before has left the buffer
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {                          // eight lanes per row, four rows per instruction
-          const int r = 4 * i + (lane >> 3), ch = lane & 7;
-          const uint4 x = ld_shared16(o_stage + r * 128 + ((ch ^ (r & 7)) << 4));
-          if (row0 + r < seq_len)
-            st_global16(obase + static_cast<int64_t>(r) * p.out_stride_tok + half * 64 + ch * 8, x);
+        for (int i = 0; i < 4; ++i) {              // two groups of eight columns: rows 0-7 and 8-15 of each
+          uint32_t x[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float f = (e & 1) ? inv_b : inv_a;
+            x[e] = pack2<T>(__uint_as_float(ov[h][8 * i + 2 * e]) * f, __uint_as_float(ov[h][8 * i + 2 * e + 1]) * f);
+          }
+          // lane i gives the address of row i % 16 of the first (i < 16) or the second group; swizzled as the tensor map has it
+          const int r = lane & 15, ch = 2 * i + (lane >> 4);
+          st_matrix4(o_stage + r * 128 + ((ch ^ (r & 7)) << 4), x);
         }
-        __syncwarp();
+        if (row0 + 16 <= seq_len) {
+          tc::fence_async_proxy();
+          __syncwarp();
+          if (lane == 0) tc::tma_store_3d(&tmap_o, o_stage, h * 64, head, seq_start + row0);
+        } else {                                   // the rows behind belong to the next sequence
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {            // eight lanes per row, four rows per instruction
+            const int r = 4 * i + (lane >> 3), ch = lane & 7;
+            const uint4 x = ld_shared16(o_stage + r * 128 + ((ch ^ (r & 7)) << 4));
+            if (row0 + r < seq_len)
+              st_global16(static_cast<T*>(p.out) + static_cast<int64_t>(seq_start + row0 + r) * p.out_stride_tok + static_cast<int64_t>(head) * kPfD + h * 64 + ch * 8, x);
+          }
+          __syncwarp();
+        }
       }
-      if ((warp & 3) == 0 && lane == 0) { PF_STAMP(2 + t, ku, 6); PF_STAMP(2 + t, ku, 7) ; }
+      if ((warp & 7) == 0 && lane == 0) PF_STAMP(2 + t, ku, 6);
     }
+    if (lane == 0) tc::bulk_wait_all();
   }
   // ---- teardown: everyone is done with tensor memory before it is freed ----
   tc::fence_before_sync();
   __syncthreads();
-  if (warp == 8) {
+  if (warp == kPpSoftWarps) {
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem, 512);
   }
@@ -1181,7 +1228,7 @@ constexpr int kPfPersistentMaxSeqs = 320;   // the persistent form keeps num_seq
                                             // memory the tile buffers and the output staging leave
 
 template <typename T>
-static int launch_prefill_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p,
+static int launch_prefill_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p, int64_t total_tokens,
                             int64_t max_tiles, int num_seqs, int ydim, cudaStream_t st) {
   static bool attr_done[64][2] = {};
   int dev = 0;
@@ -1203,12 +1250,15 @@ static int launch_prefill_t(const CUtensorMap& tq, const CUtensorMap& tk, const 
   }
   if (persistent) {
     if (!fits) return fail(MV_ERR_LIMIT, "prefill: the persistent form takes at most %d sequences", kPfPersistentMaxSeqs);
+    CUtensorMap to;
+    const int rc = make_tmap(&to, p.out, total_tokens, p.num_heads, p.out_stride_tok, std::is_same<T, __half>::value ? MV_F16 : MV_BF16, 16);
+    if (rc) return rc;
     const int64_t units = max_tiles * ydim;
     const unsigned grid = static_cast<unsigned>(units < kNumSMs ? units : kNumSMs);   // one CTA per SM
     static std::atomic<unsigned> next_slot{0};
     PrefillParams pp = p;
     pp.sched_slot = static_cast<int>(next_slot.fetch_add(1) % kPfSchedSlots);
-    prefill_persistent_kernel<T><<<grid, kPfThreads, smem, st>>>(tq, tk, tv, pp);
+    prefill_persistent_kernel<T><<<grid, kPpThreads, smem, st>>>(tq, tk, tv, to, pp);
     return check_launch("prefill_persistent_kernel");
   }
   const dim3 grid(static_cast<unsigned>(max_tiles), static_cast<unsigned>(ydim));
@@ -1225,8 +1275,8 @@ static int launch_prefill(const CUtensorMap& tq, const CUtensorMap& tk, const CU
   p.inject = g_prefill_inject.exchange(0);   // one launch only
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int ydim = num_kv_heads * p.pairs;
-  return dtype == MV_F16 ? launch_prefill_t<__half>(tq, tk, tv, p, max_tiles, num_seqs, ydim, st)
-                         : launch_prefill_t<__nv_bfloat16>(tq, tk, tv, p, max_tiles, num_seqs, ydim, st);
+  return dtype == MV_F16 ? launch_prefill_t<__half>(tq, tk, tv, p, total_tokens, max_tiles, num_seqs, ydim, st)
+                         : launch_prefill_t<__nv_bfloat16>(tq, tk, tv, p, total_tokens, max_tiles, num_seqs, ydim, st);
 }
 }  // namespace mv
 

@@ -71,6 +71,18 @@ def test_prefill_more_tiles_than_sms_with_odd_group(dtype):
     _close(_gpu(d, dtype), _oracle(d, dtype), dtype)
 
 
+@pytest.mark.parametrize("heads,kv,lens", [
+    (32, 16, [1500, 0, 700, 129, 17, 16, 15]),           # units sorted by length, one group; rows at the edges of 16
+    (64, 64, [250, 256, 31, 33, 257, 1, 240, 255]),      # several groups of heads
+    (32, 16, [300, 128, 127, 47, 48, 49, 100, 5, 260]),  # one sequence too many to be sorted
+])
+def test_prefill_order_of_units(heads, kv, lens):
+    d = synth.prefill_inputs(seed=62, num_seqs=1, len_lo=sum(lens), len_hi=sum(lens), num_heads=heads, num_kv_heads=kv, head_dim=128)
+    d["cu_seqlens"] = torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    for dtype in (torch.bfloat16, torch.float16):
+        _close(_gpu(d, dtype), _oracle(d, dtype), dtype)
+
+
 def test_prefill_batch_of_many_short_sequences():
     """More sequences than the kernel keeps a tile table for in shared memory, some of them empty."""
     g = torch.Generator().manual_seed(62)

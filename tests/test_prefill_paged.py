@@ -78,6 +78,14 @@ def test_paged_prefill_on_gpu(case, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("cached", [[0, 700, 128, 0, 127, 1], [400, 0, 0, 300, 0, 129]])
+def test_paged_prefill_order_of_units(cached):
+    """Units sorted by their number of keys, cached ones included: more units than SMs, portions of 1 to 600 tokens."""
+    new = [600, 30, 200, 1, 129, 16]
+    test_paged_prefill_on_gpu(dict(seed=6, lens=[c + n for c, n in zip(cached, new)], cached=cached, H=32, KVH=16, D=128, bs=64), torch.bfloat16)
+
+
+@pytest.mark.gpu
 def test_paged_prefill_without_prefix_equals_packed_prefill():
     """No cached tokens at all: the paged kernel path and the packed path must agree bit for bit."""
     from minivllm_b200.layers import attention as A
