@@ -416,6 +416,12 @@ int mv_add_rmsnorm(void* out, const void* x, const void* residual_in,
  */
 int mv_silu_mul(void* out, const void* gate_up, int64_t gate_up_stride,
                 int64_t rows, int inter, int dtype, void* stream);
+/*
+ * out (rows, n) = x (rows, k; row stride in elements) times w (n, k)^T for up to 16 rows, fp16 or bf16, fp32 accumulation; gated: w
+ * (2n, k) = [gate; up] and the result silu(gate) * up.  n a multiple of 8, k of 64.
+ */
+int mv_few_rows(void* out, const void* x, int64_t x_stride, const void* w, int rows, int n, int k, int gated,
+    int dtype, void* stream);
 
 /*
  * Steps between the sublayers of a decoder with an fp32 residual stream x (rows, width), updated in place, and RMS

@@ -67,6 +67,7 @@ SIGNATURES = {
     "mv_add_rmsnorm": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_i64, _c_i64, _c_ptr, _c_f32, _c_i64, _c_int,
                                 _c_int, _c_ptr]),
     "mv_silu_mul": (_c_int, [_c_ptr, _c_ptr, _c_i64, _c_i64, _c_int, _c_int, _c_ptr]),
+    "mv_few_rows": (_c_int, [_c_ptr, _c_ptr, _c_i64, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr]),
     "mv_embed_norm": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_ptr, _c_i64, _c_ptr, _c_ptr, _c_i64, _c_int, _c_int, _c_f32,
         _c_int, _c_ptr]),
     "mv_gated_residual_norm": (_c_int, [_c_ptr, _c_ptr, _c_ptr, _c_i64, _c_ptr, _c_i64, _c_ptr, _c_ptr, _c_ptr,

@@ -16,7 +16,7 @@ LIB = os.path.join(HERE, "libminivllm_b200.so")
 COMMON = ["api.cu", "metadata.cu", "sampling.cu"]
 GROUPS = {
     "qwen3": ["store_kvcache.cu", "paged_decode.cu", "paged_decode_int8.cu", "prefill_varlen.cu",
-              "paged_decode_static.cu", "pre_attention.cu", "comm.cu"],
+              "paged_decode_static.cu", "pre_attention.cu", "comm.cu", "few_rows.cu"],
     "sipazen": ["norms.cu", "latent_attention.cu", "latent_decode.cu", "latent_prefill.cu", "short_conv.cu", "mamba2.cu",
                 "mamba2_chunk.cu", "moe.cu", "grouped_gemm.cu"],
     "fozerax": ["norms.cu", "window_attention.cu", "latent_prefill.cu", "short_conv.cu", "gla.cu", "gla_chunk.cu", "gated_delta.cu",

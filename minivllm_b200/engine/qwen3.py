@@ -25,10 +25,10 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..layers.activation import silu_and_mul
 from ..layers.allreduce import shard_rows
 from ..layers.attention import Attention, qk_norm_rope_store
 from ..layers.layernorm import add_rms_norm
+from ..layers.linear import linear, swiglu_linear
 from ..utils.context import get_context
 
 RMS_EPS = 1e-5
@@ -181,12 +181,12 @@ class DecoderLayer(nn.Module):
         rank's row shard when `comm` is set, all rows otherwise), `next_gamma` = weight of the norm that follows
         this layer (next layer's input norm, or the final norm).  Returns the next layer's normalised input."""
         rows = h.shape[0]
-        o = self._attention(F.linear(h, self.qkv_w), cos, sin, rope)
-        partial = torch.mm(o, self.o_w.t(), out=comm.input_rows(rows)) if comm is not None else F.linear(o, self.o_w)
+        o = self._attention(linear(h, self.qkv_w), cos, sin, rope)
+        partial = torch.mm(o, self.o_w.t(), out=comm.input_rows(rows)) if comm is not None else linear(o, self.o_w)
         h = self._reduce_add_norm(partial, residual, self.post_norm_w, comm)
-        act = silu_and_mul(F.linear(h, self.gate_up_w))
+        act = swiglu_linear(h, self.gate_up_w)
         partial = torch.mm(act, self.down_w.t(), out=comm.input_rows(rows)) if comm is not None else \
-            F.linear(act, self.down_w)
+            linear(act, self.down_w)
         return self._reduce_add_norm(partial, residual, next_gamma, comm)
 
 
@@ -251,4 +251,4 @@ class Qwen3ForCausalLM(nn.Module):
             rank, size = vocab_shard
             per = w.shape[0] // size
             w = w[rank * per:(rank + 1) * per]
-        return F.linear(hidden, w)
+        return linear(hidden, w)

@@ -7,6 +7,41 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from .. import _cabi
+from .activation import silu_and_mul
+
+FEW_ROWS = 16
+
+
+def _few_rows(x, weight, gated):
+    """The product of a decode step's rows, or None where it is the library's: more rows, other types, sizes or layouts, or a
+    weight so large that the library's is faster (csrc/few_rows.cu)."""
+    n, k = weight.shape
+    rows = x.shape[0]
+    if not (x.is_cuda and x.dim() == 2 and 0 < rows <= FEW_ROWS and x.dtype == weight.dtype and x.shape[1] == k and
+            x.dtype in (torch.bfloat16, torch.float16)) or k % 64 or n % (16 if gated else 8) or \
+            (n * k > 8 << 20 and n > 4096) or x.stride(1) != 1 or not weight.is_contiguous() or x.device != weight.device or \
+            x.data_ptr() % 16 or weight.data_ptr() % 16 or (rows > 1 and (x.stride(0) % 8 or x.stride(0) < k)) or \
+            (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)):
+        return None
+    n = n // 2 if gated else n
+    out = torch.empty((rows, n), dtype=x.dtype, device=x.device)
+    _cabi.check(_cabi.lib().mv_few_rows(out.data_ptr(), x.data_ptr(), x.stride(0) if rows > 1 else k, weight.data_ptr(), rows, n, k,
+                                        int(gated), _cabi.dtype_code(x.dtype), _cabi.stream_ptr()))
+    return out
+
+
+def linear(x, weight):
+    """x (rows, in) times weight (out, in)^T."""
+    y = _few_rows(x, weight, False)
+    return F.linear(x, weight) if y is None else y
+
+
+def swiglu_linear(x, weight):
+    """silu_and_mul(linear(x, weight)), weight (2 * out, in) = [gate; up]."""
+    y = _few_rows(x, weight, True)
+    return silu_and_mul(F.linear(x, weight)) if y is None else y
+
 
 class StackedLinear(nn.Module):
     """parts: {name: (out, in) weight}, biases: {name: (out,)} for some of them.  Calling it with (rows, in) returns
