@@ -36,7 +36,7 @@ def _cfg(config, *names, default=None):
     return default
 
 
-SCORE_PIECE = 1 << 19       # logits that cross to the host at a time
+SCORE_PIECE = (1 << 18) - 4096      # logits that cross to the host at a time: two pieces of 16 bits and the rest in 1 MiB
 
 
 class ModelRunner:
@@ -123,6 +123,8 @@ class ModelRunner:
         self.allocate_kv_cache()
         if not self.enforce_eager:
             self.capture_cudagraph()
+        if self.keep_logits and self.device.type == "cuda":
+            self._score_buffers()                       # not in the first step: pinning takes 2 ms
 
     # ------------------------------------------------------------------ memory ---
     def kv_block_bytes(self):
@@ -446,9 +448,12 @@ class ModelRunner:
     def _score_buffers(self):
         """Pinned rows of step_logits, kept with the runner: a step has read them when it returns."""
         if self._score is None:
-            pinned = lambda *shape, dtype: torch.empty(shape, dtype=dtype).pin_memory()
-            self._score = {"given": pinned(2, self.max_num_seqs, dtype=torch.int64), "error": pinned(1, dtype=torch.int32),
-                           "logits": [pinned(SCORE_PIECE, dtype=self.dtype) for _ in range(2)],
+            item, n = torch.empty((), dtype=self.dtype).element_size(), self.max_num_seqs
+            at = (16 * n + 8 + 63) // 64 * 64
+            raw = torch.empty(at + 2 * SCORE_PIECE * item, dtype=torch.uint8).pin_memory()      # one block: pinning is dear
+            part = lambda a, count, dtype: raw[a:a + count * torch.empty((), dtype=dtype).element_size()].view(dtype)
+            self._score = {"given": part(0, 2 * n, torch.int64).view(2, n), "error": part(16 * n, 1, torch.int32),
+                           "logits": [part(at + i * SCORE_PIECE * item, SCORE_PIECE, self.dtype) for i in range(2)],
                            "done": [torch.cuda.Event() for _ in range(2)]}
         return self._score
 
