@@ -115,3 +115,28 @@ def test_fused_norm_rope_store_into_an_int8_cache(dtype):
     q2, k2 = A.qk_norm_rope_store(qkv.to(dev), pos.to(dev), cos, sin, gam.to(dev), gam.to(dev), 1e-5, H, KVH, D, kc, vc,
                                   slots.to(dev))
     assert torch.equal(q, q2) and torch.equal(k, k2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("heads,kv,tokens", [(32, 8, 6827), (7, 3, 25207), (64, 1, 4965)])
+@pytest.mark.parametrize("int8", [False, True])
+def test_many_tokens_equal_few_at_a_time(heads, kv, tokens, int8):
+    """From 320 Ki rows on a warp has a token's rows; portions of the same tokens take the other form: the same bits."""
+    from minivllm_b200.layers.attention import qk_norm_rope_store
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    D, block, blocks = 128, 64, tokens // 64 + 2
+    qkv, pos = rnd(tokens, (heads + 2 * kv) * D + 64)[:, :(heads + 2 * kv) * D], torch.randint(-2, 600, (tokens,), generator=g, device="cuda")
+    slots = torch.randperm(blocks * block, generator=g, device="cuda")[:tokens].contiguous()
+    slots[::97] = -1
+    angle = torch.arange(512, device="cuda").float()[:, None] * 1e4 ** (-torch.arange(0, D, 2, device="cuda").float() / D)
+    cos, sin, gq, gk = angle.cos(), angle.sin(), rnd(D), rnd(D)
+
+    def run(parts):
+        cache = [torch.zeros(blocks, block, kv, D, dtype=torch.int8 if int8 else torch.bfloat16, device="cuda") for _ in range(2)]
+        sc = {n: torch.zeros(blocks, block, kv, dtype=torch.float16, device="cuda") for n in ("k_scale", "v_scale")} if int8 else {}
+        out = [qk_norm_rope_store(qkv[a:b], pos[a:b], cos, sin, gq, gk, 1e-6, heads, kv, D, *cache, slots[a:b], **sc) for a, b in parts]
+        return [torch.cat(x) for x in zip(*out)] + cache + list(sc.values())
+    step = tokens // 5 + 1
+    for got, want in zip(run([(0, tokens)]), run([(a, min(tokens, a + step)) for a in range(0, tokens, step)])):
+        assert torch.equal(got, want)
