@@ -663,7 +663,8 @@ int mv_delta_scan(void* out, int64_t out_stride, const void* qkv, int64_t stride
 /*
  * The same recurrences for packed portions in chunks of 64 tokens on tensor cores, bf16: dim a multiple of 8 up to 128,
  * vdim a multiple of 8, rows on 16-byte boundaries.  tokens = cu[num_seqs]; workspace_bytes is -1 when the sizes are not
- * taken.  error_word: an int on the device that a bounded wait sets when it runs out, as in mv_prefill_varlen (version 6).
+ * taken.  error_word: an int on the device that a bounded wait sets when it runs out, as in mv_prefill_varlen (version 6);
+ * the states that the call would have advanced are then not written, nor is anything while the word is not zero.
  */
 int64_t mv_gla_chunk_workspace_bytes(int64_t tokens, int num_seqs, int heads, int dim, int vdim);
 int mv_gla_chunk_scan(void* out, int64_t out_stride, const void* q, const void* k, const void* v,

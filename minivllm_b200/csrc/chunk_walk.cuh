@@ -13,6 +13,13 @@
 // come by TMA; a sequence's ragged last chunk is copied by warps 12-15 with zeros past its end, and so are all chunks of rows
 // that are not made of whole slabs.
 //
+// A wait that runs out (or an error word that is set already) ends the CTA.  The warps that issue copies and products and those of
+// the state leave their loops before they do anything more; the others go through the rest of theirs, which then changes shared
+// memory and rows of a result that nobody may use.  (The warps that read O share a barrier; to agree there on leaving cost mLSTM
+// 1.4 %.)  Nobody arrives at a barrier behind a wait that failed: who saw one fail has also seen s_abort.  (With such arrivals a
+// launch failed, most likely where a warp's 32 met a barrier of 128 + 1, WB_EMPTY, that lacked one.)  Copies and products in flight
+// are waited for, and no state is written.
+//
 // The roles' loops are rolled: unrolled, five of them pushed one another out of the instruction cache (a fourth of the stalls),
 // and a chunk of mLSTM took 4.1 us instead of 3.6.
 // Bound: gla and time mixing read 98 KB a chunk, two column blocks of a head the same 82 KB of it, at about 6 TB/s over all SMs
@@ -27,6 +34,7 @@
 // sequences are cut into segments: a pass over each segment from a zero state (kState: no O), a join that turns the segments'
 // own states into the states in front of them, and the full pass over all segments at once.
 #pragma once
+#include <atomic>
 #include "state_chunk.cuh"
 #include "tcgen05.cuh"
 #include "tmap.cuh"
@@ -41,6 +49,8 @@ constexpr int kWalkV = 2 * kSlab;
 __host__ __device__ constexpr int tile_at(int row, int col) {
   return (col >> 6) * kSlab + row * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4) + (col & 7) * 2;
 }
+
+extern std::atomic<int> g_walk_inject;                    // api.cu; the next launch's WalkParams::inject
 
 // Scratch of a chunk and head.  kMem: [A hi, A lo, vectors]; else [Q hi, Q lo, K hi, K lo, A hi, A lo, decays].
 template <int K, bool kMem> struct WalkBlob {
@@ -71,6 +81,8 @@ struct WalkParams {
   float *seg_state, *seg_n, *seg_decay;                   // per segment and head: K x V, K (kMem), K
   int* error_word;
   bool tma;                                               // whole chunks by TMA
+  int inject;                                             // test hook, normally 0.  1: the first CTA's first state warp withholds its
+                                                          // second arrival, so that the product warp's bounded wait runs out
 };
 
 // Segment x of the batch: its sequence and its place in it.  Whole warp; false past the last.
@@ -156,7 +168,7 @@ __device__ __forceinline__ void mma_ts_4(uint32_t d_tmem, uint32_t a_tmem, uint6
 }
 }  // namespace tc
 
-enum WalkBar { WB_BLOB = 0, WB_FULL = 2, WB_EMPTY = 4, WB_SREADY = 6, WB_SDONE, WB_ODONE, WB_OFREE, WB_COUNT };
+enum WalkBar { WB_BLOB = 0, WB_FULL = 2, WB_EMPTY = 4, WB_SREADY = 6, WB_SDONE, WB_ODONE, WB_OFREE, WB_DRAIN, WB_COUNT };
 
 template <int K, bool kMem, bool kState>
 __global__ void __launch_bounds__(kWalkThreads, 1)
@@ -168,7 +180,9 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
   __shared__ uint64_t s_bar[WB_COUNT];
   __shared__ uint32_t s_tmem;
   __shared__ volatile int s_abort;
+  __shared__ int s_sticky;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int error = tid == 0 ? *reinterpret_cast<volatile int*>(p.error_word) : 0;
   // what this CTA walks
   int s, seg = 0, unit = blockIdx.x, h = blockIdx.y, block = blockIdx.z;
   if (!p.seg_chunks && p.num_seqs <= 32 && gridDim.x * gridDim.y * gridDim.z > kNumSMs) {      // longest sequences first
@@ -207,8 +221,10 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
     tc::mbar_init(bar(WB_SDONE), 1);
     tc::mbar_init(bar(WB_ODONE), 1);
     tc::mbar_init(bar(WB_OFREE), 128);
+    tc::mbar_init(bar(WB_DRAIN), 1);
     tc::mbar_fence_init();
     s_abort = 0;
+    s_sticky = error;                                      // read once so that the whole CTA agrees
   }
   if (warp == 16) {
     tc::tmem_alloc(smem_u32(&s_tmem), 512);
@@ -220,11 +236,15 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
   const uint32_t tmem = s_tmem;
   // columns: S, two buffers of [hi | lo], then O (kMem: its two products)
   const uint32_t tS = tmem, tHL = tmem + 128, tO = tmem + 384;
-  auto wait = [&](int b, int parity, int where) { tc::mbar_wait(bar(b), parity, &s_abort, p.error_word, where); };
+  auto wait = [&](int b, int parity, int where) { return tc::mbar_wait(bar(b), parity, &s_abort, p.error_word, where); };
+  auto all = [](bool ok) { return __all_sync(0xffffffffu, ok) != 0; };
+  auto aborted = [&] { return __any_sync(0xffffffffu, s_abort) != 0; };
   auto stage_at = [&](int i) { return (i & 1) * St::kBytes; };
   auto whole = [&](int i) { return p.tma && n_tok - i * kChunk >= kChunk; };    // chunk i comes by TMA
 
-  if (warp < 8) {
+  if (s_sticky != 0) {
+    // a wait ran out in a launch before: straight to the end, as prefill does
+  } else if (warp < 8) {
     // ---------------------------------------------------------------- the state
     const int row = (warp & 3) * 32 + lane, ch0 = (warp >> 2) * (K / 2);
     const bool on = row < pw;
@@ -245,11 +265,10 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
     }
     for (int i = 0; i < chunks; ++i) {
       const unsigned char* st = smem + stage_at(i);
-      if (i > 0) {
-        wait(WB_SDONE, (i - 1) & 1, 1);
-        tc::fence_after_sync();
-      }
-      wait(WB_BLOB + (i & 1), (i >> 1) & 1, 2);
+      bool ok = i == 0 || wait(WB_SDONE, (i - 1) & 1, 1);
+      ok = all(wait(WB_BLOB + (i & 1), (i >> 1) & 1, 2) && ok);
+      if (!ok) break;
+      tc::fence_after_sync();
       const float* vec = reinterpret_cast<const float*>(st + B::kVec);
       const uint32_t hl = tHL + (i & 1) * 128 + lanes + ch0 / 2;
 #pragma unroll 1
@@ -281,11 +300,11 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
       }
       tc::wait_st();
       tc::fence_before_sync();
-      tc::mbar_arrive(bar(WB_SREADY));
+      if (!(p.inject == 1 && i == 1 && warp == 0 && blockIdx.x + blockIdx.y + blockIdx.z == 0)) tc::mbar_arrive(bar(WB_SREADY));
     }
     wait(WB_SDONE, (chunks - 1) & 1, 3);
     tc::fence_after_sync();
-    const bool keep = on && (kState || (last_seg && live));
+    const bool keep = !aborted() && on && (kState || (last_seg && live));
     float* dst = (kState ? p.seg_state + seg_pair * p.K * p.V : p.state + pair * p.K * p.V) + p0 + row;
 #pragma unroll 1
     for (int c = 0; c < K / 2; c += 16) {
@@ -353,10 +372,11 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
         }
       }
       if constexpr (kState) {
-        tc::mbar_arrive(bar(WB_EMPTY + (i & 1)));
+        if (!s_abort) tc::mbar_arrive(bar(WB_EMPTY + (i & 1)));
         continue;
       }
       wait(WB_ODONE, i & 1, 4);
+      __syncwarp();
       tc::fence_after_sync();
       asm volatile("bar.sync 1, 128;" ::: "memory");       // the rows of the chunk before are stored
 #pragma unroll 1
@@ -381,8 +401,10 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
         for (int e = 0; e < 16; ++e) rows[(c + e) * kWalkCols + row] = __float2bfloat16_rn(__uint_as_float(o[e]));
       }
       tc::fence_before_sync();
-      tc::mbar_arrive(bar(WB_EMPTY + (i & 1)));            // the stage's vectors and Q are read
-      tc::mbar_arrive(bar(WB_OFREE));
+      if (!s_abort) {
+        tc::mbar_arrive(bar(WB_EMPTY + (i & 1)));          // the stage's vectors and Q are read
+        tc::mbar_arrive(bar(WB_OFREE));
+      }
       asm volatile("bar.sync 1, 128;" ::: "memory");
       __nv_bfloat16* dst = p.out + (static_cast<int64_t>(first) + i * kChunk) * p.out_stride + static_cast<int64_t>(h) * p.V + p0;
 #pragma unroll 2
@@ -392,9 +414,10 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
           *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(r) * p.out_stride + c) = *reinterpret_cast<const uint4*>(rows + r * kWalkCols + c);
       }
     }
-    if (kState && first_block && t < p.K) p.seg_decay[seg_pair * p.K + t] = prod;
+    const bool ok = !aborted();
+    if (kState && ok && first_block && t < p.K) p.seg_decay[seg_pair * p.K + t] = prod;
     if constexpr (kMem) {
-      if (keeps_n && lw == 0 && (kState || (last_seg && live))) {
+      if (ok && keeps_n && lw == 0 && (kState || (last_seg && live))) {
         float* dst = kState ? p.seg_n + seg_pair * p.K : p.n_state + pair * p.K;
 #pragma unroll
         for (int e = 0; e < kPer; ++e)
@@ -455,16 +478,17 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
         }
       }
       tc::fence_async_proxy();
-      tc::mbar_arrive(bar(WB_FULL + (i & 1)));
+      if (!s_abort) tc::mbar_arrive(bar(WB_FULL + (i & 1)));
     }
     cp_async_wait<0>();
   } else if (warp == 17) {
     // ---------------------------------------------------------------- loads
     if (lane == 0) {
-      for (int i = 0; i < chunks; ++i) {
+      int i = 0;
+      for (; i < chunks; ++i) {
         const uint32_t st = base + stage_at(i), b = bar(WB_BLOB + (i & 1));
         const bool rows = whole(i);
-        if (i >= 2) wait(WB_EMPTY + (i & 1), ((i >> 1) - 1) & 1, 13);
+        if (i >= 2 && !wait(WB_EMPTY + (i & 1), ((i >> 1) - 1) & 1, 13)) break;
         const unsigned char* src = p.scratch + (static_cast<int64_t>(chunk0 + i) * p.heads + h) * B::kBytes;
         constexpr uint32_t kBlob = kState ? (kMem ? 0 : 2 * B::kT) + B::kFloats * 4 : static_cast<uint32_t>(B::kBytes);
         constexpr uint32_t kRows = kWalkV + (kMem ? (kState ? 1 : 2) * B::kT : 0);
@@ -488,8 +512,9 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
           }
         }
       }
-      if (s_abort)                                         // a copy may still be on its way
-        for (int i = max(0, chunks - 2); i < chunks; ++i) tc::mbar_wait_timed(bar(WB_BLOB + (i & 1)), (i >> 1) & 1);
+      // Nobody may be left to wait for the copies of the last two chunks asked for (an empty stage says that those before have
+      // landed): they must not find the CTA gone.
+      for (int j = max(0, i - 2); j < i; ++j) tc::mbar_wait_timed(bar(WB_BLOB + (j & 1)), (j >> 1) & 1);
     }
     __syncwarp();
   } else {
@@ -501,10 +526,7 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
     auto km = [&](uint32_t at) { return tc::desc64(tc::desc_lo(at, 16), tc::kDescHiSw128Sbo1024); };
     for (int i = 0; i < chunks; ++i) {
       const uint32_t st = base + stage_at(i);
-      wait(WB_BLOB + (i & 1), (i >> 1) & 1, 8);
-      wait(WB_FULL + (i & 1), (i >> 1) & 1, 9);
-      wait(WB_SREADY, i & 1, 10);
-      __syncwarp();
+      if (!all(wait(WB_BLOB + (i & 1), (i >> 1) & 1, 8) && wait(WB_FULL + (i & 1), (i >> 1) & 1, 9) && wait(WB_SREADY, i & 1, 10))) break;
       tc::fence_after_sync();
       if constexpr (kMem) {
         tc::mma_ss_4<128, 128>(tS, mn(st + St::kW), mn(st + St::kK), kUpdate, true);
@@ -517,8 +539,7 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
         tc::commit_elected(bar(WB_SDONE), bar(WB_EMPTY + (i & 1)), true);
       } else {
         tc::commit_elected(bar(WB_SDONE), 0, false);
-        if (i > 0) wait(WB_OFREE, (i - 1) & 1, 11);
-        __syncwarp();
+        if (i > 0 && !all(wait(WB_OFREE, (i - 1) & 1, 11))) break;
         tc::fence_after_sync();
         const uint32_t hi = tHL + (i & 1) * 128, lo = hi + 64, q = kMem ? st + St::kQ : st + B::kQ;
 #pragma unroll
@@ -532,6 +553,11 @@ chunk_walk_kernel(const WalkParams p, const __grid_constant__ CUtensorMap map_q,
         tc::mma_ss_4<128, 2>(o2, mn(st + St::kV), km(st + B::kA + kSlab), kLocal, true);
         tc::commit_elected(bar(WB_ODONE), bar(WB_EMPTY + (i & 1)), true);
       }
+    }
+    __syncwarp();
+    if (aborted()) {                                       // nobody may have waited for the last products: they must have run
+      tc::commit_elected(bar(WB_DRAIN), 0, false);         // before tensor memory is freed
+      tc::mbar_wait_timed(bar(WB_DRAIN), 0);
     }
   }
   tc::fence_before_sync();
@@ -598,6 +624,7 @@ inline int64_t walk_segment_floats(int64_t tokens, int num_seqs, int heads, int 
 // scratch holds the chunks' blobs, `segments` (16-byte aligned) walk_segment_floats.
 template <int K, bool kMem>
 int run_walk(const char* what, WalkParams p, int64_t tokens, float* segments, cudaStream_t st) {
+  p.inject = g_walk_inject.exchange(0);                    // one call only
   p.seg_chunks = walk_segment(tokens, p.num_seqs, p.heads, p.V);
   const int64_t units = p.seg_chunks ? walk_segments(tokens, p.num_seqs, p.seg_chunks) : p.num_seqs;
   p.seg_state = segments;

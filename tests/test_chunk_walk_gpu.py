@@ -74,3 +74,48 @@ def test_segments(kind, H, K, V, first, second):
             assert _rel(S[s].cpu().double() * shift[:, None, None], want[0]) < 1e-4 and _rel(nv[s].cpu().double() * shift[:, None], want[1]) < 1e-4
         else:
             assert _rel(S[s], ref[s][1]) < 2e-4, s
+
+
+@pytest.mark.parametrize("kind", ["gla", "mlstm"])
+@pytest.mark.parametrize("lens", [[300, 200], [1024]], ids=["whole", "segments"])
+def test_a_wait_that_runs_out_ends_the_walk(kind, lens):
+    """One arrival is withheld for one call: the wait for it ends after 200 ms, the error word says so, the recurrence it befell
+    keeps the state it had (in segments, where every state depends on the first pass, all of them do), and the next call is
+    clean."""
+    import ctypes
+    from minivllm_b200 import _cabi
+    from minivllm_b200.layers import attention, gla, mlstm
+    H, K, V, n, T = 2, 128, 128, len(lens), sum(lens)
+    word = attention._error_word(torch.device("cuda", torch.cuda.current_device()))
+    q, k, v = (_rnd(i, T, H * D).to(BF).cuda() for i, D in enumerate((K, K, V)))
+    p = torch.cat([q, k, v], 1)
+    q, k, v = p.split([H * K, H * K, H * V], 1)
+    cu, slots, starts = _i32([0] + torch.tensor(lens).cumsum(0).tolist()), _i32(list(range(n))), _i32([0] * n)
+    gates = _rnd(9, T, 2 * H).cuda() if kind == "mlstm" else _rnd(9, T, H * K, mean=3.0).to(BF).cuda()
+
+    def run():
+        S, nv, m = (torch.full((n, H) + x, 7.0, device="cuda") for x in ((K, V), (K,), ()))
+        if kind == "gla":
+            return S, nv, gla.gla_scan(q, k, v, gates, 4.0, cu, slots, starts, S, H, K, V, chunked=True)
+        zero = torch.zeros(H, dtype=BF, device="cuda")
+        chain = mlstm.mlstm_gates(gates, zero, zero + 3, 9.0, cu, slots, starts, m, H)
+        return S, nv, *mlstm.mlstm_scan(q, k, v, chain, cu, slots, starts, S, nv, H, K, V, chunked=True)
+
+    want = run()
+    assert int(word.item()) == 0
+    assert _cabi.lib().mv_debug_walk_inject(ctypes.c_int(1)) == 0
+    S, nv, *_ = run()
+    code = int(word.item())
+    word.zero_()
+    assert code >> 8 == 1, f"error word {code:#x}"
+    hit = torch.zeros(n, H, dtype=torch.bool)
+    hit[0, 0] = True
+    if len(lens) == 1:
+        hit[:] = True
+    for s in range(n):
+        for h in range(H):
+            for got, ref in ((S, want[0]), (nv, want[1])):
+                assert torch.equal(got[s, h], torch.full_like(got[s, h], 7.0) if hit[s, h] else ref[s, h]), (s, h)
+    for got, ref in zip(run(), want):
+        assert torch.equal(got, ref)
+    assert int(word.item()) == 0
