@@ -131,6 +131,14 @@ constexpr int kPfSchedSlots = 1024;  // launches that can be in flight with a wo
 // Work counters of the persistent launches: [slot][0] = units handed out beyond the first one per CTA,
 // [slot][1] = CTAs that have finished.  Zero between launches: the last CTA of a launch clears its slot.
 static __device__ unsigned int g_pf_sched[kPfSchedSlots][2];
+// Who takes which: one sequence for the table, whatever the instantiation.
+static std::atomic<unsigned> g_pf_next{0};
+static std::atomic<int> g_pf_last{-1};      // the slot of the last launch, for tests
+static int pf_take_slot() {
+  const int slot = static_cast<int>(g_pf_next.fetch_add(1) % kPfSchedSlots);
+  g_pf_last.store(slot);
+  return slot;
+}
 
 template <typename T, bool kWin>
 __global__ void __launch_bounds__(kPpThreads, 1)
@@ -844,7 +852,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
 constexpr int kPfPersistentMaxSeqs = 320;   // the persistent form keeps num_seqs + 1 prefix sums in what shared
                                             // memory the tile buffers and the output staging leave
 
-// Units' work counters are handed out in turn (g_pf_sched); tmap_o's box is PfOut<kWin>::kRows rows.
+// tmap_o's box is PfOut<kWin>::kRows rows.
 template <typename T, bool kWin>
 int launch_prefill_persistent(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, PrefillParams p,
                               int64_t max_tiles, int ydim, const char* what, cudaStream_t st) {
@@ -864,8 +872,7 @@ int launch_prefill_persistent(const CUtensorMap& tq, const CUtensorMap& tk, cons
     if (dev >= 0 && dev < 64) attr_done[dev] = true;
   }
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(max_tiles * ydim, kNumSMs));   // one CTA per SM
-  static std::atomic<unsigned> next_slot{0};
-  p.sched_slot = static_cast<int>(next_slot.fetch_add(1) % kPfSchedSlots);
+  p.sched_slot = pf_take_slot();
   prefill_persistent_kernel<T, kWin><<<grid, kPpThreads, smem, st>>>(tq, tk, tv, to, p);
   return check_launch(what);
 }

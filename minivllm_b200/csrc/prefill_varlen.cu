@@ -549,6 +549,9 @@ extern "C" int mv_debug_prefill_form(int form) {
   return MV_OK;
 }
 
+// Test hook: the work counter of the last persistent launch of this process, -1 before the first.
+extern "C" int mv_debug_prefill_slot(void) { return mv::g_pf_last.load(); }
+
 // Test hook: the NEXT prefill launch of this process runs with the given fault injected on the host side of
 // the launch (see PrefillParams::inject).  Nothing faults or hangs: a bounded wait runs out, the error word is
 // set and the kernel returns.

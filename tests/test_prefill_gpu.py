@@ -192,6 +192,18 @@ def test_prefill_wait_that_runs_out_is_reported():
     _close(out.float().cpu(), _oracle(d, dtype), dtype)
 
 
+def test_prefill_launches_of_any_type_take_work_counters_of_their_own():
+    """Launches that may be in flight together, on two streams say, must not share a counter: fp16 and bf16 ones take theirs from
+    one table."""
+    d = synth.prefill_inputs(seed=66, num_seqs=2, len_lo=10, len_hi=200, num_heads=4, num_kv_heads=2, head_dim=128)
+    slots = []
+    for dtype in (torch.float16, torch.bfloat16, torch.bfloat16, torch.float16, torch.float16, torch.bfloat16):
+        out, word = torch.zeros(tuple(d["q"].shape), dtype=dtype, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        assert _call_c_abi(d, dtype, out, word) == 0
+        slots.append(_cabi.lib().mv_debug_prefill_slot())
+    assert len(set(slots)) == len(slots), slots
+
+
 def test_prefill_benchmark_configuration_exactly():
     """The prefill configuration of the benchmark plan, as `bench.py` times it: 32 sequences, lengths uniform in
     [128, 2048] (34,277 tokens with this seed), 32 query / 8 KV heads, head_dim 128, bf16 -- every sequence, every
