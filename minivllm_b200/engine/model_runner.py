@@ -36,7 +36,8 @@ def _cfg(config, *names, default=None):
     return default
 
 
-SCORE_PIECE = (1 << 18) - 4096      # logits that cross to the host at a time: two pieces of 16 bits and the rest in 1 MiB
+SCORE_PIECE = (1 << 18) - 4096      # logits of the model's type that cross to the host at a time: two pieces of 16 bits and the
+                                    # rest in 1 MiB
 
 
 class ModelRunner:
@@ -453,28 +454,30 @@ class ModelRunner:
             raw = torch.empty(at + 2 * SCORE_PIECE * item, dtype=torch.uint8).pin_memory()      # one block: pinning is dear
             part = lambda a, count, dtype: raw[a:a + count * torch.empty((), dtype=dtype).element_size()].view(dtype)
             self._score = {"given": part(0, 2 * n, torch.int64).view(2, n), "error": part(16 * n, 1, torch.int32),
-                           "logits": [part(at + i * SCORE_PIECE * item, SCORE_PIECE, self.dtype) for i in range(2)],
+                           "logits": [part(at + i * SCORE_PIECE * item, SCORE_PIECE * item, torch.uint8) for i in range(2)],
                            "done": [torch.cuda.Event() for _ in range(2)]}
         return self._score
 
     def _logits_to_host(self, logits):
-        """fp32 on the CPU, and the error word behind them in the pinned buffer.  The values cross in their own type, a piece at a
-        time through two pinned buffers, and the host's threads widen one piece beside the next one's copy.  The result's
-        pages are new ones: touching them from one thread, as a copy to unpinned memory does, took longer (0.7 ms for 16 rows
-        of 32,768) than the decode step that made the logits."""
+        """fp32 on the CPU, and the error word behind them in the pinned buffer.  The values cross in their own type, which need not
+        be the model's, a piece at a time through two pinned buffers, and the host's threads widen one piece beside the next one's
+        copy.  The result's pages are new ones: touching them from one thread, as a copy to unpinned memory does, took longer
+        (0.7 ms for 16 rows of 32,768) than the decode step that made the logits."""
         b = self._score_buffers()
         out = torch.empty(logits.shape, dtype=torch.float32)
         src, dst, waiting = logits.reshape(-1), out.view(-1), None
+        pieces = [raw.view(logits.dtype) for raw in b["logits"]]
+        step = pieces[0].numel()
 
         def widen(at, piece, done):
             done.synchronize()
             dst[at:at + piece.numel()].copy_(piece)
 
-        for i, at in enumerate(range(0, src.numel(), SCORE_PIECE)):
-            part = src[at:at + SCORE_PIECE]
-            piece, done = b["logits"][i % 2][:part.numel()], b["done"][i % 2]
+        for i, at in enumerate(range(0, src.numel(), step)):
+            part = src[at:at + step]
+            piece, done = pieces[i % 2][:part.numel()], b["done"][i % 2]
             piece.copy_(part, non_blocking=True)
-            if at + SCORE_PIECE >= src.numel():
+            if at + step >= src.numel():
                 b["error"].copy_(self.error_word, non_blocking=True)
             done.record()
             if waiting is not None:

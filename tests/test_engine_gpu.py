@@ -241,3 +241,17 @@ def test_logits_cross_to_the_host_whole():
             r._score_buffers()["error"].zero_()
             assert torch.equal(r._logits_to_host(x), x.float().cpu()), (dtype, shape)
             assert int(r._score["error"]) == 7
+
+
+@pytest.mark.parametrize("model_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16, torch.float64])
+def test_logits_of_another_type_than_the_model_cross_unrounded(model_dtype, dtype):
+    """A caller's model may return logits of another type than its weights'."""
+    from minivllm_b200.engine import model_runner
+    r = object.__new__(model_runner.ModelRunner)
+    r.max_num_seqs, r.dtype, r._score = 4, model_dtype, None
+    r.error_word = torch.zeros(1, dtype=torch.int32, device="cuda")
+    n = model_runner.SCORE_PIECE
+    for shape in ((0, 32), (1, 3), (1, n // 4), (1, n // 2 + 1), (2, n + 3), (3, 2 * n + 5)):
+        x = torch.randn(shape, device="cuda", dtype=torch.float32).to(dtype)
+        assert torch.equal(r._logits_to_host(x), x.float().cpu()), shape
