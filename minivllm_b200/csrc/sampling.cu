@@ -231,6 +231,8 @@ sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t col
   const float slope = inv_t * kLog2;
   float shift = INFINITY;                        // (slack - best) in base 2
   // Piece p has the global columns base0 + p * kPiece and on; the first piece may begin before the shard, the last end behind it.
+  // A thread meets its columns in increasing order, so that the first of equal scores is the one that it keeps: what the shard
+  // has of a first piece that it begins inside goes to thread 0 before anything else.
   const uint32_t n_cols = static_cast<uint32_t>(cols), base0 = index_offset & ~3u, lead = index_offset - base0;
   const uint32_t skip = lead ? 1u : 0u, whole = (n_cols + lead) / kPiece, pieces = whole + ((n_cols + lead) % kPiece ? 1u : 0u);
   auto draw = [&](uint32_t p, uint32_t (&bits)[kPiece]) {
@@ -245,8 +247,8 @@ sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t col
     float top = best.v;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
-    // behind an infinite score only infinities and NaN are looked at
-    shift = top == INFINITY ? -INFINITY : (0.02f + 4e-6f * fabsf(top) - top) * kLog2;
+    // behind an infinite score only those that may be infinite too, and NaN, are looked at
+    shift = top == INFINITY ? -3e38f : (0.02f + 4e-6f * fabsf(top) - top) * kLog2;
   };
   // The whole warp; lanes that are not `live` have nothing to offer, nor have columns outside the shard.
   auto consider = [&](const float (&v)[kPiece], uint32_t p, bool live, bool inside) {
@@ -264,7 +266,7 @@ sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t col
     if (!__any_sync(0xffffffffu, live && !(most < kEdge))) return;
 #pragma unroll
     for (int j = 0; j < kPiece; ++j) {
-      const uint32_t i = p * kPiece + j - lead;  // wraps below zero: not below n_cols
+      const uint32_t i = p * kPiece + j - lead;
       if (live && !((j & 1 ? x[j / 2].y : x[j / 2].x) < kEdge) && (inside || i < n_cols)) best.offer(v[j] * inv_t + race_noise(bits[j]), i);
     }
     aim();
@@ -290,6 +292,15 @@ sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t col
       for (int j = 0; j < kPiece; ++j) v[j] = Elem<T>::to_f(at[j]);
     }
   };
+  if constexpr (!kVec) {
+    if (skip && my.at == 0) {
+      uint32_t bits[kPiece];
+      draw(0, bits);
+#pragma unroll
+      for (uint32_t j = 1; j < 4; ++j)
+        if (j >= lead && j - lead < n_cols) best.offer(Elem<T>::to_f(row[j - lead]) * inv_t + race_noise(bits[j]), j - lead);
+    }
+  }
   const uint32_t rounds = whole > skip ? (whole - skip) / my.threads : 0;
   uint32_t p = skip + my.at;
   if (rounds) {
@@ -308,10 +319,10 @@ sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t col
       consider(now, p, true, true);
     }
   }
-  // what is left: less than a round of whole pieces, and the pieces over the shard's edges
-  const uint32_t left = pieces - rounds * my.threads;      // the first piece of a shard that begins inside it among them
+  // what is left: less than a round of whole pieces, and the one over the shard's end
+  const uint32_t left = pieces - skip - rounds * my.threads;
   for (uint32_t it = 0; it * my.threads < left; ++it) {
-    const uint32_t k = it * my.threads + my.at, q = k < skip ? 0 : k + rounds * my.threads;
+    const uint32_t k = it * my.threads + my.at, q = skip + k + rounds * my.threads;
     const bool live = k < left;
     float v[kPiece];
 #pragma unroll

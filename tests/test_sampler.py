@@ -264,3 +264,33 @@ def test_sampled_scores_at_any_start_and_length(rows, cols, offset, dtype):
     for r, sc in enumerate(scores):
         assert 0 <= got[r] < cols and sc[got[r]] >= sc.max() - 4e-6 * max(1.0, abs(float(sc.max()))), r
     assert np.array_equal(S.decode_keys(keys).cpu().numpy(), tokens.cpu().numpy())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("offset", [0, 1, 2, 3, 4, 7])
+def test_the_first_of_equal_scores_wins_wherever_a_shard_begins(offset, dtype):
+    """Infinite scores, NaN and rows of -inf alone: the lowest column, also when it lies in front of the shard's first whole group of
+    four and the next such column is the same thread's."""
+    from minivllm_b200.layers import sampler as S
+    cols, own = 5000, -offset % 4            # thread 0 goes on at column `own`
+    x = _logits(12, 9, cols, dtype)
+    inf, nan = float("inf"), float("nan")
+    for at in (0, own, own + 1, 4096):
+        x[0, at] = inf
+        x[1, at] = nan
+        x[3, at] = 3e38                      # times 1 / T beyond the largest fp32 value
+    x[2] = -inf
+    x[4, 1], x[4, own + 2], x[5, own + 3], x[5, 4097] = inf, inf, nan, nan
+    x[6, 0], x[6, own], x[6, own + 1] = inf, nan, nan
+    x[7] = -inf
+    x[7, -1] = inf
+    for at in (own + 1, own + 4, own + 8):   # the first columns of other threads among them
+        x[8, at] = 3e38
+    want = [0, 0, 0, 0, 1, own + 3, own if own else 0, cols - 1, own + 1]
+    temps = torch.full((9,), 0.5)
+    step = torch.tensor([3], dtype=torch.int64, device="cuda")
+    if not own:
+        x[6, 0], want[6] = inf, own + 1      # the NaN behind
+    _, tokens = S.sample_rows(x.cuda(), temps.cuda(), 9, step, index_offset=offset, want_keys=False, want_tokens=True)
+    assert (tokens.cpu() - offset).tolist() == want
