@@ -38,8 +38,8 @@ __device__ __forceinline__ long long token_of_key(long long key) {
   return static_cast<long long>(0xffffffffu - static_cast<uint32_t>(key & 0xffffffffll));
 }
 
-// One CTA per row.  A thread walks its columns in increasing order and keeps the first maximum it meets
-// (strict >), so equal logits resolve to the lowest index within a thread; across threads the keys do it.
+// A thread walks its columns in increasing order and keeps the first maximum it meets (strict >), so equal logits resolve to the
+// lowest index within a thread; across threads the keys do it.
 // The best logit or score that a thread has met: the first maximum in visiting order, and a NaN is the maximum.
 struct Best {
   float v = -INFINITY;
@@ -57,19 +57,21 @@ struct Best {
   }
 };
 
-// A row belongs to the CTAs of a cluster; thread `at` of `threads` takes every threads-th piece.
-struct RowShare {
+// A row belongs to the CTAs of a cluster (kOne: to one CTA, the numbers are constants); thread `at` of `threads` takes every
+// threads-th piece.
+template <bool kOne> struct RowShare {
   uint32_t at, threads, rank, ctas;
   __device__ __forceinline__ RowShare() {
-    ctas = cg::this_cluster().num_blocks();
-    rank = cg::this_cluster().block_rank();
+    ctas = kOne ? 1 : cg::this_cluster().num_blocks();
+    rank = kOne ? 0 : cg::this_cluster().block_rank();
     at = rank * kArgmaxThreads + threadIdx.x;
     threads = ctas * kArgmaxThreads;
   }
 };
 
 // The row's largest key from all threads of its cluster, written by its first CTA.
-__device__ __forceinline__ void finish_row(const Best& best, uint32_t index_offset, const RowShare& my, int64_t row, long long* keys,
+template <bool kOne>
+__device__ __forceinline__ void finish_row(const Best& best, uint32_t index_offset, const RowShare<kOne>& my, int64_t row, long long* keys,
                                            long long* tokens) {
   long long key = best.have ? make_key(best.v, index_offset + best.idx) : LLONG_MIN;
 #pragma unroll
@@ -101,8 +103,8 @@ __device__ __forceinline__ void finish_row(const Best& best, uint32_t index_offs
 // maxima, exact, NaN-propagating) and compared with the running one; the chunk that raised it is kept and searched for the
 // position at the end.  Chunks are visited in increasing order and only a strictly larger maximum replaces the kept chunk,
 // so the first of equal maxima survives.
-template <typename T>
-__device__ __forceinline__ void argmax_share(const T* row, int64_t cols, bool aligned, const RowShare& my, Best& best) {
+template <typename T, bool kOne>
+__device__ __forceinline__ void argmax_share(const T* row, int64_t cols, bool aligned, const RowShare<kOne>& my, Best& best) {
   // 16-byte chunks when every row starts on a 16-byte boundary
   const int64_t chunks = sizeof(T) == 2 && aligned ? cols / 8 : 0;
   if constexpr (sizeof(T) == 2) {
@@ -150,11 +152,12 @@ __device__ __forceinline__ void argmax_share(const T* row, int64_t cols, bool al
     best.offer(Elem<T>::to_f(row[i]), static_cast<uint32_t>(i));
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kArgmaxThreads)
+constexpr int kArgmaxCtasPerSM = 5;
+template <typename T, bool kOne>
+__global__ void __launch_bounds__(kArgmaxThreads, kArgmaxCtasPerSM)
 argmax_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t cols, uint32_t index_offset, bool aligned,
                    long long* __restrict__ keys, long long* __restrict__ tokens) {
-  const RowShare my;
+  const RowShare<kOne> my;
   const int64_t r = blockIdx.x / my.ctas;
   Best best;
   argmax_share(logits + r * row_stride, cols, aligned, my, best);
@@ -212,7 +215,7 @@ __global__ void __launch_bounds__(kArgmaxThreads)
 sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t cols, uint32_t index_offset, bool aligned,
                    const float* __restrict__ temperatures, unsigned long long seed, const long long* __restrict__ step_ptr,
                    long long* __restrict__ keys, long long* __restrict__ tokens) {
-  const RowShare my;
+  const RowShare<false> my;
   const uint32_t rowi = blockIdx.x / my.ctas;
   const T* row = logits + static_cast<int64_t>(rowi) * row_stride;
   const float temp = temperatures[rowi];
@@ -348,17 +351,26 @@ __global__ void argmax_decode_kernel(const long long* __restrict__ keys, int sha
   tokens[r] = token_of_key(key);
 }
 
-// A row's CTAs, one cluster: more of them while the rows alone would leave SMs with fewer than four, as long as each thread has
-// two 16-byte pieces.
+// A row's CTAs, one cluster.  Sampling, which is bound by issue, and logits that are read one by one: more of them while the rows
+// alone would leave SMs with fewer than four, as long as each thread has two 16-byte pieces.
 static unsigned row_ctas(int64_t rows, int64_t cols) {
   unsigned n = 1;
   while (n < kMaxRowCtas && rows * n < 4 * kNumSMs && cols >= static_cast<int64_t>(n) * 2 * kArgmaxThreads * 16) n *= 2;
   return n;
 }
+// Selection from 16-byte pieces is bound by memory and ends with a cluster's barriers: more CTAs only while all of them are
+// resident at once, and while the row is long enough to pay for them.  bf16, a CTA a row against this rule: 151,936 columns 16
+// rows 15.6 -> 5.5 us, 64 17.2 -> 7.9, 128 17.9 -> 10.7, 256 20.4 -> 17.3; from 512 rows on (27.8 us) one CTA, which two took 33.5
+// for.  32,768 columns 64 rows 5.0 -> 4.2, 128 5.5 -> 5.3; 256 rows 6.4 with one, 6.8 with two.
+static unsigned argmax_ctas(int64_t rows, int64_t cols) {
+  const int64_t places = cols >= 65536 ? kArgmaxCtasPerSM * kNumSMs : kArgmaxCtasPerSM * kNumSMs / 2;
+  unsigned n = 1;
+  while (n < kMaxRowCtas && rows * n * 2 <= places && cols >= static_cast<int64_t>(n) * 16384) n *= 2;
+  return n;
+}
 
 template <typename... P, typename... A>
-static int launch_rows(const char* what, void (*kernel)(P...), int64_t rows, int64_t cols, cudaStream_t st, A... args) {
-  const unsigned ctas = row_ctas(rows, cols);
+static int launch_rows(const char* what, void (*kernel)(P...), int64_t rows, unsigned ctas, cudaStream_t st, A... args) {
   if (rows * ctas > 0x7fffffffLL) return fail(MV_ERR_LIMIT, "%s: too many rows", what);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(rows) * ctas);
@@ -389,7 +401,8 @@ extern "C" int mv_argmax_rows(const void* logits, int64_t row_stride, int64_t ro
     return fail(MV_ERR_LIMIT, "argmax_rows: column index beyond 32 bits or too many rows");
   auto run = [&](auto zero) {
     using T = decltype(zero);
-    return launch_rows("argmax_rows_kernel", argmax_rows_kernel<T>, rows, cols, static_cast<cudaStream_t>(stream),
+    const unsigned ctas = sizeof(T) == 2 && aligned ? argmax_ctas(rows, cols) : row_ctas(rows, cols);
+    return launch_rows("argmax_rows_kernel", ctas == 1 ? argmax_rows_kernel<T, true> : argmax_rows_kernel<T, false>, rows, ctas, static_cast<cudaStream_t>(stream),
                        static_cast<const T*>(logits), row_stride, cols, static_cast<uint32_t>(index_offset), aligned,
                        reinterpret_cast<long long*>(keys), reinterpret_cast<long long*>(tokens));
   };
@@ -425,7 +438,7 @@ extern "C" int mv_sample_rows(const void* logits, int64_t row_stride, int64_t ro
     constexpr int kPiece = 16 / sizeof(T);
     const bool aligned = row_stride % 8 == 0 && aligned16(logits);
     const bool vec = row_stride % kPiece == 0 && aligned16(logits) && index_offset % kPiece == 0;
-    return launch_rows("sample_rows_kernel", vec ? sample_rows_kernel<T, true> : sample_rows_kernel<T, false>, rows, cols,
+    return launch_rows("sample_rows_kernel", vec ? sample_rows_kernel<T, true> : sample_rows_kernel<T, false>, rows, row_ctas(rows, cols),
                        static_cast<cudaStream_t>(stream), static_cast<const T*>(logits), row_stride, cols,
                        static_cast<uint32_t>(index_offset), aligned, temperatures, static_cast<unsigned long long>(seed),
                        reinterpret_cast<const long long*>(step), reinterpret_cast<long long*>(keys),

@@ -294,3 +294,19 @@ def test_the_first_of_equal_scores_wins_wherever_a_shard_begins(offset, dtype):
         x[6, 0], want[6] = inf, own + 1      # the NaN behind
     _, tokens = S.sample_rows(x.cuda(), temps.cuda(), 9, step, index_offset=offset, want_keys=False, want_tokens=True)
     assert (tokens.cpu() - offset).tolist() == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(1, 16376), (3, 16384), (370, 16384), (46, 65536), (47, 65536), (92, 65544), (93, 65543), (371, 65536),
+                                       (185, 32768), (186, 32768), (46, 131072)])
+def test_selection_by_any_number_of_ctas_a_row(rows, cols):
+    """One to eight CTAs a row, at the numbers of rows where it changes: the tokens are those of torch.argmax, the first of equals."""
+    from minivllm_b200.layers import sampler as S
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    for dtype in (torch.bfloat16, torch.float32):
+        x = torch.randn(rows, cols + 8, generator=g, device="cuda").to(dtype)[:, :cols]
+        x[0, cols // 3], x[0, cols - 1] = 50.0, 50.0
+        tokens = S.argmax_rows(x, want_keys=False, want_tokens=True)[1]
+        top = x.float().max(1).values
+        first = torch.where(x.float() == top[:, None], torch.arange(cols, device="cuda"), cols).min(1).values
+        assert torch.equal(tokens, first)
