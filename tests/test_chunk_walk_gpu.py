@@ -76,6 +76,26 @@ def test_segments(kind, H, K, V, first, second):
             assert _rel(S[s], ref[s][1]) < 2e-4, s
 
 
+def test_decays_are_no_further_off_than_32_bits_need():
+    """The logarithms of 63 decays, summed, from a state that decays from one token on: their mean error over heads and channels, to a
+    sum of about 40.  A logarithm's relative error is 4e-8 rms with a mean of 3e-9, the factor log2(e) of all has -1.4e-8, 5e-7
+    here; an exponential from ex2.approx and a division in the logarithm had -5.8e-8, 2.3e-6 here."""
+    from minivllm_b200.layers import gla
+    H, K, V, n, tau = 16, 128, 128, 8, 0.125          # exact, as is its reciprocal
+    T = 64 * n
+    g = torch.Generator().manual_seed(2)
+    z = (torch.randn(T, H * K, generator=g) + 3).to(BF)
+    q, k, v = torch.zeros(T, H * K, dtype=BF), torch.zeros(T, H * K, dtype=BF), torch.zeros(T, H * V, dtype=BF)
+    k[::64], v[::64] = 1.0, 1.0
+    a, b, c = torch.cat([q, k, v], 1).cuda().split([H * K, H * K, H * V], 1)
+    S = torch.zeros(n, H, K, V, device="cuda")
+    gla.gla_scan(a, b, c, z.cuda(), tau, _i32([64 * i for i in range(n + 1)]), _i32(list(range(n))), _i32([0] * n), S, H, K, V, chunked=True)
+    want = torch.nn.functional.logsigmoid(z.double()).view(n, 64, H, K)[:, 1:].sum(1) / tau
+    assert -60 < float(want.mean()) < -30
+    err = torch.log(S[..., 0].double().cpu()) - want
+    assert abs(float(err.mean())) < 1e-6 and float(err.square().mean().sqrt()) < 1e-5
+
+
 @pytest.mark.parametrize("kind", ["gla", "mlstm"])
 @pytest.mark.parametrize("lens", [[300, 200], [1024]], ids=["whole", "segments"])
 def test_a_wait_that_runs_out_ends_the_walk(kind, lens):
