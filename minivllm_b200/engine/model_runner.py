@@ -419,8 +419,7 @@ class ModelRunner:
         the mixed step.  Returns the logits at the wanted places, fp32 on the CPU."""
         seqs, counts, want = [b[0] for b in batch], [b[1] for b in batch], [b[2] for b in batch]
         if all(n == 1 for n in counts) and all(s.on_device for s in seqs):
-            given = torch.tensor([[s.slot for s in seqs], [s.last_token for s in seqs]], dtype=torch.int64)
-            given = self._score_buffers()["given"][:, :len(seqs)].copy_(given).to(self.device, non_blocking=True)
+            given = self._given([s.slot for s in seqs], [s.last_token for s in seqs]).to(self.device, non_blocking=True)
             self.state.last_token.index_copy_(0, given[0], given[1])
             temps = None if self.greedy else torch.zeros(len(seqs), device=self.device)
             if self.enforce_eager or not self.graphs:
@@ -453,10 +452,15 @@ class ModelRunner:
             at = (16 * n + 8 + 63) // 64 * 64
             raw = torch.empty(at + 2 * SCORE_PIECE * item, dtype=torch.uint8).pin_memory()      # one block: pinning is dear
             part = lambda a, count, dtype: raw[a:a + count * torch.empty((), dtype=dtype).element_size()].view(dtype)
-            self._score = {"given": part(0, 2 * n, torch.int64).view(2, n), "error": part(16 * n, 1, torch.int32),
+            self._score = {"given": part(0, 2 * n, torch.int64), "error": part(16 * n, 1, torch.int32),
                            "logits": [part(at + i * SCORE_PIECE * item, SCORE_PIECE * item, torch.uint8) for i in range(2)],
                            "done": [torch.cuda.Event() for _ in range(2)]}
         return self._score
+
+    def _given(self, slots, tokens):
+        """(2, sequences) of a scored step's slots and tokens in pinned memory, without gaps: rows cut from a wider buffer would go
+        to the device by way of a pageable copy, and the host would wait for them."""
+        return self._score_buffers()["given"][:2 * len(slots)].view(2, -1).copy_(torch.tensor([slots, tokens], dtype=torch.int64))
 
     def _logits_to_host(self, logits):
         """fp32 on the CPU, and the error word behind them in the pinned buffer.  The values cross in their own type, which need not

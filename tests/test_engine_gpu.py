@@ -255,3 +255,15 @@ def test_logits_of_another_type_than_the_model_cross_unrounded(model_dtype, dtyp
     for shape in ((0, 32), (1, 3), (1, n // 4), (1, n // 2 + 1), (2, n + 3), (3, 2 * n + 5)):
         x = torch.randn(shape, device="cuda", dtype=torch.float32).to(dtype)
         assert torch.equal(r._logits_to_host(x), x.float().cpu()), shape
+
+
+def test_given_tokens_cross_to_the_device_from_pinned_memory():
+    """A part-filled batch too: contiguous, or torch would copy it to pageable memory first."""
+    from minivllm_b200.engine import model_runner
+    r = object.__new__(model_runner.ModelRunner)
+    r.max_num_seqs, r.dtype, r._score = 7, torch.bfloat16, None
+    for n in (1, 3, 7):
+        slots, tokens = list(range(n)), [100 + i for i in range(n)]
+        given = r._given(slots, tokens)
+        assert given.is_contiguous() and given.is_pinned() and given.tolist() == [slots, tokens]
+        assert given.data_ptr() == r._score["given"].data_ptr()
