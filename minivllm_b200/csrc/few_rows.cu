@@ -5,10 +5,10 @@
 // 16-byte pieces of their rows, and the products are register MMAs: 16 tokens on the M side, 8 features on the N side, the
 // reduction index permuted so that a thread's piece is its operand of two steps.  A CTA owns 8 kTiles features and its warps
 // take 64-wide blocks of the reduction in turn, which puts a matrix of a few megabytes in flight at once; sums of the warps
-// are added in order in shared memory.  Bound: memory, and the latency of one trip to it where the matrix is small.  16 rows, bf16,
-// against the library's product: 1024 features of 3072 3.9 us (8.5), 1024 of 2048 3.5 (6.6), 4096 of 1024 3.9 (4.8), gated 3072
-// of 1024 5.3 (7.6 with the activation); the library is ahead from about 8 M weights on (6144 of 4096: 15.2 against 12.9),
-// unless the features are few (4096 of 4096: 9.4 against 10.1).
+// are added in order in shared memory.  Bound: memory, and the latency of one trip to it where the matrix is small.  us for 16 rows,
+// bf16, and of the library's product: 1,024 features of 3,072 4.0 (8.3), 1,024 of 2,048 3.5 (6.5), 4,096 of 1,024 3.9 (4.8), gated
+// 3,072 of 1,024 5.3 (7.5 with the activation), 4,096 of 12,288 21.4 (22.3).  The library is ahead where the features are more than
+// CTAs are resident for (6,144 of 4,096: 15.1 against 13.0) or the reduction is very deep: layers/linear.py has the lines.
 #include "mma.cuh"
 
 namespace mv {
@@ -99,8 +99,10 @@ static int launch_few_rows(void* out, const void* x, int64_t x_stride, const voi
   // round of two CTAs an SM up to 4,736 of them and reads x half as often.
   const int units = n / 8;
   if (units <= kNumSMs) return go(few_rows_kernel<T, 1, 16, kGated>, 1, 16);
-  if (kGated || units <= 2 * kNumSMs) return go(few_rows_kernel<T, 1, 8, kGated>, 1, 8);
-  return go(few_rows_kernel<T, kGated ? 1 : 2, 8, kGated>, kGated ? 1 : 2, 8);
+  if constexpr (!kGated) {
+    if (units > 2 * kNumSMs) return go(few_rows_kernel<T, 2, 8, false>, 2, 8);
+  }
+  return go(few_rows_kernel<T, 1, 8, kGated>, 1, 8);
 }
 
 }  // namespace mv

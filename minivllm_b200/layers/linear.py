@@ -13,6 +13,19 @@ from .activation import silu_and_mul
 FEW_ROWS = 16
 
 
+def _few_rows_pay(n, k, gated):
+    """Whether the kernel is the faster one for up to 16 rows and a weight (n, k).  us, kernel and library, 16 rows unless said:
+    4,096 x 12,288 21.4 and 22.3, 4,096 x 4,096 9.3 and 9.8, 2,048 x 18,944 21.3 and 25.7; deeper ones the library's from 2,432
+    features on (2,560 x 14,336 20.9 and 18.9).  Over 4,736 features CTAs take a second turn: 4,608 x 1,536 5.2 and 5.6, 6,144 x 1,024
+    5.3 and 5.4, but 5,120 x 1,536 7.0 and 6.3, 6,144 x 512 4.4 and 4.3, 32,768 x 256 11.0 and 5.6.  Gated, with the activation's
+    launch saved: 12,288 x 512 6.5 and 7.5, 16,384 x 512 8.0 and 7.6."""
+    if n <= 4096:
+        return k <= (18944 if n <= 2048 else 12288)
+    if n * k > 8 << 20:
+        return False
+    return n <= 12288 if gated else n <= 4736 or (n <= 6144 and 768 <= k <= 1024)
+
+
 def _few_rows(x, weight, gated):
     """The product of a decode step's rows, or None where it is the library's: more rows, other types, sizes or layouts, or a
     weight so large that the library's is faster (csrc/few_rows.cu)."""
@@ -20,7 +33,7 @@ def _few_rows(x, weight, gated):
     rows = x.shape[0]
     if not (x.is_cuda and x.dim() == 2 and 0 < rows <= FEW_ROWS and x.dtype == weight.dtype and x.shape[1] == k and
             x.dtype in (torch.bfloat16, torch.float16)) or k % 64 or n % (16 if gated else 8) or \
-            (n * k > 8 << 20 and n > 4096) or x.stride(1) != 1 or not weight.is_contiguous() or x.device != weight.device or \
+            not _few_rows_pay(n, k, gated) or x.stride(1) != 1 or not weight.is_contiguous() or x.device != weight.device or \
             x.data_ptr() % 16 or weight.data_ptr() % 16 or (rows > 1 and (x.stride(0) % 8 or x.stride(0) < k)) or \
             (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)):
         return None

@@ -6,9 +6,17 @@ import torch.nn.functional as F
 
 from minivllm_b200.layers import linear as L
 
-pytestmark = pytest.mark.gpu
+
+@pytest.mark.parametrize("n,k,gated,pay", [(4096, 12288, False, True), (4096, 12352, False, False), (2048, 18944, False, True),
+                                           (2048, 19008, False, False), (4736, 1024, False, True), (4744, 512, False, False),
+                                           (6144, 1024, False, True), (6144, 704, False, False), (6152, 1024, False, False),
+                                           (32768, 256, False, False), (12288, 512, True, True), (12304, 256, True, False),
+                                           (6144, 1024, True, True), (12288, 768, True, False)])
+def test_where_the_kernel_is_the_faster_one(n, k, gated, pay):
+    assert L._few_rows_pay(n, k, gated) is pay
 
 
+@pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("n,k", [(16, 64), (48, 128), (1184, 576), (1200, 2048), (2368, 64), (2384, 192), (4096, 1024), (1024, 3072)])
 def test_few_rows(n, k, dtype):
@@ -28,6 +36,7 @@ def test_few_rows(n, k, dtype):
         assert float(((got - want).abs() - 4 * u * want.abs()).max()) < 2 * u
 
 
+@pytest.mark.gpu
 def test_what_the_library_takes():
     w = torch.randn(64, 128, device="cuda").bfloat16()
     x = torch.randn(17, 128, device="cuda").bfloat16()
