@@ -6,11 +6,16 @@ that kernels may read it in 16-byte pieces.  `router_logits` is the one product 
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch._C import _get_tracing_state, _len_torch_dispatch_stack, _len_torch_function_stack
+from torch._C._functorch import peek_interpreter_stack
+from torch.autograd import forward_ad
+from torch.compiler import is_compiling
 
 from .. import _cabi
 from .activation import silu_and_mul
 
 FEW_ROWS = 16
+_PLAIN = (torch.Tensor, nn.Parameter)
 
 
 def _few_rows_pay(n, k, gated):
@@ -26,16 +31,28 @@ def _few_rows_pay(n, k, gated):
     return n <= 12288 if gated else n <= 4736 or (n <= 6144 and 768 <= k <= 1024)
 
 
+def _eager(x, weight):
+    """Plain tensors, and nobody about who means to see the product: subclasses, modes, tracing, autocast, forward mode and function
+    transforms are served by the library's."""
+    return type(x) in _PLAIN and type(weight) in _PLAIN and not (
+        is_compiling() or _get_tracing_state() is not None or _len_torch_dispatch_stack() or _len_torch_function_stack() or
+        torch.is_autocast_enabled() or forward_ad._current_level >= 0 or peek_interpreter_stack() is not None)
+
+
 def _few_rows(x, weight, gated):
-    """The product of a decode step's rows, or None where it is the library's: more rows, other types, sizes or layouts, or a
-    weight so large that the library's is faster (csrc/few_rows.cu)."""
+    """The product of a decode step's rows, or None where it is the library's: more rows, other types, sizes or layouts, a device
+    that is not the current one, a weight with which the library's is faster (csrc/few_rows.cu), or one that others must see."""
+    if type(x) is not torch.Tensor and not _eager(x, weight):       # before anything is asked of its sizes
+        return None
     n, k = weight.shape
     rows = x.shape[0]
     if not (x.is_cuda and x.dim() == 2 and 0 < rows <= FEW_ROWS and x.dtype == weight.dtype and x.shape[1] == k and
-            x.dtype in (torch.bfloat16, torch.float16)) or k % 64 or n % (16 if gated else 8) or \
-            not _few_rows_pay(n, k, gated) or x.stride(1) != 1 or not weight.is_contiguous() or x.device != weight.device or \
-            x.data_ptr() % 16 or weight.data_ptr() % 16 or (rows > 1 and (x.stride(0) % 8 or x.stride(0) < k)) or \
+            x.dtype in (torch.bfloat16, torch.float16)) or k % 64 or n % (16 if gated else 8) or not _few_rows_pay(n, k, gated) or \
+            x.device != weight.device or x.get_device() != torch.cuda.current_device() or not _eager(x, weight) or \
             (torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad)):
+        return None
+    if x.stride(1) != 1 or not weight.is_contiguous() or x.data_ptr() % 16 or weight.data_ptr() % 16 or \
+            (rows > 1 and (x.stride(0) % 8 or x.stride(0) < k)):
         return None
     n = n // 2 if gated else n
     out = torch.empty((rows, n), dtype=x.dtype, device=x.device)

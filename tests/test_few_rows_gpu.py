@@ -46,3 +46,43 @@ def test_what_the_library_takes():
         assert L._few_rows(a, b, False) is None
         assert L.linear(a, b).shape == (a.shape[0], b.shape[0])
     assert L.linear(x[:0], w).shape == (0, 64)
+
+
+class _Seen(torch.utils._python_dispatch.TorchDispatchMode):
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.ops = getattr(self, "ops", []) + [str(func)]
+        return func(*args, **(kwargs or {}))
+
+
+def test_who_must_see_a_product_gets_the_library_s():
+    """Modes, transforms, forward mode, tracing and subclasses; the same calls on the CPU."""
+    from torch.autograd import forward_ad
+    x, w = torch.randn(3, 64), torch.randn(16, 64)
+    assert L._eager(x, w) and L._eager(x, torch.nn.Parameter(w))
+    with _Seen() as seen:
+        assert not L._eager(x, w)
+        L.linear(x, w)
+    assert seen.ops
+    with forward_ad.dual_level():
+        y = L.linear(forward_ad.make_dual(x, torch.ones_like(x)), w)
+        assert not L._eager(x, w) and torch.equal(forward_ad.unpack_dual(y).tangent, F.linear(torch.ones_like(x), w))
+    asked = []
+    assert torch.allclose(torch.func.vmap(lambda r: (asked.append(L._eager(r, w)), L.linear(r[None], w)[0])[1])(x), F.linear(x, w), atol=1e-5)
+    assert asked == [False]
+    assert not L._eager(x.as_subclass(type("Sub", (torch.Tensor,), {})), w)
+    torch.jit.trace(lambda a: (asked.append(L._eager(a, w)), L.linear(a, w))[1], x, check_trace=False)
+    assert asked == [False, False]
+    assert L._eager(x, w)
+
+
+@pytest.mark.gpu
+def test_autocast_and_forward_mode_on_gpu():
+    from torch.autograd import forward_ad
+    x, w = torch.randn(4, 128, device="cuda").bfloat16(), torch.randn(64, 128, device="cuda").bfloat16()
+    assert L._few_rows(x, w, False) is not None
+    with torch.autocast("cuda", torch.float16):
+        assert L.linear(x, w).dtype == F.linear(x, w).dtype == torch.float16
+    with forward_ad.dual_level():
+        y = L.linear(forward_ad.make_dual(x, x), w)
+        assert torch.equal(forward_ad.unpack_dual(y).tangent, F.linear(x, w))
+    assert torch.equal(torch.func.vmap(L.linear, (0, None))(x.view(2, 2, 128), w), torch.func.vmap(F.linear, (0, None))(x.view(2, 2, 128), w))
