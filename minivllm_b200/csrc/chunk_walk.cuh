@@ -603,29 +603,46 @@ __global__ void __launch_bounds__(kJoinThreads) chunk_join_kernel(const WalkPara
   }
 }
 
-// The sizes the walk takes; the register form (state_chunk.cuh) keeps the narrow ones, where most of 128 lanes would idle.
-inline bool walk_takes(int K, int V) { return K > 32 && V > 64; }
-// Chunks of a segment, or 0 for whole sequences.  A segment costs a second, lighter pass, so sequences are cut only where that
-// brings at least three times as many CTAs, none shorter than four chunks, all of them within one wave.
-inline int walk_segment(int64_t tokens, int num_seqs, int heads, int V) {
+// Chunks of a segment, or 0 for whole sequences.  A segment costs a second, lighter pass and the join, so sequences are cut only
+// where that brings at least three times as many CTAs, none shorter than four chunks, all of them within one wave, and where the mean
+// sequence has more than three (mLSTM, whose chunks take twice as long: two) segments' chunks.  One sequence, 4 heads of 128 x 128:
+// gla 8 chunks 31.3 us whole and 37.6 in segments, 16 chunks 45.6 and 38.2; mLSTM 8 chunks 36.3 and 38.3, 16 chunks 62.7 and 37.8.
+inline int walk_segment(bool mem, int64_t tokens, int num_seqs, int heads, int V) {
   const int64_t blocks = static_cast<int64_t>(heads) * ((V + kWalkCols - 1) / kWalkCols);
   const int64_t all = kNumSMs / blocks;                     // segments there is room for
   if (num_seqs <= 0 || all < 3 * num_seqs) return 0;
   const int64_t room = num_seqs > 1 ? all - num_seqs : all; // each sequence's last segment may be a short one
   const int64_t chunks = (tokens + kChunk - 1) / kChunk, per = std::max<int64_t>(4, (chunks + room - 1) / room);
-  return chunks > per * num_seqs ? static_cast<int>(per) : 0;
+  return chunks > (mem ? 2 : 3) * per * num_seqs ? static_cast<int>(per) : 0;
+}
+// Whether the walk takes a call; the register form keeps narrow heads, where most of 128 lanes would idle, and short work, where
+// setting the walk up (2 us) is not paid back.  us, walk and register form:
+//   gla, 32 of 32 tokens, 16 heads of 64 x 128 44.0 and 40.7, 128 of 64 160 and 164; 8 heads of 64 x 72, 64 of 17 40.0 and 37.9,
+//     16 of 128 19.9 and 21.0; heads of 128 x 256, 16 of 32 32.9 and 33.8
+//   mLSTM, heads of 128: 4 x 128, 16 of 64 14.3 and 13.3, 64 of 64 24.9 and 27.5; 8 x 256, 32 of 32 42.4 and 40.6, 64 of 64 70.0 and 74.7
+//     heads of 64: 16 x 128, 64 of 64 67.9 and 62.9, 16 of 128 31.8 and 33.8, 4 of 256 23.4 and 23.0, 16 of 256 46.4 and 53.8;
+//     8 x 72, 64 of 128 55.7 and 54.2, 16 of 256 26.6 and 28.2; 4 x 128, 16 of 512 36.4 and 36.8, 1 of 512 33.9 and 31.7
+//     heads that are not made of slabs, whose q and k four warps copy: 8 x 48 (96), 8 of 1024 79.8 and 66.1
+inline bool walk_takes(bool mem, int64_t tokens, int num_seqs, int heads, int K, int V) {
+  if (K <= 32 || V <= 64) return false;
+  if (num_seqs <= 0 || walk_segment(mem, tokens, num_seqs, heads, V)) return true;
+  const int64_t mean = tokens / num_seqs, pairs = static_cast<int64_t>(num_seqs) * heads, ctas = pairs * ((V + kWalkCols - 1) / kWalkCols);
+  if (!mem) return K > 64 || mean > kChunk || (V % kWalkCols == 0 && pairs > 512);
+  if (K % 64) return false;
+  if (K > 64) return mean > kChunk || (ctas >= kNumSMs && (V <= kWalkCols || mean > kChunk / 2 || pairs > 256));
+  return ctas >= 128 ? mean >= (V % kWalkCols ? 256 : 96) : ctas >= 48 && mean >= 512;
 }
 inline int64_t walk_segments(int64_t tokens, int num_seqs, int per) { return per ? tokens / (per * kChunk) + std::min<int64_t>(num_seqs, tokens) : 0; }
 // Floats of the segments' states, n and decays.
-inline int64_t walk_segment_floats(int64_t tokens, int num_seqs, int heads, int K, int V) {
-  return walk_segments(tokens, num_seqs, walk_segment(tokens, num_seqs, heads, V)) * heads * (static_cast<int64_t>(K) * V + 2 * K);
+inline int64_t walk_segment_floats(bool mem, int64_t tokens, int num_seqs, int heads, int K, int V) {
+  return walk_segments(tokens, num_seqs, walk_segment(mem, tokens, num_seqs, heads, V)) * heads * (static_cast<int64_t>(K) * V + 2 * K);
 }
 
 // scratch holds the chunks' blobs, `segments` (16-byte aligned) walk_segment_floats.
 template <int K, bool kMem>
 int run_walk(const char* what, WalkParams p, int64_t tokens, float* segments, cudaStream_t st) {
   p.inject = g_walk_inject.exchange(0);                    // one call only
-  p.seg_chunks = walk_segment(tokens, p.num_seqs, p.heads, p.V);
+  p.seg_chunks = walk_segment(kMem, tokens, p.num_seqs, p.heads, p.V);
   const int64_t units = p.seg_chunks ? walk_segments(tokens, p.num_seqs, p.seg_chunks) : p.num_seqs;
   p.seg_state = segments;
   p.seg_n = segments + units * p.heads * p.K * p.V;

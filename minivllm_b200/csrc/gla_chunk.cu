@@ -460,9 +460,9 @@ extern "C" int64_t mv_gla_chunk_workspace_bytes(int64_t tokens, int num_seqs, in
   using namespace mv;
   if (tokens < 0 || num_seqs < 0 || heads <= 0 || !chunk_takes(dim, vdim)) return -1;
   const int64_t chunks = chunk_bound(tokens, num_seqs) * heads;
-  if (!walk_takes(dim, vdim)) return chunks * gla_scratch_bytes(dim);
+  if (!walk_takes(false, tokens, num_seqs, heads, dim, vdim)) return chunks * gla_scratch_bytes(dim);
   return chunks * (dim <= 64 ? WalkBlob<64, false>::kBytes : WalkBlob<128, false>::kBytes) +
-         walk_segment_floats(tokens, num_seqs, heads, dim, vdim) * 4;
+         walk_segment_floats(false, tokens, num_seqs, heads, dim, vdim) * 4;
 }
 
 // Both recurrences; kTime: p.zf, p.w0 and p.bonus, else p.z and p.inv_tau.
@@ -486,7 +486,7 @@ static int run_chunks(const char* what, const mv::GlaChunkParams& p, int64_t tok
     kernel<<<dim3(static_cast<unsigned>(chunks), heads), kGpThreads, bytes, st>>>(p);
     return check_launch(what);
   };
-  if (walk_takes(dim, vdim)) {
+  if (walk_takes(false, tokens, num_seqs, heads, dim, vdim)) {
     auto walk = [&](auto kk) {
       constexpr int K = decltype(kk)::value;
       const int rc = prepare(gla_prepare_kernel<K, kTime, true>, GlaPrepShape<K>::kBytes);

@@ -329,9 +329,9 @@ extern "C" int64_t mv_mlstm_chunk_workspace_bytes(int64_t tokens, int num_seqs, 
   using namespace mv;
   if (tokens < 0 || num_seqs < 0 || heads <= 0 || !chunk_takes(dim, vdim)) return -1;
   const int64_t chunks = chunk_bound(tokens, num_seqs) * heads;
-  if (!walk_takes(dim, vdim)) return chunks * mlstm_scratch_bytes(dim);
+  if (!walk_takes(true, tokens, num_seqs, heads, dim, vdim)) return chunks * mlstm_scratch_bytes(dim);
   return chunks * (dim <= 64 ? WalkBlob<64, true>::kBytes : WalkBlob<128, true>::kBytes) +
-         walk_segment_floats(tokens, num_seqs, heads, dim, vdim) * 4;
+         walk_segment_floats(true, tokens, num_seqs, heads, dim, vdim) * 4;
 }
 
 extern "C" int mv_mlstm_chunk_scan(void* out, int64_t out_stride, float* den, const void* q, const void* k, const void* v,
@@ -352,7 +352,7 @@ extern "C" int mv_mlstm_chunk_scan(void* out, int64_t out_stride, float* den, co
   const MemChunkParams p{static_cast<__nv_bfloat16*>(out), out_stride, den, c(q), c(k), c(v), stride, reinterpret_cast<const float4*>(chain),
                          q_scale, cu, slots, start, num_seqs, S, n, num_slots, heads, dim, vdim, static_cast<unsigned char*>(workspace)};
   auto st = static_cast<cudaStream_t>(stream);
-  if (walk_takes(dim, vdim)) {
+  if (walk_takes(true, tokens, num_seqs, heads, dim, vdim)) {
     auto walk = [&](auto kk) {
       constexpr int K = decltype(kk)::value;
       using Vc = MemVec<K>;

@@ -76,6 +76,17 @@ def test_segments(kind, H, K, V, first, second):
             assert _rel(S[s], ref[s][1]) < 2e-4, s
 
 
+# Both sides of the lines between whole sequences and segments, and between the walk and the register form: one and two chunks of
+# narrow heads, heads that are not made of slabs, few and many sequences.
+@pytest.mark.parametrize("kind", ["gla", "time", "mlstm"])
+@pytest.mark.parametrize("H,K,V,first,second", [(1, 64, 128, [64 * 12], [64 * 12 + 1]), (1, 128, 128, [64 * 8], [64 * 8 + 1]),
+                                                (2, 64, 128, [2100, 1, 700], [900, 0, 40]), (4, 64, 72, [64] * 3, [65] * 3),
+                                                (33, 64, 128, [17] * 16, [96] * 16), (5, 128, 256, [33] * 16, [32] * 16),
+                                                (8, 48, 96, [500] * 7, [100] * 7)], ids=str)
+def test_forms_and_lengths(kind, H, K, V, first, second):
+    test_segments(kind, H, K, V, first, second)
+
+
 def test_decays_are_no_further_off_than_32_bits_need():
     """The logarithms of 63 decays, summed, from a state that decays from one token on: their mean error over heads and channels, to a
     sum of about 40.  A logarithm's relative error is 4e-8 rms with a mean of 3e-9, the factor log2(e) of all has -1.4e-8, 5e-7
