@@ -418,7 +418,7 @@ def case_sample(device, pk, iters=20):
         return p.div_(torch.empty_like(p).exponential_(1).clamp_min_(1e-10)).argmax(dim=-1)
     ref = _time_calls([torch_race], max(2, iters // 4), 2)
     return _hbm(ms, x.numel() * 2 + 512 * 8, pk, torch_softmax_race_us=ref * 1e3,
-                note="compute-bound (Philox + two logarithms per logit); the HBM figure is for scale only")
+                note="compute-bound (Philox + a bound of each score); the HBM figure is for scale only")
 
 
 def case_allreduce_emulated(device, pk, iters=20):

@@ -25,10 +25,10 @@
 // Bound: gla and time mixing read 98 KB a chunk, two column blocks of a head the same 82 KB of it, at about 6 TB/s over all SMs
 // (L2); mLSTM the chain of w V, state and update.  Before (register MMAs): 885 and 242 us for the two walks below.
 //   1 x 16,384 tokens, 8 heads of 128 x 256 (gla, 9 segments): 38 us own states, 11 us join, 74 to 84 us walk
-//   16 x 512-1536 tokens, 8 heads of 128 x 256 (mLSTM): 138 us
+//   16 x 512-1536 tokens, 8 heads of 128 x 256 (mLSTM): 121 us
 //
-// More CTAs than SMs: the longest sequences go first (mLSTM, 16 x 512-1536 tokens, 256 CTAs: 138 -> 121 us of the walk; gla on
-// the same: 216 -> 191 us in all).
+// More CTAs than SMs: the longest sequences go first (that mLSTM walk, 256 CTAs, took 138 us in the order of the batch; gla on the
+// same, in all: 216 -> 191 us).
 //
 // A sequence's chunks take their time one after the other.  Where sequences, heads and column blocks are too few for the SMs,
 // sequences are cut into segments: a pass over each segment from a zero state (kState: no O), a join that turns the segments'

@@ -573,13 +573,16 @@ extern "C" int mv_window_prefill(void* out, int64_t out_stride, const void* q, i
   // 32 sequences of 128 to 2048 tokens, 16/4 heads, window 1024: 316 -> 183 us; 64 x 512 tokens: 236 -> 126; 2 x 8192: 217 -> 160.
   const int group = heads / kv_heads, pairs = (group + 1) / 2;
   const int64_t tiles = (tokens + kPfTile - 1) / kPfTile + num_seqs;
+  int slot = -1;
   if (dim == 128 && vdim == 128 && !turn && group >= 2 && (bias ? std::min(distances, win) : 1) <= kPfMaxDistances &&
-      num_seqs <= kPfPersistentMaxSeqs && static_cast<int64_t>(kv_heads) * pairs <= 65535 && tiles <= 0x7fffffff) {
+      num_seqs <= kPfPersistentMaxSeqs && static_cast<int64_t>(kv_heads) * pairs <= 65535 && tiles <= 0x7fffffff &&
+      (slot = pf_take_slot(static_cast<cudaStream_t>(stream))) >= 0) {
     CUtensorMap to;
     rc = make_tmap_bf16(&to, out, vdim, heads, tokens, vdim, out_stride, 1, PfOut<true>::kRows, w);
     if (rc) return rc;
     PrefillParams pp{};
     pp.out = out;
+    pp.sched_slot = slot;
     pp.out_stride_tok = out_stride;
     pp.cu_seqlens = cu_q;
     pp.cu_seqlens_k = cu_k;

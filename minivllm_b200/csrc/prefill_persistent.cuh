@@ -1,6 +1,6 @@
 // The persistent prefill kernel on tcgen05: causal attention over packed sequences or a paged cache (prefill_varlen.cu), or with a
-// sliding window, a bias per distance and a sink per head over packed keys (kWin; latent_prefill.cu).  Roles, tensor memory and
-// arithmetic as in prefill_varlen.cu.
+// sliding window, a bias per distance and a sink per head over packed keys (kWin; latent_prefill.cu).  Tensor memory and arithmetic
+// as in prefill_varlen.cu; sixteen softmax warps and the roles below.
 #pragma once
 #include "mma.cuh"
 #include "tcgen05.cuh"
@@ -17,8 +17,7 @@ constexpr int kPfHalfBytes = kPfTile * 128;                 // one 64-element ha
 constexpr int kPfTileBytes = 2 * kPfHalfBytes;              // 32 KB
 constexpr int kPfStages = 2;
 constexpr int kPfSmemBytes = 2 * kPfTileBytes + 2 * kPfStages * kPfTileBytes + 1024;  // Q(2 heads) + K ring + V ring + align
-// Which of the 32 score pairs of a half row take the polynomial exp2 (the others use the special-function unit).
-constexpr float kRescaleThreshold = 8.f;                    // log2 units
+constexpr float kRescaleThreshold = 8.f;                    // of a row's maximum, log2 units
 
 struct PrefillParams {
   void* out;
@@ -127,15 +126,30 @@ __device__ __forceinline__ uint4 ld_shared16(uint32_t addr) {
 constexpr int kPfSortSeqs = 8;      // sequences up to which units are sorted: a lookup goes through them, several times where they
                                     // have few tiles (at 32 sequences, 128 to 2048 tokens, 421 us instead of 395)
 constexpr int kPfUnitRing = 4;      // units handed from the producer warp to the other roles ahead of time
-constexpr int kPfSchedSlots = 1024;  // launches that can be in flight with a work counter of their own
-// Work counters of the persistent launches: [slot][0] = units handed out beyond the first one per CTA,
-// [slot][1] = CTAs that have finished.  Zero between launches: the last CTA of a launch clears its slot.
-static __device__ unsigned int g_pf_sched[kPfSchedSlots][2];
-// Who takes which: one sequence for the table, whatever the instantiation.
+// Work counters of the persistent launches: [slot][0] = units handed out beyond the first one per CTA, [slot][1] = CTAs that have
+// finished.  Zero between launches: the last CTA of a launch clears its slot.  Launches take the first kPfSchedSlots in turn, one
+// sequence for the table whatever the instantiation, so that as many may be in flight.  A captured launch keeps its slot for as long
+// as its graph is replayed, beside any number of others: those have slots of their own, each handed out once.
+constexpr int kPfSchedSlots = 1024, kPfGraphSlots = 4096;
+static __device__ unsigned int g_pf_sched[kPfSchedSlots + kPfGraphSlots][2];
 static std::atomic<unsigned> g_pf_next{0};
-static std::atomic<int> g_pf_last{-1};      // the slot of the last launch, for tests
-static int pf_take_slot() {
-  const int slot = static_cast<int>(g_pf_next.fetch_add(1) % kPfSchedSlots);
+static std::atomic<int> g_pf_graph_next{0};
+static std::atomic<int> g_pf_last{-1};      // what the last launch was given, for tests
+// -1: captured launches have taken all of theirs; the caller has a form without counters.
+static int pf_take_slot(cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &status) != cudaSuccess) {
+    cudaGetLastError();
+    status = cudaStreamCaptureStatusNone;
+  }
+  int slot = -1;
+  if (status == cudaStreamCaptureStatusNone) {
+    slot = static_cast<int>(g_pf_next.fetch_add(1) % kPfSchedSlots);
+  } else {
+    int n = g_pf_graph_next.load();
+    while (n < kPfGraphSlots && !g_pf_graph_next.compare_exchange_weak(n, n + 1)) {}
+    if (n < kPfGraphSlots) slot = kPfSchedSlots + n;
+  }
   g_pf_last.store(slot);
   return slot;
 }
@@ -310,9 +324,9 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
   // What the producer warp publishes for unit k of this CTA (slot k % kPfUnitRing): all the other roles need to
   // know about it, so that none of them has the lookup above on its critical path; n_kv = 0 says there is no
   // more work.  Every other warp says when it no longer needs the slot (UEMPTY, one arrival per warp): the MMA
-  // warp once it has read the step count, a softmax warp after its epilogue, which reads the output rows' place
-  // from the slot only then (four registers fewer across the KV loop).
-  // What the MMA warp needs of a unit, in one register (the warp runs on 40): the number of KV steps and two flags.
+  // warp once it has read the step count, a softmax warp behind its last KV step, where it reads the output rows' place (not
+  // before: four registers fewer across the KV loop), ahead of its epilogue.
+  // What the MMA warp needs of a unit, in one register (the warp runs on 64): the number of KV steps and two flags.
   constexpr int kUnitHasB = 1 << 30, kUnitSplitP = 1 << 29, kUnitSteps = (1 << 29) - 1;
   auto next_unit_steps = [&](int kk) {
     const int slot = kk % kPfUnitRing;
@@ -477,7 +491,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
                                tc::desc64(v_lo0 + s * (kPfTileBytes >> 4), desc_hi), idesc_pv, accum, commit_bar);
       };
       int gk = 0, k = 0;             // KV steps and units so far
-      // Barrier phases in one register (this warp runs on 40): bit t = parity of the steps so far of head t
+      // Barrier phases in one register (this warp runs on 64): bit t = parity of the steps so far of head t
       // (PREADY), bit 2 + t = parity of the units it has finished (OFREE), bit 4 + t = it has finished one.
       uint32_t phases = 0;
       // First QK of a unit whose first KV step has ring index g0.  With a single KV step it is also the last use
@@ -854,9 +868,9 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
 constexpr int kPfPersistentMaxSeqs = 320;   // the persistent form keeps num_seqs + 1 prefix sums in what shared
                                             // memory the tile buffers and the output staging leave
 
-// tmap_o's box is PfOut<kWin>::kRows rows.
+// p.sched_slot is taken; tmap_o's box is PfOut<kWin>::kRows rows.
 template <typename T, bool kWin>
-int launch_prefill_persistent(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, PrefillParams p,
+int launch_prefill_persistent(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const PrefillParams& p,
                               int64_t max_tiles, int ydim, const char* what, cudaStream_t st) {
   constexpr int kPref = ((kPfPersistentMaxSeqs + 1) * 4 + 15) / 16 * 16, kBase = kPfSmemBytes + PfOut<kWin>::kBytes;
   constexpr int kMost = kBase + kPref + (kWin ? 4 * (kPfBefore + kPfMaxDistances + kPfAfter) * 4 : 0);
@@ -874,7 +888,6 @@ int launch_prefill_persistent(const CUtensorMap& tq, const CUtensorMap& tk, cons
     if (dev >= 0 && dev < 64) attr_done[dev] = true;
   }
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(max_tiles * ydim, kNumSMs));   // one CTA per SM
-  p.sched_slot = pf_take_slot();
   prefill_persistent_kernel<T, kWin><<<grid, kPpThreads, smem, st>>>(tq, tk, tv, to, p);
   return check_launch(what);
 }

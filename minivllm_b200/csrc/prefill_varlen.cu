@@ -503,12 +503,12 @@ static std::atomic<int> g_prefill_inject{0};
 
 static std::atomic<int> g_prefill_form{0};   // measurement hook: 0 = choose, 1 = one CTA per tile, 2 = persistent
 template <typename T>
-static int launch_prefill_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p, int64_t total_tokens,
+static int launch_prefill_t(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, PrefillParams& p, int64_t total_tokens,
                             int64_t max_tiles, int ydim, cudaStream_t st) {
   const int form = g_prefill_form.load();
   const bool fits = p.num_seqs <= kPfPersistentMaxSeqs;
-  if (form ? form == 2 : fits) {
-    if (!fits) return fail(MV_ERR_LIMIT, "prefill: the persistent form takes at most %d sequences", kPfPersistentMaxSeqs);
+  if (form == 2 && !fits) return fail(MV_ERR_LIMIT, "prefill: the persistent form takes at most %d sequences", kPfPersistentMaxSeqs);
+  if ((form ? form == 2 : fits) && (p.sched_slot = pf_take_slot(st)) >= 0) {
     CUtensorMap to;
     const int rc = make_tmap(&to, p.out, total_tokens, p.num_heads, p.out_stride_tok, std::is_same<T, __half>::value ? MV_F16 : MV_BF16, PfOut<false>::kRows);
     return rc ? rc : launch_prefill_persistent<T, false>(tq, tk, tv, to, p, max_tiles, ydim, "prefill_persistent_kernel", st);
@@ -552,6 +552,8 @@ extern "C" int mv_debug_prefill_form(int form) {
 
 // Test hook: the work counter of the last persistent launch of this process, -1 before the first.
 extern "C" int mv_debug_prefill_slot(void) { return mv::g_pf_last.load(); }
+// Test hook: as if captured launches had taken `taken` work counters; returns how many they have.
+extern "C" int mv_debug_prefill_graph_slots(int taken) { return mv::g_pf_graph_next.exchange(taken); }
 
 // Test hook: the NEXT prefill launch of this process runs with the given fault injected on the host side of
 // the launch (see PrefillParams::inject).  Nothing faults or hangs: a bounded wait runs out, the error word is

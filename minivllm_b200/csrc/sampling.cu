@@ -171,8 +171,10 @@ argmax_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int64_t col
 // only on that column, so the vocabulary shards of a tensor-parallel model reduce independently and merge by
 // the same 64-bit MAX as the greedy keys -- provided every rank draws the SAME E_i for global column i.
 // Hence a counter-based generator: Philox4x32-10 with key = seed and counter = (global column / 4, row, step),
-// whose four 32-bit outputs serve columns 4g .. 4g+3.  u = (top 24 bits + 0.5) / 2^24 lies strictly inside
-// (0, 1); E = -log(u) (>= 3e-8, so the reference's clamp at 1e-10 never binds).  A row with T == 0 is greedy.
+// whose four 32-bit outputs serve columns 4g .. 4g+3.  u = (top 24 bits + 0.5) / 2^24, rounded to 32-bit floating point; E = -log(u).
+// u is above 0, but the sum is rounded to even from 2^23 on, and its largest value, one column's in 2^24, to 2^24: u is 1 there, E
+// is 0 and the score +inf (NaN for a logit of -inf), so that such a column wins its row.  The oracle has the same rounding.  Other
+// E are at least 1e-7, so the reference's clamp at 1e-10 never binds.  A row with T == 0 is greedy.
 // ---------------------------------------------------------------------------------------------
 struct Philox {
   uint32_t x, y, z, w;

@@ -204,6 +204,42 @@ def test_prefill_launches_of_any_type_take_work_counters_of_their_own():
     assert len(set(slots)) == len(slots), slots
 
 
+def test_captured_prefill_launches_keep_work_counters_that_no_other_launch_takes():
+    """A graph's launch uses its counter at every replay, beside launches that take theirs in turn; when all of those counters are
+    taken, a capture gets the form without one, and the results are the same."""
+    d = synth.prefill_inputs(seed=67, num_seqs=3, len_lo=100, len_hi=700, num_heads=8, num_kv_heads=2, head_dim=128)
+    lib, dtype = _cabi.lib(), torch.bfloat16
+    outs = [torch.zeros(tuple(d["q"].shape), dtype=dtype, device=DEV) for _ in range(3)]
+    word = torch.zeros(1, dtype=torch.int32, device=DEV)
+    q, k, v, cu = (d[n].to(DEV) for n in ("q", "k", "v", "cu_seqlens"))
+    q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
+
+    def call(out):
+        s = torch.cuda.current_stream().cuda_stream
+        assert lib.mv_prefill_varlen(out.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0),
+                                     cu.data_ptr(), cu.numel() - 1, q.shape[0], 8, 2, 128, float(d["scale"]), word.data_ptr(),
+                                     _cabi.dtype_code(dtype), s) == 0
+        return lib.mv_debug_prefill_slot()
+
+    eager = [call(outs[0]) for _ in range(3)]
+    taken, graphs, slots = 0, [], []
+    for n in (None, None, 1 << 20):
+        if n is not None:
+            taken = lib.mv_debug_prefill_graph_slots(ctypes.c_int(n))
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            slots.append(call(outs[len(graphs) - 1]))
+    lib.mv_debug_prefill_graph_slots(ctypes.c_int(taken))
+    assert slots[2] == -1 and len(set(eager + slots)) == 6 and max(eager) < 1024 <= min(slots[:2])
+    for g in graphs:
+        g.replay()
+        g.replay()
+    want = _oracle(d, dtype)
+    for out in outs:
+        _close(out.float().cpu(), want, dtype)
+    assert int(word.item()) == 0
+
+
 def test_prefill_benchmark_configuration_exactly():
     """The prefill configuration of the benchmark plan, as `bench.py` times it: 32 sequences, lengths uniform in
     [128, 2048] (34,277 tokens with this seed), 32 query / 8 KV heads, head_dim 128, bf16 -- every sequence, every
