@@ -159,11 +159,10 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tm_qn, const __grid_co
             else if (b < p.nd) tc::tma_load_3d(dst, &tm_qn, 64 * b, head, row, bar(LB_Q));
             else tc::tma_load_3d(dst, &tm_qr, 64 * (b - p.nd), head, row, bar(LB_Q));
           }
-        int k_asked = 0, v_asked = 0;        // behind a wait that ran out, anyone's, nothing more is asked for
-        for (int i = 0; i < n_kv - lo_a; ++i) {
-          const int s = i % KS, row = k_start + (lo_a + i) * kLfTile;
-          if (!tc::mbar_wait(bar(LB_KEMPTY + s), ((i / KS) & 1) ^ 1, abort_flag, p.error_word, 1) || *abort_flag) break;
-          k_asked = i + 1;
+        int asked = 0;           // behind a wait that ran out, anyone's, no further step is asked for
+        for (; asked < n_kv - lo_a && !*abort_flag; ++asked) {
+          const int i = asked, s = i % KS, row = k_start + (lo_a + i) * kLfTile;
+          tc::mbar_wait(bar(LB_KEMPTY + s), ((i / KS) & 1) ^ 1, abort_flag, p.error_word, 1);
           tc::mbar_expect_tx(bar(LB_KFULL + s), Sh::kKBytes);
           for (int b = 0; b < Sh::kKBytes / kLfBox; ++b) {
             const uint32_t dst = k_smem + s * Sh::kKBytes + b * kLfBox;
@@ -172,16 +171,17 @@ latent_prefill_kernel(const __grid_constant__ CUtensorMap tm_qn, const __grid_co
             else tc::tma_load_3d(dst, &tm_kr, 64 * (b - p.nd), 0, row, bar(LB_KFULL + s));
           }
           const int vs = i % VS;
-          if (!tc::mbar_wait(bar(LB_VEMPTY + vs), ((i / VS) & 1) ^ 1, abort_flag, p.error_word, 2) || *abort_flag) break;
-          v_asked = i + 1;
+          tc::mbar_wait(bar(LB_VEMPTY + vs), ((i / VS) & 1) ^ 1, abort_flag, p.error_word, 2);
           tc::mbar_expect_tx(bar(LB_VFULL + vs), Sh::kVBytes);
           for (int b = 0; b < NV; ++b)
             tc::tma_load_3d(v_smem + vs * Sh::kVBytes + b * kLfBox, &tm_v, 64 * b, kv_head, row, bar(LB_VFULL + vs));
         }
         if (*abort_flag) {       // copies in flight must land before the shared memory goes away
           tc::mbar_wait_timed(bar(LB_Q), 0);
-          for (int i = max(k_asked - KS, 0); i < k_asked; ++i) tc::mbar_wait_timed(bar(LB_KFULL + i % KS), (i / KS) & 1);
-          for (int i = max(v_asked - VS, 0); i < v_asked; ++i) tc::mbar_wait_timed(bar(LB_VFULL + i % VS), (i / VS) & 1);
+          for (int i = max(asked - 2, 0); i < asked; ++i) {
+            if (i >= asked - KS) tc::mbar_wait_timed(bar(LB_KFULL + i % KS), (i / KS) & 1);
+            if (i >= asked - VS) tc::mbar_wait_timed(bar(LB_VFULL + i % VS), (i / VS) & 1);
+          }
         }
       }
     } else if (warp == 9) {

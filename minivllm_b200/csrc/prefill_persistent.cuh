@@ -397,7 +397,6 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
         tc::tma_prefetch_desc(&tmap_k);
         tc::tma_prefetch_desc(&tmap_v);
         int gk = 0, k = 0;          // KV steps and units so far: ring stages and phases run on across units
-        int q_asked = 0, k_asked = 0, v_asked = 0;      // loads asked for: none any more behind a wait that ran out, anyone's
         long long u = blockIdx.x;   // first unit; later ones from the counter
         for (;; ++k) {
           // publish unit k (or the end) for the other roles; the index of the one after it is claimed further
@@ -419,8 +418,7 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
           if (!live) break;
           PF_STAMP(0, k, 0);
           PF_STAMP(0, k, 1);
-          if (!tc::mbar_wait_compact<true>(bar(PB_QEMPTY), (k & 1) ^ 1, abort_flag, p.error_word, 11) || *abort_flag) break;   // passes at once for k = 0
-          q_asked = k + 1;
+          tc::mbar_wait_compact<true>(bar(PB_QEMPTY), (k & 1) ^ 1, abort_flag, p.error_word, 11);   // passes at once for k = 0
           PF_STAMP(0, k, 2);
           const int row0 = w.seq_start + w.q0;
           tc::mbar_expect_tx(bar(PB_Q), (w.has_b ? 2 : 1) * kPfTileBytes);
@@ -445,18 +443,17 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
             }
           };
           for (int j = 0; j < w.n_kv; ++j, ++gk) {
+            if (*abort_flag) break;                  // behind a wait that ran out, anyone's, no further step is asked for
             // Take the next unit as late as its latency allows (it passes under the waits of this unit's last
             // loads, and the MMA warp wants the unit by this unit's last step): a unit claimed earlier is one
             // that an idle SM cannot take at the end of the launch.
             if (j == max(w.n_kv - 2, 0)) u = static_cast<long long>(gridDim.x) + atomicAdd(&sched[0], 1u);
             const int s = gk % kPfStages;
             const uint32_t ph = ((gk / kPfStages) & 1) ^ 1;
-            if (!tc::mbar_wait_compact<true>(bar(PB_KEMPTY + s), ph, abort_flag, p.error_word, 1) || *abort_flag) break;
-            k_asked = gk + 1;
+            tc::mbar_wait_compact<true>(bar(PB_KEMPTY + s), ph, abort_flag, p.error_word, 1);
             tc::mbar_expect_tx(bar(PB_KFULL + s), kPfTileBytes);
             load_kv_tile(&tmap_k, k_smem + s * kPfTileBytes, j, bar(PB_KFULL + s));
-            if (!tc::mbar_wait_compact<true>(bar(PB_VEMPTY + s), ph, abort_flag, p.error_word, 2) || *abort_flag) break;
-            v_asked = gk + 1;
+            tc::mbar_wait_compact<true>(bar(PB_VEMPTY + s), ph, abort_flag, p.error_word, 2);
             tc::mbar_expect_tx(bar(PB_VFULL + s), kPfTileBytes);
             load_kv_tile(&tmap_v, v_smem + s * kPfTileBytes, j, bar(PB_VFULL + s));
             if (j == 0) PF_STAMP(0, k, 4);
@@ -469,9 +466,11 @@ prefill_persistent_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gr
         // After an abort nobody may be left to consume the loads already issued: give them time to land before
         // the CTA (and its shared memory) goes away.  A full barrier completes its phase when its bytes arrive.
         if (*abort_flag) {
-          if (q_asked > 0) tc::mbar_wait_timed(bar(PB_Q), (q_asked - 1) & 1);
-          for (int g2 = max(k_asked - kPfStages, 0); g2 < k_asked; ++g2) tc::mbar_wait_timed(bar(PB_KFULL + g2 % kPfStages), (g2 / kPfStages) & 1);
-          for (int g2 = max(v_asked - kPfStages, 0); g2 < v_asked; ++g2) tc::mbar_wait_timed(bar(PB_VFULL + g2 % kPfStages), (g2 / kPfStages) & 1);
+          if (k > 0) tc::mbar_wait_timed(bar(PB_Q), (k - 1) & 1);
+          for (int g2 = max(gk - kPfStages, 0); g2 < gk; ++g2) {
+            tc::mbar_wait_timed(bar(PB_KFULL + g2 % kPfStages), (g2 / kPfStages) & 1);
+            tc::mbar_wait_timed(bar(PB_VFULL + g2 % kPfStages), (g2 / kPfStages) & 1);
+          }
         }
       }
     } else if (warp == kPpSoftWarps + 1) {

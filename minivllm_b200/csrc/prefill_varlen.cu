@@ -180,16 +180,14 @@ prefill_varlen_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
               tc::tma_load_3d(dst + h * kPfHalfBytes + r * p.box_rows * 128, tm, 64 * h, kvh, slot, full_bar);
           }
         };
-        int k_asked = 0, v_asked = 0;        // behind a wait that ran out, anyone's, nothing more is asked for
-        for (int j = 0; j < n_kv; ++j) {
-          const int s = j % kPfStages;
+        int asked = 0;                       // behind a wait that ran out, anyone's, no further step is asked for
+        for (; asked < n_kv && !*abort_flag; ++asked) {
+          const int j = asked, s = j % kPfStages;
           const uint32_t ph = ((j / kPfStages) & 1) ^ 1;
-          if (!tc::mbar_wait(bar(BAR_KEMPTY + s), ph, abort_flag, p.error_word, 1) || *abort_flag) break;
-          k_asked = j + 1;
+          tc::mbar_wait(bar(BAR_KEMPTY + s), ph, abort_flag, p.error_word, 1);
           tc::mbar_expect_tx(bar(BAR_KFULL + s), kPfTileBytes);
           load_kv_tile(&tmap_k, k_smem + s * kPfTileBytes, j, bar(BAR_KFULL + s));
-          if (!tc::mbar_wait(bar(BAR_VEMPTY + s), ph, abort_flag, p.error_word, 2) || *abort_flag) break;
-          v_asked = j + 1;
+          tc::mbar_wait(bar(BAR_VEMPTY + s), ph, abort_flag, p.error_word, 2);
           tc::mbar_expect_tx(bar(BAR_VFULL + s), kPfTileBytes);
           load_kv_tile(&tmap_v, v_smem + s * kPfTileBytes, j, bar(BAR_VFULL + s));
         }
@@ -197,8 +195,10 @@ prefill_varlen_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_c
         // the CTA (and its shared memory) goes away.  A full barrier completes its phase when its bytes arrive.
         if (*abort_flag) {
           tc::mbar_wait_timed(bar(BAR_Q), 0);
-          for (int j = max(k_asked - kPfStages, 0); j < k_asked; ++j) tc::mbar_wait_timed(bar(BAR_KFULL + j % kPfStages), (j / kPfStages) & 1);
-          for (int j = max(v_asked - kPfStages, 0); j < v_asked; ++j) tc::mbar_wait_timed(bar(BAR_VFULL + j % kPfStages), (j / kPfStages) & 1);
+          for (int j = max(asked - kPfStages, 0); j < asked; ++j) {
+            tc::mbar_wait_timed(bar(BAR_KFULL + j % kPfStages), (j / kPfStages) & 1);
+            tc::mbar_wait_timed(bar(BAR_VFULL + j % kPfStages), (j / kPfStages) & 1);
+          }
         }
       }
     } else if (warp == 9) {

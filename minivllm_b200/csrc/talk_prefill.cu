@@ -125,13 +125,11 @@ talk_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
   if (warp >= 16) {
     tc::setmaxnreg_dec_40();
     if (warp == 16 && !idle) {
-      int t = 0, unit = 0, q_asked = 0, k_asked = 0, v_asked = 0;      // behind a wait that ran out, anyone's, nothing more is asked for
-      bool ok = true;
+      int t = 0, unit = 0;
       auto values = [&](int i) {              // of the unit's tile i, converged
         const int at = t + i, s = at & 1;
-        ok = __all_sync(0xffffffffu, ok && tc::mbar_wait(bar(TB_VEMPTY + s), ((at >> 1) & 1) ^ 1, abort_flag, p.error_word, 2) && !*abort_flag);
-        if (!ok) return;
-        v_asked = at + 1;
+        tc::mbar_wait(bar(TB_VEMPTY + s), ((at >> 1) & 1) ^ 1, abort_flag, p.error_word, 2);
+        __syncwarp();
         if (lane == 0) tc::mbar_expect_tx(bar(TB_VFULL + s), w.boxes * kTpBox);
         __syncwarp();
 #pragma unroll
@@ -139,20 +137,19 @@ talk_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
           if (b < w.boxes)
             tc::tma_load_3d_elected(v_smem + (s * all + b) * kTpBox, &tm_v, 64 * (b % p.boxes), w.v0 + b / p.boxes, w.k_start + i * kTpTile, bar(TB_VFULL + s));
       };
-      for (int u = blockIdx.x; ok && w.find(p, cu_q, cu_k, u); u += gridDim.x, ++unit) {
+      for (int u = blockIdx.x; !*abort_flag && w.find(p, cu_q, cu_k, u); u += gridDim.x, ++unit) {
         __syncwarp();
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(bar(TB_QEMPTY), (unit & 1) ^ 1, abort_flag, p.error_word, 3) && !*abort_flag);
-        if (!ok) break;
-        q_asked = unit + 1;
+        tc::mbar_wait(bar(TB_QEMPTY), (unit & 1) ^ 1, abort_flag, p.error_word, 3);
+        __syncwarp();
         if (lane == 0) tc::mbar_expect_tx(bar(TB_QFULL), kQBytes);
         __syncwarp();
 #pragma unroll
         for (int b = 0; b < NQ; ++b) tc::tma_load_3d_elected(q_smem + b * kTpBox, &tm_q, 64 * b, w.head, w.q_start + w.q0, bar(TB_QFULL));
-        for (int i = 0; i < w.n; ++i) {       // keys one tile ahead of values
-          const int at = t + i, s = at % KS;
-          ok = __all_sync(0xffffffffu, ok && tc::mbar_wait(bar(TB_KEMPTY + s), ((at / KS) & 1) ^ 1, abort_flag, p.error_word, 1) && !*abort_flag);
-          if (!ok) break;
-          k_asked = at + 1;
+        int asked = 0;                        // behind a wait that ran out, anyone's, no further tile is asked for
+        for (; asked < w.n && !__any_sync(0xffffffffu, *abort_flag); ++asked) {      // keys one tile ahead of values
+          const int i = asked, at = t + i, s = at % KS;
+          tc::mbar_wait(bar(TB_KEMPTY + s), ((at / KS) & 1) ^ 1, abort_flag, p.error_word, 1);
+          __syncwarp();
           if (lane == 0) tc::mbar_expect_tx(bar(TB_KFULL + s), kQBytes);
           __syncwarp();
 #pragma unroll
@@ -160,13 +157,15 @@ talk_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_const
             tc::tma_load_3d_elected(k_smem + s * kQBytes + b * kTpBox, &tm_k, 64 * b, w.kv_head, w.k_start + i * kTpTile, bar(TB_KFULL + s));
           if (i > 0) values(i - 1);
         }
-        values(w.n - 1);
-        t += w.n;
+        if (asked > 0) values(asked - 1);
+        t += asked;
       }
-      if (*abort_flag) {                   // copies in flight must land before the shared memory goes away
-        if (q_asked > 0) tc::mbar_wait_timed(bar(TB_QFULL), (q_asked - 1) & 1);
-        for (int at = max(k_asked - KS, 0); at < k_asked; ++at) tc::mbar_wait_timed(bar(TB_KFULL + at % KS), (at / KS) & 1);
-        for (int at = max(v_asked - 2, 0); at < v_asked; ++at) tc::mbar_wait_timed(bar(TB_VFULL + (at & 1)), (at >> 1) & 1);
+      if (*abort_flag && unit > 0) {       // copies in flight must land before the shared memory goes away
+        tc::mbar_wait_timed(bar(TB_QFULL), (unit & 1) ^ 1);
+        for (int at = max(t - 2, 0); at < t; ++at) {
+          tc::mbar_wait_timed(bar(TB_KFULL + at % KS), (at / KS) & 1);
+          tc::mbar_wait_timed(bar(TB_VFULL + (at & 1)), (at >> 1) & 1);
+        }
       }
     } else if (warp == 17 && !idle) {
       const uint32_t idesc_qk = tc::instr_desc_f16(1, 1, false, kTpTile, kTpTile);
