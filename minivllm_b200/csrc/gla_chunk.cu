@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kGpThreads, 2) gla_prepare_kernel(const GlaChu
   // Blocks 0 .. 5 of A below the diagonal, (1,0) (2,0) (2,1) (3,0) (3,1) (3,2), then the four on it: one per warp.
   const bool diag = warp >= 6;
   const int bi = diag ? warp - 6 : warp == 0 ? 1 : warp < 3 ? 2 : 3, bj = diag ? bi : warp - bi * (bi - 1) / 2;
-  bool mine = warp < 10;
+  bool mine = warp < 10 && bi * 16 < nt;                 // rows of A past the sequence's end are nobody's
   if (mine && diag) {
     float least = 0.f;
     for (int c = lane; c < K; c += 32) least = fminf(least, tab(Sh::kTot, bi)[c]);
