@@ -570,7 +570,8 @@ extern "C" int mv_window_prefill(void* out, int64_t out_stride, const void* q, i
   const int win = static_cast<int>(std::min<int64_t>(window, 1 << 30));
   // Heads of 128 in groups: persistent CTAs, two heads of a group over the same keys.  What is left for the kernel above: other
   // sizes, turned results, groups of one head (half of every unit would be empty), long tables, many sequences.
-  // 32 sequences of 128 to 2048 tokens, 16/4 heads, window 1024: 316 -> 183 us; 64 x 512 tokens: 236 -> 126; 2 x 8192: 217 -> 160.
+  // 32 sequences of 128 to 2048 tokens, 16/4 heads, window 1024: 318 -> 211 us; a graph of launches on one input: 316 -> 183, 64 x 512
+  // tokens 236 -> 126, 2 x 8192 217 -> 160.
   const int group = heads / kv_heads, pairs = (group + 1) / 2;
   const int64_t tiles = (tokens + kPfTile - 1) / kPfTile + num_seqs;
   int slot = -1;

@@ -98,8 +98,9 @@ __device__ __forceinline__ float ex2(float x) {
 //   warpgroup of its own for the epilogue was measured too: it takes issue slots from the softmax and gained half as much.
 //   Output: rows leave by TMA through each warp's staging buffer (a thread storing its own row makes 32 lines per
 //   instruction, and the stores of one unit then hold up every shared-memory access of the SM for about 2,000 cycles).
-//   32/8 heads, bf16: 32 sequences of 128 to 2048 tokens 422 -> 396 us; 16 portions behind cached halves 278 -> 243; 64 x 512
-//   tokens 306 -> 229 us.  Long sequences run at the power limit (56 % of the tensor cycles at 1.5 GHz, 1.2 PFLOP/s).
+//   32/8 heads, bf16, a graph of six launches on one input: 32 sequences of 128 to 2048 tokens 422 -> 396 us; 16 portions behind
+//   cached halves 278 -> 243; 64 x 512 tokens 306 -> 229 us.  Inputs that change from call to call: 492 -> 464 and 307 -> 277.
+//   Long sequences run at the power limit (56 % of the tensor cycles at 1.5 GHz, 1.2 PFLOP/s).
 //   Code size: the MMA warp shares an instruction cache with the large softmax loop.  Its waits are the compact
 //   form (rolled spin, the long-wait part a call) and the two warps with few registers keep their loops small;
 //   with unrolled waits the same kernel was 25 % slower on the 32-sequence benchmark.
@@ -124,7 +125,7 @@ __device__ __forceinline__ uint4 ld_shared16(uint32_t addr) {
   return v;
 }
 constexpr int kPfSortSeqs = 8;      // sequences up to which units are sorted: a lookup goes through them, several times where they
-                                    // have few tiles (at 32 sequences, 128 to 2048 tokens, 421 us instead of 395)
+                                    // have few tiles (at 32 sequences, 128 to 2048 tokens, one input, 421 us instead of 395)
 constexpr int kPfUnitRing = 4;      // units handed from the producer warp to the other roles ahead of time
 // Work counters of the persistent launches: [slot][0] = units handed out beyond the first one per CTA, [slot][1] = CTAs that have
 // finished.  Zero between launches: the last CTA of a launch clears its slot.  Launches take the first kPfSchedSlots in turn, one
